@@ -290,7 +290,7 @@ int kspir_packing_rlwes(kspir_ctx* ctx, int client, uint64_t* rlwes, uint64_t* r
  * stream); the call then waits for that stream (cudaStreamSynchronize) and
  * reads a validation word back, so it returns only after its work is done
  * and blocks the calling thread until then.
- * Scratch: a fixed file-scope device array of about 6.3 MiB (plus 192 KiB of
+ * Scratch: a fixed file-scope device array of about 6.3 MiB (plus 300 KiB of
  * transform tables) that every GPU loading this library holds until the
  * process exits.  All calls on a device share it, so calls that overlap on
  * the GPU (other threads, other streams) race and must be serialised by the

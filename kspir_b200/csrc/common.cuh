@@ -37,11 +37,20 @@ enum Chan : int { CH_Q1 = 0, CH_Q2 = 1, CH_BS = 2, CH_P = 3, CH_BA_BS = 4, CH_BA
 // __constant__ memory.
 struct ChanConst {
     uint32_t q;
-    uint32_t two_q;
+    uint32_t nq;           // -q mod 2^32
     uint64_t barrett;      // floor(2^64 / q)
-    uint32_t ninv, ninv_p; // N^-1 mod q and its Shoup companion
-    uint32_t ninv_w, ninv_w_p;   // N^-1 times the last inverse layer's twiddle (psi^-N/2), Shoup
+    uint32_t rq;           // round(2^32 / q)
+    uint32_t qinv;         // q^-1 mod 2^32 (mont_redc)
     uint32_t bsinv, bsinv_p;  // bsMod^-1 mod crtMod, reduced mod q (crt channels only)
+    // factors of the resident keys (k_keys_from_words), canonical: -2^32 (giant,
+    // packing; bsMod rows of the baby keys), 2^32 (RGSW), -bsMod^-1 2^32 (baby)
+    uint32_t kneg, kpos, kbaby;
+    uint32_t xs;           // kbaby, centred
+    // transform twiddles every thread shares (ntt.cuh), as {w, round(w 2^32 / q)}
+    // with w centred: the first forward pass (entry m + i: psi^brv(m + i), m = 1,
+    // 2, 4, 8), the powers 0..7 of psi^(-2N/16) of the inverse's 16-point
+    // transforms, and psi^(-256 t) of its outputs
+    uint2 fw[16], iw[8], ic[16];
 };
 
 struct DevConst {
@@ -78,6 +87,76 @@ __device__ __forceinline__ uint32_t reduce64(uint64_t p, uint32_t q, uint64_t ba
     const uint32_t qh = (uint32_t)__umul64hi(p, barrett);
     const uint32_t r = (uint32_t)p - qh * q;
     return umin(r, r - q);
+}
+
+// ---------------------------------------------------------------------------
+// signed lazy words of the transforms: any word below 8 q in magnitude
+// (q < 2^28) stands for its residue
+
+// y w mod q within (-|y| / 2^33, 1 + |y| / 2^33) q; w = {centred, round(w 2^32 / q)}.
+// The quotient is the floor: rounding it would keep products within +-q/2, but the
+// rounding addend costs two additions beside the mul.hi (the wide
+// multiply-add is split), more than the few reductions that the wider
+// range needs.
+__device__ __forceinline__ uint32_t mul_lazy(uint32_t y, uint2 w, uint32_t nq) {
+    return y * w.x + (uint32_t)__mulhi((int)y, (int)w.y) * nq;
+}
+
+// decimation-in-time butterfly: (X + wY, X - wY); widens a range of +-B q to
+// +-(1.03125 B + 1) q
+__device__ __forceinline__ void bfly(uint32_t& X, uint32_t& Y, uint2 w, uint32_t nq) {
+    const uint32_t s = Y * w.x + X + (uint32_t)__mulhi((int)Y, (int)w.y) * nq;
+    Y = 2 * X - s;
+    X = s;
+}
+
+// to within (-0.11, 1.11) q
+__device__ __forceinline__ uint32_t reduce_lazy(uint32_t x, uint32_t rq, uint32_t nq) {
+    return x + (uint32_t)__mulhi((int)x, (int)rq) * nq;
+}
+
+// +-6 q to +-3 q; +-8 q to +-2 q
+__device__ __forceinline__ uint32_t fold6(uint32_t x, uint32_t q) { return umin(x, x + 6 * q) - 3 * q; }
+__device__ __forceinline__ uint32_t fold8(uint32_t x, uint32_t q) {
+    const uint32_t r = umin(x, x + 8 * q);
+    return umin(r, r - 4 * q) - 2 * q;
+}
+
+// p 2^-32 mod q within +-(|p| / 2^32 + q/2) for a signed 64-bit p (Montgomery: the
+// low words of p and m q are equal).  Two multiplies, where an exact 64-bit
+// Barrett reduction takes about fourteen instructions; the resident keys
+// carry the factor 2^32.
+__device__ __forceinline__ uint32_t mont_redc(uint64_t p, const ChanConst& c) {
+    const uint32_t m = (uint32_t)p * c.qinv;
+    return (uint32_t)(p >> 32) - (uint32_t)__mulhi((int)m, (int)c.q);
+}
+
+// a word in (-q, q), (-q, 2q), (-2q, 2q) or (-4q, 4q) to [0, q)
+__device__ __forceinline__ uint32_t canon_pm1(uint32_t x, uint32_t q) { return umin(x, x + q); }
+__device__ __forceinline__ uint32_t canon_m1p2(uint32_t x, uint32_t q) {
+    const uint32_t r = umin(x, x + q);
+    return umin(r, r - q);
+}
+
+__device__ __forceinline__ uint32_t canon_pm2(uint32_t x, uint32_t q) {
+    const uint32_t r = umin(x, x + 2 * q);
+    return umin(r, r - q);
+}
+__device__ __forceinline__ uint32_t canon_pm4(uint32_t x, uint32_t q) {
+    uint32_t r = umin(x, x + 4 * q);
+    r = umin(r, r - 2 * q);
+    return umin(r, r - q);
+}
+
+// to [0, q)
+__device__ __forceinline__ uint32_t canon_lazy(uint32_t x, const ChanConst& c) {
+    return canon_m1p2(reduce_lazy(x, c.rq, c.nq), c.q);
+}
+
+// a canonical residue to [-q/2, q/2]
+__device__ __forceinline__ uint32_t centre(uint32_t x, uint32_t q) {
+    const uint32_t h = q >> 1, u = x + h;
+    return umin(u, u - q) - h;
 }
 
 __device__ __forceinline__ uint32_t mulmod(uint32_t a, uint32_t b, int ch) {
@@ -178,6 +257,11 @@ __device__ __forceinline__ int auto_src(int k, uint32_t ginv, bool* neg) {
 
 // q - x, and 0 for x = 0 (0 - x wraps above q - x for every other x)
 __device__ __forceinline__ uint32_t negmod(uint32_t x, uint32_t q) { return umin(q - x, 0u - x); }
+
+// acc += a * b, signed
+__device__ __forceinline__ void mad_wide_s(uint64_t& acc, uint32_t a, uint32_t b) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
+}
 
 // acc += a * b with a 32x32->64-bit product, as one fused wide multiply-add
 __device__ __forceinline__ void mad_wide(uint64_t& acc, uint32_t a, uint32_t b) {

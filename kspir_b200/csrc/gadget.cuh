@@ -31,6 +31,26 @@ __device__ __forceinline__ void decompose_b(uint64_t x, uint64_t q, const Gadget
     }
 }
 
+// decompose_b of the value with residues (r1, r2) mod (q1, q2), or of its negative
+// (`neg`; the negative of 0 counts as crtMod, which decomposes like 0), the CRT
+// folded into the sum: d = offset +- (r1 + q1 t), plus crtMod when negated.
+template <int ELL>
+__device__ __forceinline__ void decompose_b_res(uint32_t r1, uint32_t r2, bool neg, const GadgetB& g, int32_t* dig) {
+    const uint32_t t = shoup_mul(submod(r2, umin(r1, r1 - kQ2), kQ2), c_dev.q1inv_mod_q2, c_dev.q1inv_mod_q2_p, kQ2);
+    uint64_t d = neg ? g.offset + kCrtMod : g.offset;
+    d += (uint64_t)(int64_t)(int32_t)(neg ? 0u - r1 : r1);
+    mad_wide_s(d, neg ? 0u - kQ1 : kQ1, t);
+    if (d > kCrtMod) d -= kCrtMod;
+    d >>= g.base_bits;
+    const uint32_t mask = (1u << g.gbits) - 1;
+    const int32_t half = 1 << (g.gbits - 1);
+#pragma unroll
+    for (int j = 0; j < ELL; j++) {
+        dig[j] = (int32_t)((uint32_t)d & mask) - half;
+        d >>= g.gbits;
+    }
+}
+
 // decompose_bsgs (reference utils.cpp:1120-1189) over crt_inv_bsgs
 // (utils.cpp:516-532): the 80-bit CRT value of (x mod crtMod, y mod bsMod),
 // then VARIANT-B digits of it modulo M = crtMod * bsMod.

@@ -86,7 +86,7 @@ __host__ __device__ __forceinline__ int fa_counter_words(int R) { return FC_PER_
 enum : int { FT_T_START = 0, FT_T_HEAD, FT_T_SCAN0, FT_T_SCAN1, FT_T_GIANT, FT_T_EXT, FT_T_END, FT_T_COUNT = 8 };
 
 constexpr int kFaPrepChunks = kN / kNttThreads;   // 8
-constexpr int kFaKsSmem = kN * 8 + 4 * kPadN * 4;  // twiddles + four padded polynomials
+constexpr int kFaKsSmem = 4 * kPadN * 4;          // four padded polynomials
 
 template <int N1, int SCAN_WARPS>
 struct FaCfg {
@@ -221,27 +221,15 @@ __device__ __forceinline__ bool fa_level_reads_ext(int levels, int lv) { return 
 
 template <bool INVERSE>
 __device__ __forceinline__ void fa_ntt_job(const FaArgs& A, NttJob jb, uint8_t* smem) {
-    uint2* tws = reinterpret_cast<uint2*>(smem);
-    uint32_t* s = reinterpret_cast<uint32_t*>(smem + kN * 8);
+    uint32_t* s = reinterpret_cast<uint32_t*>(smem);
     jb.src = shifted(jb.src, ws_off(A.bt));
     jb.dst = shifted(jb.dst, ws_off(A.bt));
-    stage_twiddles(tws, A.tabs, jb.ch, INVERSE ? NTT_INV : NTT_FWD);
-    ntt_job_run<INVERSE, KsSync>(jb, tws, s);
+    ntt_job_run<INVERSE, KsSync, kNttThreads>(jb, A.tabs, s);
 }
 
-// one rotation (key index ki, component comp), both primes: k_baby_pair's work
+// one rotation (key index ki, component comp), both primes: k_baby_rot<1>'s work
 __device__ __forceinline__ void fa_rotation(const FaArgs& A, const BabyArgs& a, int ki, int comp, uint8_t* smem) {
-    uint2* tws = reinterpret_cast<uint2*>(smem);
-    uint32_t* S = reinterpret_cast<uint32_t*>(smem + kN * 8);
-    uint32_t* S2 = S + kPadN;
-    BabyRot R;
-    stage_twiddles(tws, A.tabs, CH_BS, NTT_INV);
-    baby_setup<3>(R, a, A.keys, A.bt, ki, comp);
-    baby_bs_part<3, KsSync>(R, a, S, tws, true);
-#pragma unroll
-    for (int it = 0; it < kPerThread; it++) S2[pidx(R.tid) + it * kPadStep] = S[pidx(R.tid) + it * kPadStep];
-    baby_crt_part<3, KsSync>(R, a, S, tws, A.tabs, 0);
-    baby_crt_part<3, KsSync>(R, a, S2, tws, A.tabs, 1);
+    baby_rotation<1, KsSync>(reinterpret_cast<uint32_t*>(smem), a, A.keys, A.tabs, A.bt, ki, comp);
 }
 
 // giant step (r, c): the key switch of evalAutoRNSCRT for output row c of
@@ -249,80 +237,17 @@ __device__ __forceinline__ void fa_rotation(const FaArgs& A, const BabyArgs& a, 
 // terms are added into acc[r].
 template <int ELL>
 __device__ __forceinline__ void fa_giant(const FaArgs& A, int r, int c, uint8_t* smem) {
-    uint2* tws = reinterpret_cast<uint2*>(smem);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem + kN * 8);   // [4][N]
-    const int N1 = A.N1, N2 = kN / 2 / N1;
-    const int rows = A.R * N2, row = r * N2 + c;
-    const int tid = threadIdx.x;
-    const uint32_t* sout = shifted(A.w.sout, ws_off(A.bt));
-    const uint32_t* gkeys = shifted(A.keys.giant, key_off(A.bt));
-    uint32_t* acc = A.acc + (size_t)r * 4 * kN;
-#pragma unroll
-    for (int ch = 0; ch < 2; ch++) {
-        stage_twiddles(tws, A.tabs, ch, NTT_INV);
-#pragma unroll
-        for (int k = tid; k < kN / 4; k += kNttThreads)
-            *reinterpret_cast<uint4*>(P + ch * kPadN + pidx(4 * k)) =
-                __ldcg(reinterpret_cast<const uint4*>(sout + sout_idx(row, 0 * 2 + ch, 4 * k, rows)));
-        cta_ntt_inverse<KsSync>(P + ch * kPadN, tws, ch);
-    }
-    const uint32_t e = (uint32_t)(N1 * c) & 2047u;
-    uint32_t ginv = 1, b5 = 5, x = (2048u - e) & 2047u;
-    while (x) { if (x & 1) ginv = (ginv * b5) & (2 * kN - 1); b5 = (b5 * b5) & (2 * kN - 1); x >>= 1; }
-    uint32_t dres[kPerThreadG][ELL][2];
-#pragma unroll
-    for (int it = 0; it < kPerThreadG; it++) {
-        const int k = tid + it * kNttThreads;
-        bool neg;
-        const int src = auto_src(k, ginv, &neg);
-        uint64_t v = crt_compose_res(P[pidx(src)], P[kPadN + pidx(src)]);
-        if (neg && v) v = kCrtMod - v;
-        int32_t dig[kMaxEll];
-        decompose_b(v, kCrtMod, A.gad.giant, dig);
-#pragma unroll
-        for (int j = 0; j < ELL; j++) {
-            dres[it][j][0] = signed_to_res(dig[j], kQ1);
-            dres[it][j][1] = signed_to_res(dig[j], kQ2);
-        }
-    }
-    KsSync::sync();
-#pragma unroll
-    for (int it = 0; it < kPerThreadG; it++)
-#pragma unroll
-        for (int j = 0; j < ELL; j++)
-#pragma unroll
-            for (int ch = 0; ch < 2; ch++) P[(j * 2 + ch) * kPadN + pidx(tid) + it * kPadStep] = dres[it][j][ch];
-    const uint32_t* key = gkeys + (size_t)(c - 1) * ELL * 2 * 2 * kN;   // [ELL][2 comp][2 ch][N]
-    const uint16_t* sig = A.sigma_giant + (size_t)(c - 1) * kN;
-#pragma unroll 1
-    for (int ch = 0; ch < 2; ch++) {
-        KsSync::sync();
-        stage_twiddles(tws, A.tabs, ch, NTT_FWD);
-        cta_ntt_forward_m<ELL, KsSync>(P + ch * kPadN, 2 * kPadN, tws, ch);
-        const uint32_t q = c_dev.ch[ch].q;
-#pragma unroll
-        for (int it = 0; it < kPerThreadG; it++) {
-            const int k = tid + it * kNttThreads;
-            uint64_t sa = 0, sb = 0;
-#pragma unroll
-            for (int j = 0; j < ELL; j++) {
-                const uint32_t d = P[(j * 2 + ch) * kPadN + pidx(tid) + it * kPadStep];
-                mad_wide(sa, d, __ldg(key + ((j * 2 + 0) * 2 + ch) * kN + k));
-                mad_wide(sb, d, __ldg(key + ((j * 2 + 1) * 2 + ch) * kN + k));
-            }
-            const uint32_t bv = __ldcg(sout + sout_idx(row, 1 * 2 + ch, sig[k], rows));
-            atomicAdd(acc + (size_t)(0 * 2 + ch) * kN + k, negmod(mod_crt(sa, ch), q));
-            atomicAdd(acc + (size_t)(1 * 2 + ch) * kN + k, addmod(bv, negmod(mod_crt(sb, ch), q), q));
-        }
-    }
+    const int N2 = kN / 2 / A.N1;
+    giant_body<ELL, KsSync>(reinterpret_cast<uint32_t*>(smem), shifted(A.w.sout, ws_off(A.bt)),
+                            A.acc + (size_t)r * 4 * kN, shifted(A.keys.giant, key_off(A.bt)), A.sigma_giant, A.N1,
+                            A.tabs, A.gad.giant, r * N2 + c, c, A.R * N2);
 }
 
 // external product of sub-database r on prime ch: the first-dimension result
 // is (acc[r] + scan row 0) mod q (k_giant_finish's sum); the task of prime 0
 // also keeps it (NTT form) in the workspace's result for the diagnostics.
 __device__ __forceinline__ void fa_ext(const FaArgs& A, int r, int ch, uint8_t* smem) {
-    uint2* tws = reinterpret_cast<uint2*>(smem);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem + kN * 8);
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem);
     const int N2 = kN / 2 / A.N1, rows = A.R * N2, row0 = r * N2;
     const int tid = threadIdx.x;
     const size_t wo = ws_off(A.bt);
@@ -332,7 +257,6 @@ __device__ __forceinline__ void fa_ext(const FaArgs& A, int r, int ch, uint8_t* 
 #pragma unroll
     for (int pch = 0; pch < 2; pch++) {
         const ChanConst cq = c_dev.ch[pch];
-        stage_twiddles(tws, A.tabs, pch, NTT_INV);
 #pragma unroll
         for (int comp = 0; comp < 2; comp++) {
             const int cv = comp * 2 + pch;
@@ -349,11 +273,11 @@ __device__ __forceinline__ void fa_ext(const FaArgs& A, int r, int ch, uint8_t* 
                 if (ch == 0) reinterpret_cast<uint4*>(result + (size_t)cv * kN)[k4] = v;
             }
         }
-        cta_ntt_inverse_m<2, KsSync>(P + pch * kPadN, 2 * kPadN, tws, pch);
+        cta_ntt_inverse_m<2, KsSync>(P + pch * kPadN, 2 * kPadN, A.tabs, pch);
     }
     const uint32_t* rgsw = shifted(A.keys.rgsw, key_off(A.bt));
     uint32_t* ext = shifted(A.w.ext, wo) + (size_t)r * 4 * kN;
-    ext_tail<2, KsSync>(P, tws, rgsw, nullptr, ext, A.tabs, A.gad.ext, ch);
+    ext_tail<2, KsSync>(P, rgsw, nullptr, ext, A.tabs, A.gad.ext, ch);
 }
 
 __device__ __forceinline__ void fa_pack_fwd(const FaArgs& A, int lv, int j, int ch, int d, uint8_t* smem) {

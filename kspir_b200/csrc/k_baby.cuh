@@ -11,13 +11,25 @@
 //   out.a = NTT((INTT(A_crt) - x2a) * bsMod^-1),  x2a = INTT_bs(A_bs)
 //   out.b = NTT((INTT(B_crt) + auto_g(b) - x2b) * bsMod^-1),
 //           x2b = INTT_bs(B_bs) + auto_g(b mod bsMod)
-// (twosteps.cpp:1034-1071).  All of it is exact arithmetic mod crtMod with
-// canonical values, so by linearity of the transform the same words are
-//   out.a = (A_crt - NTT(x2a)) * bsMod^-1
-//   out.b = (B_crt + NTT(b)[sigma_g] - NTT(x2b)) * bsMod^-1
+// (twosteps.cpp:1034-1071).  All of it is exact arithmetic mod crtMod and
+// bsMod with canonical values, so by linearity of the transform the same words are
+//   out.a = A_crt * bsMod^-1 - NTT(x2a) * bsMod^-1
+//   out.b = B_crt * bsMod^-1 + (NTT(b) * bsMod^-1)[sigma_g] - NTT(x2b) * bsMod^-1
+//   x2b   = INTT_bs(B_bs + NTT_bs(b)[sigma_g])
 // where sigma_g is the slot permutation of X -> X^g in the NTT domain.  Only
 // the bsMod channel is brought to coefficient form (x2 must be the canonical
 // integer < bsMod); the crt channels stay in the NTT domain throughout.
+//
+// The resident keys carry the signs, bsMod^-1 and 2^32 (k_keys_from_words), so a
+// slot is the Montgomery reduction of one 64-bit sum of four products: the
+// three digits' and NTT(x2) times a constant.  The query side keeps the three
+// digits of a slot and its b side by side (16 bytes), one gather per slot for
+// the three digits of both components.
+//
+// What bounds it: instruction issue and the multiply pipe (ntt.cuh), with the
+// keys (22 MiB per client) streaming from L2 or HBM beside it.  Batch of 64:
+// 1.20 ms with one component per CTA, conditional-subtraction transforms and
+// 64-bit Barrett reductions, 0.77 ms in this form.
 #pragma once
 
 #include <type_traits>
@@ -29,15 +41,13 @@
 namespace kspir {
 
 struct BabyArgs {
-    const uint32_t* dig;     // [ell][3 ch][N] source digits, NTT form
-    const uint32_t* srcB;    // [2 ch][N] NTT form of the source b (crt)
-    const uint32_t* srcBbs;  // [N] source b mod bsMod, coefficient form
-    const int32_t* perms;    // caller permutations [N1][N] (reference test-pir.cpp:92-93)
-    const uint16_t* sigma;   // [N1/2][N] slot permutation of X -> X^(5^(i+1))
+    const uint32_t* dig;     // [3 ch][N][4]: the three digits and b of a slot, NTT form (crt channels: b * bsMod^-1)
+    const uint16_t* perms;   // caller permutations [N1][N] (reference test-pir.cpp:92-93), lane order
+    const uint16_t* sigma;   // [N1/2][N] slot permutation of X -> X^(5^(i+1)), lane order
     uint64_t* cipherbuf;     // [N][N1][2]
-    uint32_t* interA;        // outputs of the intermediate rotation (or null)
-    uint32_t* interB;
-    uint32_t* inter_bs;
+    uint32_t* interA;        // outputs of the intermediate rotation: a before the modswitch [2 ch][N], NTT form
+    uint32_t* inter_dig;     // its b as the fourth word of the second half's dig
+    uint32_t* inter_bs;      // its a mod bsMod [N], coefficient form
     int32_t N1;
     int32_t col_base;        // cipherbuf column of key index 0
     int32_t inter_idx;       // key index whose pre-modswitch state is exported, or -1
@@ -53,186 +63,193 @@ __host__ __device__ __forceinline__ size_t cipherbuf_rm_idx(int col, int comp, i
     return ((size_t)(col * 2 + comp) * 2 + ch) * kN + z;
 }
 
-// 5^e mod 2N
-__device__ __forceinline__ uint32_t pow5_mod2n(uint32_t e) {
-    uint32_t r = 1, b = 5;
-    while (e) {
-        if (e & 1) r = (r * b) & (2 * kN - 1);
-        b = (b * b) & (2 * kN - 1);
-        e >>= 1;
-    }
-    return r;
-}
-
-constexpr int kBabyPairSmem = kN * 8 + 2 * kPadN * 4;   // twiddles + two padded polynomials
-constexpr int kPerThread = kN / kNttThreads; // 8 coefficients per thread
-
-// Per-rotation state shared by the two kernel shapes below.
-struct BabyRot {
-    int ki, comp, col, tid;
-    bool inter;
-    size_t wo;              // workspace offset of the query
-    const uint32_t* kbs;    // bsMod keys of rotation ki
-    const uint32_t* kcrt;   // crt keys of rotation ki
-    const int32_t* perm;    // caller permutation of rotation ki
-};
+constexpr int kBabyEll = 3;
+constexpr int kBabyPolys1 = 2, kBabyPolys2 = 4;   // padded polynomials: x2 of one or two components, per prime
 
 // Loads of the query-side inputs (digits, b): written by earlier kernels, so a
 // stand-alone launch (CtaSync) reads them through L1 (their gathers reuse
 // lines across the rotations on an SM); inside the fused answer kernel other
 // CTAs write them during the launch, so those loads bypass L1.
-template <class Sync>
-__device__ __forceinline__ uint32_t ld_query(const uint32_t* p) {
+template <class Sync, class T>
+__device__ __forceinline__ T ld_query(const T* p) {
     if constexpr (std::is_same<Sync, CtaSync>::value) return __ldg(p);
     else return __ldcg(p);
 }
 
-// perm[k] of this thread's coefficients (reloaded by each multiply-accumulate
-// rather than held in registers across the transforms)
-__device__ __forceinline__ void baby_perm(const BabyRot& R, int* pk) {
+// the permutation entries of a thread's coefficients u + 256 (4 v + w), w = 0..3
+__device__ __forceinline__ void perm4(const uint16_t* __restrict__ p, int i, uint32_t* o) {
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(p) + i);
+    o[0] = a.x & 0xffff; o[1] = a.x >> 16; o[2] = a.y & 0xffff; o[3] = a.y >> 16;
+}
+
+// sum_j d_j[perm] key_j of four coefficients: the vector of component `comp`
+// added to acc; d: the gathered slots, key: [j][comp][...] at stride `jstride`
+// vectors between digits
+__device__ __forceinline__ void baby_mac4(uint64_t* acc, const uint4* d, const uint4* __restrict__ key, int jstride) {
 #pragma unroll
-    for (int it = 0; it < kPerThread; it++) pk[it] = __ldg(R.perm + R.tid + it * kNttThreads);
+    for (int j = 0; j < kBabyEll; j++) {
+        const uint4 k = __ldg(key + (size_t)j * jstride);
+        const uint32_t kw[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+        for (int w = 0; w < 4; w++) mad_wide_s(acc[w], j == 0 ? d[w].x : j == 1 ? d[w].y : d[w].z, kw[w]);
+    }
 }
 
-// The workspace pointers of BabyArgs are slot-0 pointers: each use adds the
-// query's workspace offset R.wo (kept as one value rather than seven shifted
-// pointers, which would pin fourteen registers for the whole kernel).
-template <int ELL>
-__device__ __forceinline__ void baby_setup(BabyRot& R, const BabyArgs& a, const ClientKeysDev& keys,
-                                           const Batch& bt, int ki, int comp) {
-    R.ki = ki;
-    R.comp = comp;
-    R.col = a.col_base + ki;
-    R.tid = threadIdx.x;
-    R.inter = (ki == a.inter_idx);
-    R.wo = ws_off(bt);
-    const size_t ko = key_off(bt);
-    R.kbs = shifted(keys.baby_bs, ko) + (size_t)ki * ELL * 2 * kN;
-    R.kcrt = shifted(keys.baby_crt, ko) + (size_t)ki * ELL * 2 * 2 * kN;
-    R.perm = a.perms + (size_t)(ki + 1) * kN;
-}
+// Rotation ki of one query by 512 threads, COMPS components: both (COMPS = 2),
+// or the one given (1).  P: 2 COMPS padded polynomials.
+//
+//  1. bsMod part in the NTT domain, eight slots per thread;
+//  2. x2 by the inverse transform mod bsMod, one component per thread group
+//     (COMPS = 1: the second group waits), stored twice;
+//  3. NTT_ch(x2), one prime per group: with COMPS = 2 both components of the
+//     prime share one set of twiddle loads;
+//  4. the crt products, the modswitch and the cipherbuf store, one prime per
+//     group, sixteen slots per thread, one digit gather for both components.
+template <int COMPS, class Sync>
+__device__ __forceinline__ void baby_rotation(uint32_t* P, const BabyArgs& a, const ClientKeysDev& keys,
+                                              const NttTables& tabs, const Batch& bt, int ki, int comp0) {
+    const int g = thread_group(), u = threadIdx.x & (kNttGroup - 1);
+    const bool inter = ki == a.inter_idx;
+    // slot-0 workspace pointers: each use adds the query's offset
+    const size_t wo = ws_off(bt), ko = key_off(bt);
+    const uint16_t* perm = a.perms + (size_t)(ki + 1) * kN;
+    const uint16_t* sig = a.sigma + (size_t)ki * kN;
+    const uint4* dig = reinterpret_cast<const uint4*>(shifted(a.dig, wo));
 
-// x2 of this component into S (coefficient form, canonical mod bsMod):
-//   INTT_bs(-sum_j d_j[perm] * key_j) (+ auto_g(b mod bsMod) for comp 1).
-// The caller has staged the bsMod inverse twiddles into tws (unsynchronised).
-// export_inter: this CTA writes the intermediate rotation's x2.
-template <int ELL, class Sync = CtaSync>
-__device__ __forceinline__ void baby_bs_part(const BabyRot& R, const BabyArgs& a, uint32_t* S, const uint2* tws,
-                                             bool export_inter) {
-    const int tid = R.tid;
+    // 1. sum_j d_j key_j (+ NTT_bs(b)[sigma] for component b) mod bsMod
     {
-        const ChanConst cb = c_dev.ch[CH_BS];
-        int pk[kPerThread];
-        baby_perm(R, pk);
-        uint64_t acc[kPerThread];
+        const ChanConst& cb = c_dev.ch[CH_BS];
+        const uint4* kbs = reinterpret_cast<const uint4*>(shifted(keys.baby_bs, ko) + (size_t)ki * kBabyEll * 2 * kN);
 #pragma unroll
-        for (int it = 0; it < kPerThread; it++) acc[it] = 0;
+        for (int vv = 0; vv < 2; vv++) {
+            const int v = 2 * g + vv, i = v * kNttGroup + u;
+            uint32_t pk[4];
+            uint4 d[4];
+            perm4(perm, i, pk);
 #pragma unroll
-        for (int j = 0; j < ELL; j++) {
-            const uint32_t* d = shifted(a.dig, R.wo) + (size_t)(j * 3 + CH_BS) * kN;
-            const uint32_t* kk = R.kbs + (size_t)(j * 2 + R.comp) * kN;
+            for (int w = 0; w < 4; w++) d[w] = ld_query<Sync>(dig + CH_BS * kN + pk[w]);
 #pragma unroll
-            for (int it = 0; it < kPerThread; it++)
-                acc[it] += (uint64_t)ld_query<Sync>(d + pk[it]) * __ldg(kk + tid + it * kNttThreads);
+            for (int c = 0; c < COMPS; c++) {
+                const int comp = COMPS == 2 ? c : comp0;
+                uint64_t acc[4] = {0, 0, 0, 0};
+                baby_mac4(acc, d, kbs + comp * (kN / 4) + i, 2 * kN / 4);
+                uint32_t r[4];
+#pragma unroll
+                for (int w = 0; w < 4; w++) r[w] = mont_redc(acc[w], cb);
+                if (comp == 1) {
+                    perm4(sig, i, pk);
+#pragma unroll
+                    for (int w = 0; w < 4; w++) {
+                        r[w] = canon_m1p2(r[w] + ld_query<Sync>(reinterpret_cast<const uint32_t*>(dig + CH_BS * kN + pk[w]) + 3), cb.q);
+                        // the second half's b mod bsMod is this sum
+                        if (inter) shifted(a.inter_dig, wo)[(size_t)(CH_BS * kN + u + kNttGroup * (4 * v + w)) * 4 + 3] = r[w];
+                    }
+                } else {
+#pragma unroll
+                    for (int w = 0; w < 4; w++) r[w] = canon_pm1(r[w], cb.q);
+                }
+#pragma unroll
+                for (int w = 0; w < 4; w++) P[2 * c * kPadN + pidx(u) + (4 * v + w) * kPadGroupStep] = r[w];
+            }
         }
-#pragma unroll
-        for (int it = 0; it < kPerThread; it++)
-            S[pidx(tid) + it * kPadStep] = negmod(reduce64(acc[it], cb.q, cb.barrett), cb.q);
     }
-    cta_ntt_inverse<Sync>(S, tws, CH_BS);
 
-    if (R.comp == 1) {
-        // x2b += auto_g(b mod bsMod)   (automorphic_rns, twosteps.cpp:1045-1048)
-        const uint32_t ginv = pow5_mod2n(2048u - (uint32_t)(R.ki + 1));
-        const uint32_t qb = c_dev.ch[CH_BS].q;
+    // 2. x2, once for each prime
+    {
+        const int comp = COMPS == 2 ? g : comp0;
+        uint32_t* S = P + (COMPS == 2 ? 2 * g : 0) * kPadN;
+        uint32_t* bs_out = inter && comp == 0 ? shifted(a.inter_bs, wo) : nullptr;
+        auto out = [&](int, int t, uint32_t x) {
+            S[pidx(u) + t * kPadGroupStep] = x;
+            S[kPadN + pidx(u) + t * kPadGroupStep] = x;
+            if (bs_out) bs_out[u + kNttGroup * t] = x;
+        };
+        Sync::sync();
+        if (COMPS == 2 || g == 0) group_ntt_inverse<1, GroupSync>(S, kPadN, tabs, CH_BS, u, out);
+    }
+
+    // 3.
+    const int ch = g;
+    uint32_t* S = P + ch * kPadN;
+    Sync::sync();
+    group_ntt_forward<COMPS, GroupSync, true>(S, 2 * kPadN, tabs, ch, u);   // x2 < bsMod < q / 14: signed, lazy
+
+    // 4.
+    const ChanConst& cc = c_dev.ch[ch];
+    const uint4* kcrt = reinterpret_cast<const uint4*>(shifted(keys.baby_crt, ko) + (size_t)ki * kBabyEll * 4 * kN);
+    const int col = a.col_base + ki;
+    uint32_t* cb32 = reinterpret_cast<uint32_t*>(shifted(a.cipherbuf, wo));
+    auto cb_at = [&](int comp, int k) -> uint32_t* {
+        return cb32 + (a.cb_rm ? cipherbuf_rm_idx(col, comp, ch, k) : (((size_t)k * a.N1 + col) * 2 + comp) * 2 + ch);
+    };
 #pragma unroll
-        for (int it = 0; it < kPerThread; it++) {
-            const int k = tid + it * kNttThreads;
-            const int pk2 = pidx(tid) + it * kPadStep;
-            bool neg;
-            const int src = auto_src(k, ginv, &neg);
-            uint32_t v = ld_query<Sync>(shifted(a.srcBbs, R.wo) + src);
-            if (neg) v = negmod(v, qb);
-            S[pk2] = addmod(S[pk2], v, qb);
+    for (int v = 0; v < 4; v++) {
+        const int i = v * kNttGroup + u;
+        uint32_t pk[4];
+        uint4 d[4];
+        perm4(perm, i, pk);
+#pragma unroll
+        for (int w = 0; w < 4; w++) d[w] = ld_query<Sync>(dig + ch * kN + pk[w]);
+#pragma unroll
+        for (int c = 0; c < COMPS; c++) {
+            const int comp = COMPS == 2 ? c : comp0;
+            uint64_t acc[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int w = 0; w < 4; w++)
+                mad_wide_s(acc[w], S[2 * c * kPadN + pidx(u) + (4 * v + w) * kPadGroupStep], cc.xs);
+            baby_mac4(acc, d, kcrt + (comp * 2 + ch) * (kN / 4) + i, 4 * kN / 4);
+            uint32_t r[4];
+            // below (3 q + 6.7 q) q / 2 / 2^32 + q / 2 < 0.9 q in magnitude
+#pragma unroll
+            for (int w = 0; w < 4; w++) r[w] = mont_redc(acc[w], cc);
+            if (comp == 1) {
+                perm4(sig, i, pk);
+#pragma unroll
+                for (int w = 0; w < 4; w++)
+                    r[w] = canon_m1p2(r[w] + ld_query<Sync>(reinterpret_cast<const uint32_t*>(dig + ch * kN + pk[w]) + 3), cc.q);
+            } else {
+#pragma unroll
+                for (int w = 0; w < 4; w++) r[w] = canon_pm1(r[w], cc.q);
+            }
+#pragma unroll
+            for (int w = 0; w < 4; w++) *cb_at(comp, u + kNttGroup * (4 * v + w)) = r[w];
         }
     }
-    if (R.inter && export_inter) {
+    if (inter) {
+        // the state before the modswitch: a = out * bsMod + x2, and b * bsMod^-1 =
+        // out + x2 * bsMod^-1 as the second half's b
+#pragma unroll 1
+        for (int t = 0; t < 16; t++) {
+            const int k = u + kNttGroup * t;
 #pragma unroll
-        for (int it = 0; it < kPerThread; it++) {
-            const int k = tid + it * kNttThreads;
-            shifted(a.inter_bs, R.wo)[R.comp * kN + k] = S[pidx(tid) + it * kPadStep];
+            for (int c = 0; c < COMPS; c++) {
+                const int comp = COMPS == 2 ? c : comp0;
+                const uint32_t o = *cb_at(comp, k);   // this thread's own store
+                const uint32_t x2 = canon_lazy(S[2 * c * kPadN + pidx(u) + t * kPadGroupStep], cc);
+                if (comp == 0)
+                    shifted(a.interA, wo)[ch * kN + k] = reduce64((uint64_t)o * kBsMod + x2, cc.q, cc.barrett);
+                else
+                    shifted(a.inter_dig, wo)[(size_t)(ch * kN + k) * 4 + 3] =
+                        addmod(o, shoup_mul(x2, cc.bsinv, cc.bsinv_p, cc.q), cc.q);
+            }
         }
     }
 }
 
-// Prime ch of the rotation: NTT_ch(x2) from S (in place), the crt
-// multiply-accumulate, the modswitch, and the cipherbuf store.  Starts with
-// a barrier (x2 complete, tws free) and stages the forward twiddles itself.
-template <int ELL, class Sync = CtaSync>
-__device__ __forceinline__ void baby_crt_part(const BabyRot& R, const BabyArgs& a, uint32_t* S, uint2* tws,
-                                              const NttTables& tabs, int ch) {
-    const int tid = R.tid, comp = R.comp;
-    const uint16_t* __restrict__ sig = a.sigma + (size_t)R.ki * kN;
-    uint32_t* cb32 = reinterpret_cast<uint32_t*>(shifted(a.cipherbuf, R.wo));
-    uint32_t* inter_out = shifted(comp == 0 ? a.interA : a.interB, R.wo);
-    Sync::sync();   // x2 complete and the previous twiddles no longer read
-    stage_twiddles(tws, tabs, ch, NTT_FWD);
-    cta_ntt_forward<Sync, true>(S, tws, ch);   // NTT_ch(x2), x2 < bsMod < q; outputs in [0, 4q)
-
-    const ChanConst cc = c_dev.ch[ch];
-    int pk[kPerThread];
-    baby_perm(R, pk);
-    uint64_t acc[kPerThread];
-#pragma unroll
-    for (int it = 0; it < kPerThread; it++) acc[it] = 0;
-#pragma unroll
-    for (int j = 0; j < ELL; j++) {
-        const uint32_t* d = shifted(a.dig, R.wo) + (size_t)(j * 3 + ch) * kN;
-        const uint32_t* kk = R.kcrt + (size_t)((j * 2 + comp) * 2 + ch) * kN;
-#pragma unroll
-        for (int it = 0; it < kPerThread; it++)
-            acc[it] += (uint64_t)ld_query<Sync>(d + pk[it]) * __ldg(kk + tid + it * kNttThreads);
-    }
-#pragma unroll
-    for (int it = 0; it < kPerThread; it++) {
-        const int k = tid + it * kNttThreads;
-        uint32_t A = negmod(mod_crt(acc[it], ch), cc.q);
-        if (comp == 1) A = addmod(A, ld_query<Sync>(shifted(a.srcB, R.wo) + ch * kN + sig[k]), cc.q);
-        if (R.inter) inter_out[ch * kN + k] = A;
-        // (A - S) bsMod^-1 with S in [0, 4q): A + 4q - S is in (0, 5q), and the
-        // Shoup product reduces any 32-bit input to a canonical residue
-        const uint32_t r = shoup_mul(A + 2 * cc.two_q - S[pidx(tid) + it * kPadStep], cc.bsinv, cc.bsinv_p, cc.q);
-        if (a.cb_rm)
-            cb32[cipherbuf_rm_idx(R.col, comp, ch, k)] = r;
-        else
-            cb32[(((size_t)k * a.N1 + R.col) * 2 + comp) * 2 + ch] = r;
-    }
-}
-
-// One CTA per (rotation, component): blockIdx.x = 2*ki + comp, blockIdx.y =
-// query of the batch.  The bsMod part runs once for both primes (six
-// transforms per rotation; a shape with one CTA per prime as well, which
-// recomputes it, ran eight and measured slower for single queries too once
-// the reductions were minimum-form).  MINB 2: at 3 CTAs per SM (40-42 registers) it spills, and
-// measured slower (batch of 64: baby steps 1.55 ms at 3, 1.32 ms at 2).
-template <int ELL, int MINB>
-__global__ void __launch_bounds__(kNttThreads, MINB) k_baby_pair(BabyArgs a, ClientKeysDev keys, NttTables tabs, Batch bt) {
+// Both components of a rotation per CTA (batches: one digit gather and one set
+// of forward twiddles for both), or one (single queries: 126 CTAs instead of
+// 63): blockIdx.x = ki, or 2 ki + comp; blockIdx.y = query of the batch.
+template <int COMPS>
+__global__ void __launch_bounds__(kNttThreads, 2) k_baby_rot(BabyArgs a, ClientKeysDev keys, NttTables tabs, Batch bt) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);
-    uint32_t* S2 = S + kPadN;
-    BabyRot R;
     pdl_launch_dependents();
-    stage_twiddles(tws, tabs, CH_BS, NTT_INV);
-    baby_setup<ELL>(R, a, keys, bt, blockIdx.x >> 1, blockIdx.x & 1);
+    if (COMPS == 1) {
+        warm_twiddles(tabs, CH_BS, NTT_INV, threadIdx.x, kNttThreads);
+        warm_twiddles(tabs, thread_group(), NTT_FWD, threadIdx.x & (kNttGroup - 1), kNttGroup);
+    }
     pdl_wait();   // the digits come from the previous kernel
-    baby_bs_part<ELL>(R, a, S, tws, true);
-    // the second prime transforms its own copy of x2 (each thread copies the
-    // coefficients it wrote: no barrier needed)
-#pragma unroll
-    for (int it = 0; it < kPerThread; it++) S2[pidx(R.tid) + it * kPadStep] = S[pidx(R.tid) + it * kPadStep];
-    baby_crt_part<ELL>(R, a, S, tws, tabs, 0);
-    baby_crt_part<ELL>(R, a, S2, tws, tabs, 1);
+    baby_rotation<COMPS, CtaSync>(reinterpret_cast<uint32_t*>(smem_raw), a, keys, tabs, bt,
+                                  COMPS == 2 ? blockIdx.x : blockIdx.x >> 1, blockIdx.x & 1);
 }
 
 }  // namespace kspir

@@ -74,14 +74,12 @@ struct ClientQueryArgs {
     uint32_t* out;             // [n][3 ch][2 (a, b)][N] residues, coefficient form
 };
 
-constexpr int kClientSmem = 2 * kN * 8 + 3 * kPadN * 4;   // forward + inverse twiddles, 3 polynomials
+constexpr int kClientSmem = 3 * kPadN * 4;   // 3 polynomials
 
 // grid (3 channels: q1, q2, bsMod; n queries), 512 threads
 __global__ void __launch_bounds__(kNttThreads) k_client_query(ClientQueryArgs a, NttTables tabs) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* twf = reinterpret_cast<uint2*>(smem_raw);
-    uint2* twi = twf + kN;
-    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw + 2 * kN * 8);
+    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw);
     uint32_t* A = S + kPadN;
     uint32_t* T = A + kPadN;
     const int ch = blockIdx.x == 0 ? CH_Q1 : blockIdx.x == 1 ? CH_Q2 : CH_BS;
@@ -90,17 +88,14 @@ __global__ void __launch_bounds__(kNttThreads) k_client_query(ClientQueryArgs a,
     const uint64_t* s = a.secrets + (size_t)qi * kN;
     const uint32_t row = a.rows[qi];
 
-    // me = INTT_p(m) first (its twiddles in twf), then the channel's tables
-    stage_twiddles(twf, tabs, CH_P, NTT_INV);
+    // me = INTT_p(m) first
     for (int i = tid; i < kN; i += kNttThreads) T[pidx(i)] = 0;
     __syncthreads();
     if (tid == 0) {
         T[pidx(a.qenc[row])] = 1;
         T[pidx(a.qenc[kN - 1 - row])] = 1;
     }
-    cta_ntt_inverse(T, twf, CH_P);
-    stage_twiddles(twf, tabs, ch, NTT_FWD);
-    stage_twiddles(twi, tabs, ch, NTT_INV);
+    cta_ntt_inverse_m<1>(T, kPadN, tabs, CH_P);
     const uint32_t bsq = ch == CH_BS ? 0u : (uint32_t)(kBsMod % q);
     for (int i = tid; i < kN; i += kNttThreads) {
         const uint32_t e = client_err(a.seed, qi, i, q);
@@ -115,12 +110,12 @@ __global__ void __launch_bounds__(kNttThreads) k_client_query(ClientQueryArgs a,
         const uint32_t stream = ch == CH_Q1 ? RS_A_Q1 : ch == CH_Q2 ? RS_A_Q2 : RS_A_BS;
         A[pidx(i)] = (uint32_t)(client_rand64(a.seed, qi, stream, i) % q);
     }
-    cta_ntt_forward_m<2>(S, 2 * kPadN, twf, ch);   // S and T
+    cta_ntt_forward_m<2>(S, 2 * kPadN, tabs, ch);   // S and T
     for (int i = tid; i < kN; i += kNttThreads) {
         const int p = pidx(i);
         S[p] = addmod(mulmod(A[p], S[p], ch), T[p], q);   // b = a * s + t, NTT form
     }
-    cta_ntt_inverse_m<2>(S, kPadN, twi, ch);           // b (S) and a (A) to coefficient form
+    cta_ntt_inverse_m<2>(S, kPadN, tabs, ch);           // b (S) and a (A) to coefficient form
     uint32_t* o = a.out + ((size_t)qi * 3 + (ch == CH_Q1 ? 0 : ch == CH_Q2 ? 1 : 2)) * 2 * kN;
     for (int i = tid; i < kN; i += kNttThreads) {
         o[i] = A[pidx(i)];
@@ -146,29 +141,25 @@ __global__ void __launch_bounds__(kNttThreads) k_client_decrypt(const uint64_t* 
                                                                 const uint64_t* __restrict__ resp, uint64_t qinv,
                                                                 uint32_t* __restrict__ out, NttTables tabs) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* twf = reinterpret_cast<uint2*>(smem_raw);
-    uint2* twi = twf + kN;
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw + 2 * kN * 8);   // a, b, s
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);   // a, b, s
     const int ch = blockIdx.x;
     const uint32_t qi = blockIdx.y, tid = threadIdx.x;
     const uint32_t q = c_dev.ch[ch].q;
     const uint64_t* rp = resp + (size_t)qi * 2 * kN;
     const uint64_t* s = secrets + (size_t)qi * kN;
-    stage_twiddles(twf, tabs, ch, NTT_FWD);
-    stage_twiddles(twi, tabs, ch, NTT_INV);
     for (int i = tid; i < kN; i += kNttThreads) {
         P[pidx(i)] = (uint32_t)(rp[i] % q);
         P[kPadN + pidx(i)] = (uint32_t)(rp[kN + i] % q);
         P[2 * kPadN + pidx(i)] = (uint32_t)(s[i] % q);
     }
-    cta_ntt_forward_m<3>(P, kPadN, twf, ch);
+    cta_ntt_forward_m<3>(P, kPadN, tabs, ch);
     const uint32_t qv = (uint32_t)(qinv % q);
     for (int i = tid; i < kN; i += kNttThreads) {
         const int p = pidx(i);
         const uint32_t as = mulmod(P[p], P[2 * kPadN + p], ch);
         P[kPadN + p] = mulmod(submod(P[kPadN + p], as, q), qv, ch);   // INTT is linear: scale first
     }
-    cta_ntt_inverse(P + kPadN, twi, ch);
+    cta_ntt_inverse_m<1>(P + kPadN, kPadN, tabs, ch);
     uint32_t* o = out + ((size_t)qi * 2 + ch) * kN;
     for (int i = tid; i < kN; i += kNttThreads) o[i] = P[kPadN + pidx(i)];
 }

@@ -29,8 +29,8 @@
 namespace kspir {
 
 constexpr int kDbRowsPerCta = 4;
-// twiddles of one (channel, direction) + 4 polynomials mod q1 + 4 mod q2
-constexpr int kDbRowsSmem = kN * 8 + 2 * kDbRowsPerCta * kPadN * 4;
+// 4 polynomials mod q1 + 4 mod q2
+constexpr int kDbRowsSmem = 2 * kDbRowsPerCta * kPadN * 4;
 
 // Entry D[R][c] of the diagonal rearrangement of one sub-database.
 __device__ __forceinline__ size_t db_diag_index(int R, int c) {
@@ -51,15 +51,12 @@ __global__ void __launch_bounds__(kNttThreads, 1)
 k_db_rows(const uint64_t* __restrict__ raw, const uint16_t* __restrict__ gtab, uint64_t* __restrict__ out,
           uint64_t* __restrict__ rows, int N1, NttTables tabs) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint8_t* smem = smem_raw;
-    uint2* tws = reinterpret_cast<uint2*>(smem);
-    uint32_t* s1 = reinterpret_cast<uint32_t*>(smem + kN * 8);    // 4 rows, mod p then mod q1
+    uint32_t* s1 = reinterpret_cast<uint32_t*>(smem_raw);         // 4 rows, mod p then mod q1
     uint32_t* s2 = s1 + kDbRowsPerCta * kPadN;                    // 4 rows, mod q2
     const int R0 = blockIdx.x * kDbRowsPerCta;
     const size_t sub = (size_t)blockIdx.y * kN * (kN / 2);
     const uint64_t* data = raw + sub;
 
-    stage_twiddles(tws, tabs, CH_P, NTT_INV);
 #pragma unroll
     for (int t = 0; t < kDbRowsPerCta; t++) {
         const int R = R0 + t;
@@ -67,21 +64,16 @@ k_db_rows(const uint64_t* __restrict__ raw, const uint16_t* __restrict__ gtab, u
         for (int m = threadIdx.x; m < kN; m += kNttThreads)
             s1[t * kPadN + pidx(m)] = (uint32_t)__ldg(data + db_diag_index(R, __ldg(g + m)));
     }
-    cta_ntt_inverse_m<kDbRowsPerCta>(s1, kPadN, tws, CH_P);
+    cta_ntt_inverse_m<kDbRowsPerCta>(s1, kPadN, tabs, CH_P);
 
-    // lift to signed and split per prime; the forward twiddles of q1 replace p's
-    const uint32_t q1 = c_dev.ch[CH_Q1].q, q2 = c_dev.ch[CH_Q2].q;
+    // lift to signed: the same small word serves both primes
     constexpr uint32_t half = kP / 2;
     for (int k = threadIdx.x; k < kDbRowsPerCta * kPadN; k += kNttThreads) {
         const uint32_t v = s1[k];
-        s1[k] = v > half ? v + (q1 - kP) : v;
-        s2[k] = v > half ? v + (q2 - kP) : v;
+        s1[k] = s2[k] = v > half ? v - kP : v;
     }
-    __syncthreads();
-    stage_twiddles(tws, tabs, CH_Q1, NTT_FWD);
-    cta_ntt_forward_m<kDbRowsPerCta>(s1, kPadN, tws, CH_Q1);
-    stage_twiddles(tws, tabs, CH_Q2, NTT_FWD);
-    cta_ntt_forward_m<kDbRowsPerCta>(s2, kPadN, tws, CH_Q2);
+    cta_ntt_forward_m<kDbRowsPerCta, CtaSync, false>(s1, kPadN, tabs, CH_Q1);
+    cta_ntt_forward_m<kDbRowsPerCta, CtaSync, false>(s2, kPadN, tabs, CH_Q2);
 
     if (ROWS) {
         // the canonical value mod crtMod of each slot, row by row (coalesced)

@@ -171,7 +171,7 @@ __global__ void k_off_decomp(const uint64_t* __restrict__ in, uint32_t* __restri
 }
 
 constexpr int kOffPolys = kOffEll + 1;                       // b and the five digits
-constexpr int kOffSmem = kN * 8 + kOffPolys * kPadN * 4;     // twiddles + six padded polynomials
+constexpr int kOffSmem = kOffPolys * kPadN * 4;              // six padded polynomials
 
 // (b) per row j and channel slot s (0, 1: q1, q2; 2.. : the second modulus):
 // transforms of b and of the digits, the key products with the offline key
@@ -185,18 +185,16 @@ __global__ void __launch_bounds__(kNttThreads) k_off_keyswitch(const uint32_t* _
                                                                uint32_t* __restrict__ res, NttTables tabs,
                                                                OffChain ch) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);   // [b, d0..d4][N]
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);   // [b, d0..d4][N]
     const int j = blockIdx.y, s = blockIdx.x;
     const int chan = s == 0 ? CH_Q1 : s == 1 ? CH_Q2 : off_chan2(ch, s - 2);
     const int ell = ch.g.ell;
     const int tid = threadIdx.x;
     const uint32_t q = c_dev.ch[chan].q;
     const uint64_t bar = c_dev.ch[chan].barrett;
-    stage_twiddles(tws, tabs, chan, NTT_FWD);
     poly_to_smem(P, bres + ((size_t)j * 4 + s) * kN);
     for (int i = 0; i < ell; i++) poly_to_smem(P + (1 + i) * kPadN, dig + (((size_t)j * kOffEll + i) * 4 + s) * kN);
-    cta_ntt_forward_m<kOffPolys>(P, kPadN, tws, chan);
+    cta_ntt_forward_m<kOffPolys>(P, kPadN, tabs, chan);
     const int krow0 = s < 2 ? 0 : kOffEll;   // offline key rows of this modulus
     uint32_t outa[kN / kNttThreads], outb[kN / kNttThreads];
 #pragma unroll
@@ -220,8 +218,7 @@ __global__ void __launch_bounds__(kNttThreads) k_off_keyswitch(const uint32_t* _
         P[pk] = outa[it];
         P[kPadN + pk] = outb[it];
     }
-    stage_twiddles(tws, tabs, chan, NTT_INV);   // the forward transforms ended with a barrier
-    cta_ntt_inverse_m<2>(P, kPadN, tws, chan);
+    cta_ntt_inverse_m<2>(P, kPadN, tabs, chan);
     uint32_t* o = res + ((size_t)j * 4 + s) * 2 * kN;
     poly_from_smem(o, P);
     poly_from_smem(o + kN, P + kPadN);
@@ -282,17 +279,15 @@ __global__ void __launch_bounds__(kNttThreads) k_off_intt_key(const uint32_t* __
                                                               uint32_t* __restrict__ res, NttTables tabs,
                                                               OffChain ch) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);
     const int row = blockIdx.z, comp = blockIdx.y, s = blockIdx.x;
     const int j = row % kOffRows;
     const bool second = row >= kOffRows;
     if ((second && s >= ch.nch2) || (!second && s >= 2)) return;   // the whole CTA leaves together
     const int slot = second ? 2 + s : s;
     const int chan = slot == 0 ? CH_Q1 : slot == 1 ? CH_Q2 : off_chan2(ch, slot - 2);
-    stage_twiddles(tws, tabs, chan, NTT_INV);
     poly_to_smem(P, kres + ((size_t)row * 2 + comp) * 4 * kN + (size_t)slot * kN);
-    cta_ntt_inverse(P, tws, chan);
+    cta_ntt_inverse_m<1>(P, kPadN, tabs, chan);
     poly_from_smem(res + (((size_t)j * 4 + slot) * 2 + comp) * kN, P);
 }
 
@@ -306,14 +301,12 @@ __global__ void __launch_bounds__(kNttThreads) k_off_modswitch(const uint64_t* _
                                                                uint32_t* __restrict__ res, uint64_t aux_inv,
                                                                NttTables tabs) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);
     const int ch = blockIdx.x & 1, comp = (blockIdx.x >> 1) & 1, j = (blockIdx.x >> 2) % kOffRows;
     const int key = blockIdx.x / (4 * kOffRows);
     const uint32_t q = c_dev.ch[ch].q;
     const uint64_t bar = c_dev.ch[ch].barrett;
     const uint32_t ainv = (uint32_t)(aux_inv % q);
-    stage_twiddles(tws, tabs, ch, NTT_FWD);
     const uint64_t* kw = keys + (size_t)key * 6 * 2 * kN;
     const uint64_t* a = kw + ((size_t)j * 2 + comp) * kN;
     const uint64_t* x = kw + ((size_t)(j + kOffRows) * 2 + comp) * kN;
@@ -322,7 +315,7 @@ __global__ void __launch_bounds__(kNttThreads) k_off_modswitch(const uint64_t* _
         const uint64_t v = av >= xv ? av - xv : av + kCrtMod - xv;   // EltwiseSubMod, both below crtMod
         P[pidx(k)] = reduce64((uint64_t)(uint32_t)(v % q) * ainv, q, bar);
     }
-    cta_ntt_forward(P, tws, ch);
+    cta_ntt_forward_m<1>(P, kPadN, tabs, ch);
     poly_from_smem(res + (((size_t)key * kOffRows + j) * 2 + comp) * 2 * kN + (size_t)ch * kN, P);
 }
 

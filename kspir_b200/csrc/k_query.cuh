@@ -9,8 +9,10 @@ namespace kspir {
 // Per coefficient k of the caller's query (coefficient form, reference
 // encrypt.cpp:488-493):
 //  * digits of decompose_bsgs(query a mod crtMod, query a mod bsMod)
-//    (evalAutoSRNSFirst, twosteps.cpp:960-968), as residues of q1, q2, bs;
-//  * query b as residues (its crt transform feeds the hoisted b terms);
+//    (evalAutoSRNSFirst, twosteps.cpp:960-968), signed words that serve the
+//    three channels;
+//  * query b: times bsMod^-1 per prime (its crt transform is the b term of the
+//    modswitched rotations), and mod bsMod;
 //  * the RNS modswitch of the query itself, (x_crt - x_bs) * bsMod^-1 mod
 //    crtMod (twosteps.cpp:1073-1086), as residues before its transform.
 // k < N; ws is already the query's workspace slot.
@@ -19,18 +21,14 @@ __device__ __forceinline__ void query_prep_one(const Workspace& ws, const Gadget
     const uint32_t a_bs = (uint32_t)ws.q64[2 * kN + k], b_bs = (uint32_t)ws.q64[3 * kN + k];
     int32_t dig[kMaxEll];
     decompose_bsgs(a_crt, a_bs, g, dig);
-    for (int j = 0; j < g.ell; j++) {
-        ws.dig0[(j * 3 + CH_Q1) * kN + k] = signed_to_res(dig[j], kQ1);
-        ws.dig0[(j * 3 + CH_Q2) * kN + k] = signed_to_res(dig[j], kQ2);
-        ws.dig0[(j * 3 + CH_BS) * kN + k] = signed_to_res(dig[j], kBsMod);
-    }
-    const uint32_t bq1 = mod_q1(b_crt), bq2 = mod_q2(b_crt);
-    ws.qbn[k] = bq1;
-    ws.qbn[kN + k] = bq2;
-    ws.qbbs[k] = b_bs;
-    const uint32_t aq1 = mod_q1(a_crt), aq2 = mod_q2(a_crt);
+    for (int j = 0; j < g.ell; j++) ws.digraw[j * kN + k] = (uint32_t)dig[j];
     const ChanConst& c1 = c_dev.ch[CH_Q1];
     const ChanConst& c2 = c_dev.ch[CH_Q2];
+    const uint32_t bq1 = mod_q1(b_crt), bq2 = mod_q2(b_crt);
+    ws.qb[k] = shoup_mul(bq1, c1.bsinv, c1.bsinv_p, kQ1);
+    ws.qb[kN + k] = shoup_mul(bq2, c2.bsinv, c2.bsinv_p, kQ2);
+    ws.qb[2 * kN + k] = b_bs;
+    const uint32_t aq1 = mod_q1(a_crt), aq2 = mod_q2(a_crt);
     ws.col0[0 * kN + k] = shoup_mul(submod(aq1, a_bs, kQ1), c1.bsinv, c1.bsinv_p, kQ1);
     ws.col0[1 * kN + k] = shoup_mul(submod(aq2, a_bs, kQ2), c2.bsinv, c2.bsinv_p, kQ2);
     ws.col0[2 * kN + k] = shoup_mul(submod(bq1, b_bs, kQ1), c1.bsinv, c1.bsinv_p, kQ1);
@@ -61,11 +59,7 @@ __device__ __forceinline__ void inter_decomp_one(const Workspace& ws, const Gadg
     const uint32_t a_bs = __ldcg(ws.inter_bs + k);
     int32_t dig[kMaxEll];
     decompose_bsgs(a_crt, a_bs, g, dig);
-    for (int j = 0; j < g.ell; j++) {
-        ws.dig1[(j * 3 + CH_Q1) * kN + k] = signed_to_res(dig[j], kQ1);
-        ws.dig1[(j * 3 + CH_Q2) * kN + k] = signed_to_res(dig[j], kQ2);
-        ws.dig1[(j * 3 + CH_BS) * kN + k] = signed_to_res(dig[j], kBsMod);
-    }
+    for (int j = 0; j < g.ell; j++) ws.digraw[j * kN + k] = (uint32_t)dig[j];
 }
 
 __global__ void k_inter_decomp(Workspace ws, GadgetBsgs g, Batch bt) {

@@ -10,11 +10,43 @@
 // external product remain for the allocation-free entry point.
 #pragma once
 
+#include "k_baby.cuh"
 #include "ntt.cuh"
 #include "pipeline.cuh"
 #include "ptx.cuh"
 
 namespace kspir {
+
+// The key products of a thread's coefficients u + 256 (4 v + w), w = 0..3, on prime
+// ch: ra, rb = sum over the ROWS polynomials d (in shared memory at stride
+// `dstride`, lazy signed words below 6.7 q) times the keys of components a
+// and b, reduced to within +-1 q.  The keys (lane order, centred, times +-2^32:
+// k_keys_from_words) come as one 16-byte vector per row and component, at
+// `krow` vectors between rows and `kcomp` between components.
+// |sum| <= ROWS 6.7 q q / 2 < 2^60; / 2^32 it is 0.21 ROWS q at most, and the
+// Montgomery term adds q / 2: within +-q for ROWS = 2, +-1.4 q for ROWS = 4.
+template <int ROWS>
+__device__ __forceinline__ void key_mac4(const uint32_t* d, int dstride, const uint4* __restrict__ key, int krow,
+                                         int kcomp, int ch, uint32_t* ra, uint32_t* rb) {
+    uint64_t sa[4] = {0, 0, 0, 0}, sb[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < ROWS; j++) {
+        const uint4 ka = __ldg(key + j * krow), kb = __ldg(key + j * krow + kcomp);
+        const uint32_t kaw[4] = {ka.x, ka.y, ka.z, ka.w}, kbw[4] = {kb.x, kb.y, kb.z, kb.w};
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            const uint32_t dv = d[j * dstride + w * kPadGroupStep];
+            mad_wide_s(sa[w], dv, kaw[w]);
+            mad_wide_s(sb[w], dv, kbw[w]);
+        }
+    }
+    const ChanConst& cc = c_dev.ch[ch];
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        ra[w] = mont_redc(sa[w], cc);
+        rb[w] = mont_redc(sb[w], cc);
+    }
+}
 
 // ---------------------------------------------------------------------------
 // giant steps
@@ -45,7 +77,7 @@ __global__ void k_ext_decomp(const uint32_t* __restrict__ ecoef, uint32_t* __res
 }
 
 // dynamic shared memory of the fused multiply-accumulate + inverse-transform kernels
-constexpr int kMacSmem = kN * 8 + kPadN * 4;
+constexpr int kMacSmem = kPadN * 4;
 
 // One CTA per (r, comp, ch): ext = INTT( init + sum_row digit_row * rgsw[row].comp ),
 // init being the caller's NTT-domain accumulator (zero on the answer path,
@@ -55,12 +87,10 @@ __global__ void __launch_bounds__(kNttThreads) k_ext_mac_intt(const uint32_t* __
                                                               const uint32_t* __restrict__ init,
                                                               uint32_t* __restrict__ ext, int rows, NttTables tabs) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* s = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);
+    uint32_t* s = reinterpret_cast<uint32_t*>(smem_raw);
     constexpr int T = kNttThreads;
     const int ch = blockIdx.x % 2, comp = (blockIdx.x / 2) % 2, r = blockIdx.x / 4;
     const ChanConst cc = c_dev.ch[ch];
-    stage_twiddles(tws, tabs, ch, NTT_INV);
     const uint32_t* d = edig + (size_t)r * rows * 2 * kN;
 #pragma unroll
     for (int k = threadIdx.x; k < kN; k += T) {
@@ -70,7 +100,7 @@ __global__ void __launch_bounds__(kNttThreads) k_ext_mac_intt(const uint32_t* __
         const uint32_t m = reduce64(acc, cc.q, cc.barrett);
         s[pidx(k)] = init ? addmod(init[((size_t)r * 4 + comp * 2 + ch) * kN + k], m, cc.q) : m;
     }
-    cta_ntt_inverse(s, tws, ch);
+    cta_ntt_inverse_m<1>(s, kPadN, tabs, ch);
     uint32_t* o = ext + ((size_t)r * 4 + comp * 2 + ch) * kN;
 #pragma unroll
     for (int k = threadIdx.x; k < kN; k += T) o[k] = s[pidx(k)];
@@ -95,92 +125,94 @@ static_assert((uint64_t)kGiantTermsPerAcc * (kQ1 - 1) < (1ull << 32) && kQ2 < kQ
 
 constexpr int kGiantPolys = 4;   // two primes x two digits (ell = 2)
 constexpr int kPerThreadG = kN / kNttThreads;
-// The transforms read the device twiddle tables through L1 rather than a
-// staged shared-memory copy: 72 KiB of shared memory and 40 registers give 3
-// CTAs per SM (a staged copy made it 104 KiB and 2 CTAs per SM, 8 % slower).
 constexpr int kGiantSmem = kGiantPolys * kPadN * 4;
 
-template <int ELL>
-__global__ void __launch_bounds__(kNttThreads, 3)
-    k_giant_fused(const uint32_t* __restrict__ sout, uint32_t* acc0, uint32_t* acc1,
-                  const uint32_t* __restrict__ gkeys, const uint16_t* __restrict__ gsigma, int N1, NttTables tabs,
-                  GadgetB g, int R, Batch bt) {
+// The key switch of output row `row` (= r N2 + c) into acc ([comp][prime][N] of
+// sub-database r), by 512 threads.  Each 256-thread group runs one prime: its
+// inverse transform of a, and, after both have met for the decomposition,
+// the transforms of the two digits (one set of twiddle loads for both) and
+// the key products.  Bounded by the multiply pipe and instruction issue (57 and
+// 54 % busy at 2 CTAs per SM; the six transforms alone take 0.75 of the 1.18 ms
+// of a batch of 64 at r = 16, which was 1.56 ms with conditional-subtraction
+// radix-8 transforms and 64-bit Barrett reductions).
+template <int ELL, class Sync>
+__device__ __forceinline__ void giant_body(uint32_t* P, const uint32_t* __restrict__ sout, uint32_t* acc,
+                                           const uint32_t* __restrict__ gkeys, const uint16_t* __restrict__ gsigma,
+                                           int N1, const NttTables& tabs, const GadgetB& g, int row, int c, int rows) {
     static_assert(2 * ELL <= kGiantPolys, "shared-memory polynomials");
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);   // [kGiantPolys][N]
-    const int N2 = kN / 2 / N1;
-    const int rows = R * N2;
-    const int rc = blockIdx.x;
-    const int r = rc / (N2 - 1), c = rc % (N2 - 1) + 1;
-    const int row = r * N2 + c;
-    const int tid = threadIdx.x;
-    sout = shifted(sout, ws_off(bt));
-    gkeys = shifted(gkeys, key_off(bt));
-    uint32_t* acc = shifted((acc1 && !(c & 1)) ? acc1 : acc0, ws_off(bt)) + (size_t)r * 4 * kN;
-    pdl_launch_dependents();
+    const int ch = thread_group(), u = threadIdx.x & (kNttGroup - 1);
 
-    // a of output[c], both primes, to coefficient form
+    // a of output[c] on this group's prime, to coefficient form
 #pragma unroll
-    for (int ch = 0; ch < 2; ch++) {
-        pdl_wait();   // the scan output comes from the previous kernel
-#pragma unroll
-        for (int k = tid; k < kN / 4; k += kNttThreads)
-            *reinterpret_cast<uint4*>(P + ch * kPadN + pidx(4 * k)) =
-                __ldcg(reinterpret_cast<const uint4*>(sout + sout_idx(row, 0 * 2 + ch, 4 * k, rows)));
-        cta_ntt_inverse(P + ch * kPadN, twiddle_table(tabs, ch, NTT_INV), ch);
-    }
-    // X -> X^g, g = 5^(N1 c), then the digits (registers first: P is overwritten)
+    for (int k = u; k < kN / 4; k += kNttGroup)
+        *reinterpret_cast<uint4*>(P + ch * kPadN + pidx(4 * k)) =
+            __ldcg(reinterpret_cast<const uint4*>(sout + sout_idx(row, 0 * 2 + ch, 4 * k, rows)));
+    GroupSync::sync();
+    group_ntt_inverse<1, GroupSync>(P + ch * kPadN, kPadN, tabs, ch, u);
+    Sync::sync();
+    // X -> X^g, g = 5^(N1 c), then the digits (registers first: P is overwritten).
+    // g = 1 mod 256 (N1 >= 64), so coefficient u + 256 t comes from u + 256 h with
+    // h = (u g^-1 >> 8) + t g^-1 mod 32, negated when h >= 16.
     const uint32_t e = (uint32_t)(N1 * c) & 2047u;
     uint32_t ginv = 1, b5 = 5, x = (2048u - e) & 2047u;
     while (x) { if (x & 1) ginv = (ginv * b5) & (2 * kN - 1); b5 = (b5 * b5) & (2 * kN - 1); x >>= 1; }
-    uint32_t dres[kPerThreadG][ELL][2];
+    int32_t dres[kPerThreadG][ELL];
+    uint32_t h = ((u * ginv) >> 8) + 8 * ch * ginv;
+    const uint32_t* Pu = P + pidx(u);
 #pragma unroll
-    for (int it = 0; it < kPerThreadG; it++) {
-        const int k = tid + it * kNttThreads;
-        bool neg;
-        const int src = auto_src(k, ginv, &neg);
-        uint64_t v = crt_compose_res(P[pidx(src)], P[kPadN + pidx(src)]);
-        if (neg && v) v = kCrtMod - v;
-        int32_t dig[kMaxEll];
-        decompose_b(v, kCrtMod, g, dig);
-#pragma unroll
-        for (int j = 0; j < ELL; j++) {
-            dres[it][j][0] = signed_to_res(dig[j], kQ1);
-            dres[it][j][1] = signed_to_res(dig[j], kQ2);
-        }
+    for (int it = 0; it < kPerThreadG; it++) {   // coefficient u + 256 (8 ch + it)
+        const uint32_t* src = Pu + (h & 15) * kPadGroupStep;
+        decompose_b_res<ELL>(src[0], src[kPadN], h & 16, g, dres[it]);
+        h += ginv;
     }
-    __syncthreads();
+    Sync::sync();
+    // a digit is a small signed word, the same for both primes
 #pragma unroll
     for (int it = 0; it < kPerThreadG; it++)
 #pragma unroll
         for (int j = 0; j < ELL; j++)
 #pragma unroll
-            for (int ch = 0; ch < 2; ch++) P[(j * 2 + ch) * kPadN + pidx(tid) + it * kPadStep] = dres[it][j][ch];
-    // digit transforms and the key multiply-accumulate, prime by prime
-    const uint32_t* key = gkeys + (size_t)(c - 1) * ELL * 2 * 2 * kN;   // [ELL][2 comp][2 ch][N]
+            for (int p = 0; p < 2; p++)
+                P[(p * ELL + j) * kPadN + pidx(u) + (8 * ch + it) * kPadGroupStep] = (uint32_t)dres[it][j];
+    uint32_t* D = P + ch * ELL * kPadN;
+    Sync::sync();
+    group_ntt_forward<ELL, GroupSync, true>(D, kPadN, tabs, ch, u);   // signed, below 6.7 q
+    const uint32_t q = c_dev.ch[ch].q;
+    const uint4* key = reinterpret_cast<const uint4*>(gkeys + (size_t)(c - 1) * ELL * 4 * kN + (size_t)ch * kN);
     const uint16_t* sig = gsigma + (size_t)(c - 1) * kN;
-#pragma unroll 1
-    for (int ch = 0; ch < 2; ch++) {
-        __syncthreads();
-        // digits j of this prime: P[j*2+ch], left in [0, 4q) (they only feed the
-        // exact multiply-accumulate below)
-        cta_ntt_forward_m<ELL, CtaSync, true>(P + ch * kPadN, 2 * kPadN, twiddle_table(tabs, ch, NTT_FWD), ch);
-        const ChanConst cc = c_dev.ch[ch];
+    uint32_t* acc_a = acc + (size_t)ch * kN + u;
+    uint32_t* acc_b = acc_a + 2 * kN;
 #pragma unroll
-        for (int it = 0; it < kPerThreadG; it++) {
-            const int k = tid + it * kNttThreads;
-            uint64_t sa = 0, sb = 0;
+    for (int v = 0; v < 4; v++) {
+        const int i = v * kNttGroup + u;
+        uint32_t sl[4], ra[4], rb[4];
+        perm4(sig, i, sl);
+        uint32_t bv[4];
 #pragma unroll
-            for (int j = 0; j < ELL; j++) {
-                const uint32_t d = P[(j * 2 + ch) * kPadN + pidx(tid) + it * kPadStep];
-                mad_wide(sa, d, __ldg(key + ((j * 2 + 0) * 2 + ch) * kN + k));
-                mad_wide(sb, d, __ldg(key + ((j * 2 + 1) * 2 + ch) * kN + k));
-            }
-            const uint32_t bv = __ldcg(sout + sout_idx(row, 1 * 2 + ch, sig[k], rows));
-            atomicAdd(acc + (size_t)(0 * 2 + ch) * kN + k, negmod(mod_crt(sa, ch), cc.q));
-            atomicAdd(acc + (size_t)(1 * 2 + ch) * kN + k, addmod(bv, negmod(mod_crt(sb, ch), cc.q), cc.q));
+        for (int w = 0; w < 4; w++) bv[w] = __ldcg(sout + sout_idx(row, 1 * 2 + ch, sl[w], rows));
+        key_mac4<ELL>(D + pidx(u) + 4 * v * kPadGroupStep, kPadN, key + i, 4 * kN / 4, 2 * kN / 4, ch, ra, rb);
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            atomicAdd(acc_a + kNttGroup * (4 * v + w), canon_pm1(ra[w], q));
+            atomicAdd(acc_b + kNttGroup * (4 * v + w), canon_m1p2(rb[w] + bv[w], q));
         }
     }
+}
+
+template <int ELL>
+__global__ void __launch_bounds__(kNttThreads, 2)
+    k_giant_fused(const uint32_t* __restrict__ sout, uint32_t* acc0, uint32_t* acc1,
+                  const uint32_t* __restrict__ gkeys, const uint16_t* __restrict__ gsigma, int N1, NttTables tabs,
+                  GadgetB g, int R, Batch bt) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    const int N2 = kN / 2 / N1;
+    const int rc = blockIdx.x;
+    const int r = rc / (N2 - 1), c = rc % (N2 - 1) + 1;
+    pdl_launch_dependents();
+    pdl_wait();   // the scan output comes from the previous kernel
+    giant_body<ELL, CtaSync>(reinterpret_cast<uint32_t*>(smem_raw), shifted(sout, ws_off(bt)),
+                             shifted((acc1 && !(c & 1)) ? acc1 : acc0, ws_off(bt)) + (size_t)r * 4 * kN,
+                             shifted(gkeys, key_off(bt)), gsigma, N1, tabs, g, r * N2 + c, c, R * N2);
 }
 
 // result[r][comp][ch][k] = (output[0] + the giant-step accumulators) mod q,
@@ -223,10 +255,10 @@ namespace kspir {
 //   a' = -sum_d dig_d * key[d].a,  b' = NTT(temp.b) - sum_d dig_d * key[d].b
 //   out[j] = INTT(a', b') + c2
 constexpr int kPackPolys = 5;    // ell = 4 digits + temp.b
-constexpr int kPackSmem = kN * 8 + kPackPolys * kPadN * 4;
+constexpr int kPackSmem = kPackPolys * kPadN * 4;
 
 template <int ELL>
-__global__ void __launch_bounds__(kNttThreads) k_pack_fused(const uint32_t* __restrict__ in,
+__global__ void __launch_bounds__(kNttThreads, 2) k_pack_fused(const uint32_t* __restrict__ in,
                                                             uint32_t* __restrict__ out,
                                                             const uint32_t* __restrict__ key, int I, uint32_t ginv,
                                                             NttTables tabs, GadgetB g, Batch bt) {
@@ -235,15 +267,13 @@ __global__ void __launch_bounds__(kNttThreads) k_pack_fused(const uint32_t* __re
     in = shifted(in, ws_off(bt));
     out = shifted(out, ws_off(bt));
     key = shifted(key, key_off(bt));
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);   // [kPackPolys][N]
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);   // [kPackPolys][N]
     const int j = blockIdx.x >> 1, ch = blockIdx.x & 1;
     const int tid = threadIdx.x;
     const uint32_t* r0 = in + (size_t)j * 4 * kN;
     const uint32_t* cc = in + (size_t)(I + j) * 4 * kN;
     const uint32_t q = c_dev.ch[ch].q;
     pdl_launch_dependents();
-    stage_twiddles(tws, tabs, ch, NTT_FWD);
     pdl_wait();   // the level input comes from the previous kernel
     // launched after that kernel completes (no early launch), and no CTA writes
     // the level input: its gathers below read through L1
@@ -273,29 +303,27 @@ __global__ void __launch_bounds__(kNttThreads) k_pack_fused(const uint32_t* __re
         decompose_b(crt_compose_res(ra[0], ra[1]), kCrtMod, g, dig);
         const int pk = pidx(tid) + it * kPadStep;
 #pragma unroll
-        for (int d = 0; d < ELL; d++) P[d * kPadN + pk] = signed_to_res(dig[d], q);
+        for (int d = 0; d < ELL; d++) P[d * kPadN + pk] = (uint32_t)dig[d];
         const uint32_t vb = submod(__ldg(r0 + (1 * 2 + ch) * kN + src), cshift(1, ch, src), q);
-        P[ELL * kPadN + pk] = neg ? negmod(vb, q) : vb;
+        P[ELL * kPadN + pk] = neg ? 0u - vb : vb;
     }
-    cta_ntt_forward_m<ELL + 1, CtaSync, true>(P, kPadN, tws, ch);   // outputs in [0, 4q)
+    cta_ntt_forward_m<ELL + 1, CtaSync, true>(P, kPadN, tabs, ch);   // signed, below 6.7 q
+    const int g2 = thread_group(), u = tid & (kNttGroup - 1);
 #pragma unroll
-    for (int it = 0; it < kPerThreadG; it++) {
-        const int k = tid + it * kNttThreads;
-        uint64_t sa = 0, sb = 0;
+    for (int vv = 0; vv < 2; vv++) {
+        const int v = 2 * g2 + vv;
+        uint32_t* p = P + pidx(u) + 4 * v * kPadGroupStep;
+        uint32_t ra[4], rb[4];
+        key_mac4<ELL>(p, kPadN, reinterpret_cast<const uint4*>(key + ch * kN) + v * kNttGroup + u, 4 * kN / 4, 2 * kN / 4,
+                      ch, ra, rb);
 #pragma unroll
-        for (int d = 0; d < ELL; d++) {
-            const uint32_t dv = P[d * kPadN + pidx(tid) + it * kPadStep];
-            mad_wide(sa, dv, __ldg(key + ((d * 2 + 0) * 2 + ch) * kN + k));
-            mad_wide(sb, dv, __ldg(key + ((d * 2 + 1) * 2 + ch) * kN + k));
+        for (int w = 0; w < 4; w++) {   // only this thread reads these coefficients of the rows
+            const uint32_t b = reduce_lazy(p[ELL * kPadN + w * kPadGroupStep], c_dev.ch[ch].rq, c_dev.ch[ch].nq);
+            p[w * kPadGroupStep] = canon_pm2(ra[w], q);
+            p[kPadN + w * kPadGroupStep] = canon_pm4(rb[w] + b, q);
         }
-        const uint32_t a2 = negmod(mod_crt(sa, ch), q);
-        const int pk = pidx(tid) + it * kPadStep;
-        const uint32_t b2 = submod(canon4q(P[ELL * kPadN + pk], q), mod_crt(sb, ch), q);
-        P[pk] = a2;            // only this thread reads index k of these rows
-        P[kPadN + pk] = b2;
     }
-    stage_twiddles(tws, tabs, ch, NTT_INV);   // the forward transforms ended with a barrier
-    cta_ntt_inverse_m<2>(P, kPadN, tws, ch);
+    cta_ntt_inverse_m<2>(P, kPadN, tabs, ch);
 #pragma unroll
     for (int it = 0; it < kPerThreadG; it++) {
         const int k = tid + it * kNttThreads;
@@ -317,7 +345,7 @@ __global__ void __launch_bounds__(kNttThreads) k_pack_fused(const uint32_t* __re
 //                     inverse transform -> + c2 into out[j]
 // Same residues as k_pack_fused (sums mod q in another order).
 constexpr int kPackPartPolys = 2 * 5 * 2;   // per pair: [prime][ELL + 1][comp]
-constexpr int kPackSplitSmem = kN * 8 + kPadN * 4;
+constexpr int kPackSplitSmem = kPadN * 4;
 
 // One split forward task, pair j, prime ch, digit d (d = ELL: temp.b); in,
 // part and key already point at the query's workspace and key slot.  Shared
@@ -328,22 +356,23 @@ __device__ __forceinline__ void pack_split_fwd_body(const uint32_t* __restrict__
                                                     const NttTables& tabs, const GadgetB& g, int j, int ch, int d,
                                                     uint8_t* smem_raw) {
     static_assert(2 * (ELL + 1) * 2 <= kPackPartPolys, "term buffer");
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);
+    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw);
     const int tid = threadIdx.x;
     const uint32_t* r0 = in + (size_t)j * 4 * kN;
     const uint32_t* cc = in + (size_t)(I + j) * 4 * kN;
     const uint32_t q = c_dev.ch[ch].q;
     pdl_launch_dependents();
-    stage_twiddles(tws, tabs, ch, NTT_FWD);
+    warm_twiddles(tabs, ch, NTT_FWD, tid, kNttThreads);
     // the key words of this digit, loaded while the previous kernel finishes
     // (keys are never written by the answer), used after the transform
-    uint32_t ka[kPerThreadG], kb[kPerThreadG];
+    const int g2 = thread_group(), u = tid & (kNttGroup - 1);
+    uint4 ka[2], kb[2];
     if (d < ELL) {
+        const uint4* k4 = reinterpret_cast<const uint4*>(key + (size_t)(d * 4 + ch) * kN) + 2 * g2 * kNttGroup + u;
 #pragma unroll
-        for (int it = 0; it < kPerThreadG; it++) {
-            ka[it] = __ldg(key + ((d * 2 + 0) * 2 + ch) * kN + tid + it * kNttThreads);
-            kb[it] = __ldg(key + ((d * 2 + 1) * 2 + ch) * kN + tid + it * kNttThreads);
+        for (int vv = 0; vv < 2; vv++) {
+            ka[vv] = __ldg(k4 + vv * kNttGroup);
+            kb[vv] = __ldg(k4 + 2 * kN / 4 + vv * kNttGroup);
         }
     }
     pdl_wait();   // the level input comes from the previous kernel
@@ -368,24 +397,32 @@ __device__ __forceinline__ void pack_split_fwd_body(const uint32_t* __restrict__
             }
             int32_t dig[kMaxEll];
             decompose_b(crt_compose_res(ra[0], ra[1]), kCrtMod, g, dig);
-            v = signed_to_res(dig[d], q);
+            v = (uint32_t)dig[d];
         } else {
             const uint32_t vb = submod(__ldcg(r0 + (1 * 2 + ch) * kN + src), cshift(1, ch, src), q);
-            v = neg ? negmod(vb, q) : vb;
+            v = neg ? 0u - vb : vb;
         }
         S[pidx(tid) + it * kPadStep] = v;
     }
-    cta_ntt_forward<Sync, true>(S, tws, ch);   // outputs in [0, 4q)
+    cta_ntt_forward_m<1, Sync, true>(S, kPadN, tabs, ch);   // signed, below 6.7 q
     uint32_t* pa = part + (((size_t)j * 2 + ch) * (ELL + 1) + d) * 2 * kN;
+    const ChanConst& cc2 = c_dev.ch[ch];
 #pragma unroll
-    for (int it = 0; it < kPerThreadG; it++) {
-        const int k = tid + it * kNttThreads;
-        const uint32_t dv = S[pidx(tid) + it * kPadStep];
-        if (d < ELL) {
-            pa[k] = mod_crt((uint64_t)dv * ka[it], ch);
-            pa[kN + k] = mod_crt((uint64_t)dv * kb[it], ch);
-        } else {
-            pa[k] = canon4q(dv, q);   // NTT(temp.b)
+    for (int vv = 0; vv < 2; vv++) {
+        const uint32_t kaw[4] = {ka[vv].x, ka[vv].y, ka[vv].z, ka[vv].w}, kbw[4] = {kb[vv].x, kb[vv].y, kb[vv].z, kb[vv].w};
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            const int t = 4 * (2 * g2 + vv) + w, k = u + kNttGroup * t;
+            const uint32_t dv = S[pidx(u) + t * kPadGroupStep];
+            if (d < ELL) {   // within +-0.71 q
+                uint64_t sa = 0, sb = 0;
+                mad_wide_s(sa, dv, kaw[w]);
+                mad_wide_s(sb, dv, kbw[w]);
+                pa[k] = canon_pm1(mont_redc(sa, cc2), q);
+                pa[kN + k] = canon_pm1(mont_redc(sb, cc2), q);
+            } else {
+                pa[k] = canon_lazy(dv, cc2);   // NTT(temp.b)
+            }
         }
     }
 }
@@ -409,12 +446,11 @@ __device__ __forceinline__ void pack_split_inv_body(const uint32_t* __restrict__
                                                     uint32_t* __restrict__ out, int I, const NttTables& tabs, int j,
                                                     int ch, int comp, uint32_t* __restrict__ c2out,
                                                     uint8_t* smem_raw) {
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);
+    uint32_t* S = reinterpret_cast<uint32_t*>(smem_raw);
     const int tid = threadIdx.x;
     const uint32_t q = c_dev.ch[ch].q;
     pdl_launch_dependents();
-    stage_twiddles(tws, tabs, ch, NTT_INV);
+    warm_twiddles(tabs, ch, NTT_INV, tid, kNttThreads);
     pdl_wait();   // the terms come from the previous kernel
     const uint32_t* pj = part + ((size_t)j * 2 + ch) * (ELL + 1) * 2 * kN;
 #pragma unroll
@@ -423,8 +459,8 @@ __device__ __forceinline__ void pack_split_inv_body(const uint32_t* __restrict__
         uint32_t sum = 0;
 #pragma unroll
         for (int d = 0; d < ELL; d++) sum = addmod(sum, __ldcg(pj + ((size_t)d * 2 + comp) * kN + k), q);
-        // a' = -sum_d dig_d key[d].a ;  b' = NTT(temp.b) - sum_d dig_d key[d].b
-        S[pidx(tid) + it * kPadStep] = comp == 0 ? negmod(sum, q) : submod(__ldcg(pj + (size_t)ELL * 2 * kN + k), sum, q);
+        // a' = sum_d dig_d (-key[d].a) ;  b' = NTT(temp.b) + sum_d dig_d (-key[d].b)
+        S[pidx(tid) + it * kPadStep] = comp == 0 ? sum : addmod(__ldcg(pj + (size_t)ELL * 2 * kN + k), sum, q);
     }
     // c2 = X^I c + r of the level input, loaded ahead of the transform
     const uint32_t* r0 = in + (size_t)j * 4 * kN;
@@ -438,7 +474,7 @@ __device__ __forceinline__ void pack_split_inv_body(const uint32_t* __restrict__
         c2[it] = addmod(sh, __ldcg(r0 + (comp * 2 + ch) * kN + k), q);
         if (c2out) c2out[((size_t)(I + j) * 4 + comp * 2 + ch) * kN + k] = c2[it];
     }
-    cta_ntt_inverse<Sync>(S, tws, ch);
+    cta_ntt_inverse_m<1, Sync>(S, kPadN, tabs, ch);
 #pragma unroll
     for (int it = 0; it < kPerThreadG; it++) {
         const int k = tid + it * kNttThreads;
@@ -463,7 +499,7 @@ __global__ void __launch_bounds__(kNttThreads) k_pack_split_inv(const uint32_t* 
 // row * rgsw[row], inverse transform, into ext [comp][ch][N].  rgsw, init and
 // ext point at the query's key slot and its polynomial r.
 template <int ELL, class Sync>
-__device__ __forceinline__ void ext_tail(uint32_t* P, uint2* tws, const uint32_t* __restrict__ rgsw,
+__device__ __forceinline__ void ext_tail(uint32_t* P, const uint32_t* __restrict__ rgsw,
                                          const uint32_t* __restrict__ init, uint32_t* __restrict__ ext,
                                          const NttTables& tabs, const GadgetS& g, int ch) {
     const int tid = threadIdx.x;
@@ -478,7 +514,7 @@ __device__ __forceinline__ void ext_tail(uint32_t* P, uint2* tws, const uint32_t
             decompose_signed(crt_compose_res(P[(comp * 2 + 0) * kPadN + pk], P[(comp * 2 + 1) * kPadN + pk]), kCrtMod, g,
                              dig);
 #pragma unroll
-            for (int t = 0; t < ELL; t++) dres[it][comp * ELL + t] = signed_to_res(dig[t], ch ? kQ2 : kQ1);
+            for (int t = 0; t < ELL; t++) dres[it][comp * ELL + t] = (uint32_t)dig[t];
         }
     }
     Sync::sync();
@@ -486,31 +522,29 @@ __device__ __forceinline__ void ext_tail(uint32_t* P, uint2* tws, const uint32_t
     for (int it = 0; it < kPerThreadG; it++)
 #pragma unroll
         for (int row = 0; row < 2 * ELL; row++) P[row * kPadN + pidx(tid) + it * kPadStep] = dres[it][row];
-    stage_twiddles(tws, tabs, ch, NTT_FWD);
-    cta_ntt_forward_m<2 * ELL, Sync, true>(P, kPadN, tws, ch);   // digits in [0, 4q), for the exact sum below
-    const ChanConst cq = c_dev.ch[ch];
-    uint32_t outv[kPerThreadG][2];
+    cta_ntt_forward_m<2 * ELL, Sync, true>(P, kPadN, tabs, ch);   // signed, below 6.7 q
+    const uint32_t q = c_dev.ch[ch].q;
+    const int g2 = thread_group(), u = tid & (kNttGroup - 1);
 #pragma unroll
-    for (int it = 0; it < kPerThreadG; it++) {
-        const int k = tid + it * kNttThreads;
+    for (int vv = 0; vv < 2; vv++) {
+        const int v = 2 * g2 + vv;
+        uint32_t* p = P + pidx(u) + 4 * v * kPadGroupStep;
+        uint32_t ra[4], rb[4];
+        key_mac4<2 * ELL>(p, kPadN, reinterpret_cast<const uint4*>(rgsw + ch * kN) + v * kNttGroup + u, 4 * kN / 4,
+                          2 * kN / 4, ch, ra, rb);
 #pragma unroll
-        for (int comp = 0; comp < 2; comp++) {
-            uint64_t s = 0;
-#pragma unroll
-            for (int row = 0; row < 2 * ELL; row++)
-                mad_wide(s, P[row * kPadN + pidx(tid) + it * kPadStep], __ldg(rgsw + ((row * 2 + comp) * 2 + ch) * kN + k));
-            const uint32_t m = mod_crt(s, ch);
-            outv[it][comp] = init ? addmod(__ldcg(init + (size_t)(comp * 2 + ch) * kN + k), m, cq.q) : m;
+        for (int w = 0; w < 4; w++) {   // only this thread reads these coefficients of the rows
+            const int k = u + kNttGroup * (4 * v + w);
+            uint32_t oa = canon_pm2(ra[w], q), ob = canon_pm2(rb[w], q);
+            if (init) {
+                oa = addmod(__ldcg(init + (size_t)ch * kN + k), oa, q);
+                ob = addmod(__ldcg(init + (size_t)(2 + ch) * kN + k), ob, q);
+            }
+            p[w * kPadGroupStep] = oa;
+            p[kPadN + w * kPadGroupStep] = ob;
         }
     }
-#pragma unroll
-    for (int it = 0; it < kPerThreadG; it++) {
-        const int pk = pidx(tid) + it * kPadStep;
-        P[pk] = outv[it][0];        // only this thread reads this slot of rows 0, 1
-        P[kPadN + pk] = outv[it][1];
-    }
-    stage_twiddles(tws, tabs, ch, NTT_INV);   // the forward transforms ended with a barrier
-    cta_ntt_inverse_m<2, Sync>(P, kPadN, tws, ch);
+    cta_ntt_inverse_m<2, Sync>(P, kPadN, tabs, ch);
 #pragma unroll
     for (int it = 0; it < kPerThreadG; it++) {
         const int k = tid + it * kNttThreads;
@@ -526,10 +560,10 @@ __device__ __forceinline__ void ext_tail(uint32_t* P, uint2* tws, const uint32_t
 //   INTT(first_dim) (both primes, to compose) -> decompose_rlwe (2 ell rows)
 //   -> row transforms -> init + sum_row row * rgsw[row] -> INTT
 constexpr int kExtPolys = 4;
-constexpr int kExtSmem = kN * 8 + kExtPolys * kPadN * 4;
+constexpr int kExtSmem = kExtPolys * kPadN * 4;
 
 template <int ELL>
-__global__ void __launch_bounds__(kNttThreads) k_ext_fused(const uint32_t* __restrict__ first_dim,
+__global__ void __launch_bounds__(kNttThreads, 2) k_ext_fused(const uint32_t* __restrict__ first_dim,
                                                            const uint32_t* __restrict__ rgsw,
                                                            const uint32_t* __restrict__ init,
                                                            uint32_t* __restrict__ ext,
@@ -542,28 +576,25 @@ __global__ void __launch_bounds__(kNttThreads) k_ext_fused(const uint32_t* __res
     ext = shifted(ext, ws_off(bt));
     coef_out = shifted(coef_out, ws_off(bt));
     rgsw = shifted(rgsw, key_off(bt));
-    uint2* tws = reinterpret_cast<uint2*>(smem_raw);
-    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw + kN * 8);   // [4][N]
+    uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);   // [4][N]
     const int r = blockIdx.x >> 1, ch = blockIdx.x & 1;
     const uint32_t* fd = first_dim + (size_t)r * 4 * kN;          // [comp][prime][N]
     pdl_launch_dependents();
     // first_dim to coefficient form, all four polynomials (P[comp * 2 + prime])
 #pragma unroll
     for (int pch = 0; pch < 2; pch++) {
-        if (pch) __syncthreads();
-        stage_twiddles(tws, tabs, pch, NTT_INV);
         pdl_wait();   // the first-dimension results come from the previous kernel
 #pragma unroll
         for (int comp = 0; comp < 2; comp++) {
             poly_to_smem(P + (comp * 2 + pch) * kPadN, fd + (comp * 2 + pch) * kN);
         }
-        cta_ntt_inverse_m<2>(P + pch * kPadN, 2 * kPadN, tws, pch);   // a and b of this prime
+        cta_ntt_inverse_m<2>(P + pch * kPadN, 2 * kPadN, tabs, pch);   // a and b of this prime
     }
     if (coef_out && ch == 0) {
 #pragma unroll
         for (int i = 0; i < 4; i++) poly_from_smem(coef_out + ((size_t)r * 4 + i) * kN, P + i * kPadN);
     }
-    ext_tail<ELL, CtaSync>(P, tws, rgsw, init ? init + (size_t)r * 4 * kN : nullptr, ext + (size_t)r * 4 * kN, tabs, g,
+    ext_tail<ELL, CtaSync>(P, rgsw, init ? init + (size_t)r * 4 * kN : nullptr, ext + (size_t)r * 4 * kN, tabs, g,
                            ch);
 }
 

@@ -229,9 +229,9 @@ struct kspir_ctx {
     uint8_t* dbop = nullptr;          // its database operand [N][2][G] tiles
     int G = 0;
     uint8_t* qop = nullptr;           // its query operand: launch at slot0 uses qop_at(slot0)
-    int32_t* perms = nullptr;
+    uint16_t* perms = nullptr;        // [N1][N], lane order
     bool perms_loaded = false;
-    uint32_t* tw = nullptr;           // [3][4][N]
+    uint2* tw = nullptr;              // [CH_COUNT][kTwChannel]
     uint16_t* sigma_baby = nullptr;   // [N1/2][N]
     uint16_t* sigma_giant = nullptr;  // [N2-1][N]
     NttTables ntabs{};
@@ -352,12 +352,11 @@ Workspace ws_host(const kspir_ctx* c, int s) {
     const size_t off = (size_t)s * c->ws_bytes;
     w.q64 += (size_t)s * 4 * kN;
     w.resp64 += (size_t)s * 2 * kN;
+    w.digraw = host_shift(w.digraw, off);
     w.dig0 = host_shift(w.dig0, off);
-    w.qbn = host_shift(w.qbn, off);
-    w.qbbs = host_shift(w.qbbs, off);
+    w.qb = host_shift(w.qb, off);
     w.col0 = host_shift(w.col0, off);
     w.interA = host_shift(w.interA, off);
-    w.interB = host_shift(w.interB, off);
     w.inter_bs = host_shift(w.inter_bs, off);
     w.inter_acoef = host_shift(w.inter_acoef, off);
     w.dig1 = host_shift(w.dig1, off);
@@ -410,6 +409,45 @@ uint64_t chan_root(int ch) {
     }
 }
 
+// a transform twiddle: {w centred in (-q/2, q/2), round(w 2^32 / q)}, both signed
+uint2 lazy_twiddle(uint64_t w, uint32_t q) {
+    const int64_t c = w > q / 2 ? (int64_t)w - q : (int64_t)w;
+    const int64_t a = c < 0 ? -c : c;
+    const int64_t p = (int64_t)((((uint64_t)a << 33) / q + 1) / 2);   // |w| 2^32 / q to nearest, below 2^31
+    return make_uint2((uint32_t)c, (uint32_t)(c < 0 ? -p : p));
+}
+
+// The device table of one channel (layout in ntt.cuh).
+void build_twiddles(uint64_t psi, uint32_t q, uint2* out) {
+    std::vector<uint32_t> pw(2 * kN);   // psi^e
+    pw[0] = 1;
+    for (int e = 1; e < 2 * kN; e++) pw[e] = (uint32_t)((uint64_t)pw[e - 1] * psi % q);
+    const uint64_t ninv = h_invmod(kN, q);
+    // entry e of unit i of a pass with `units` units
+    auto at = [](uint2* t, int units, int i, int e) -> uint2& { return t[((size_t)(e / 2) * units + i) * 2 + (e & 1)]; };
+    uint2* inv = out + kTwFwd;
+    for (int units : {16, 256}) {
+        uint2* f = units == 16 ? out : out + kTwPass1;
+        for (int i = 0; i < units; i++) {
+            at(f, units, i, 0) = make_uint2(0, 0);
+            if (units == 16) at(inv, 16, i, 0) = make_uint2(0, 0);
+            for (int e = 1; e < 16; e++) {
+                const int l = e < 2 ? 0 : e < 4 ? 1 : e < 8 ? 2 : 3, m = 1 << l, k = e - m;   // layer, place in it
+                // forward: psi^brv(n) of table index n = (units + i) 2^l + k
+                at(f, units, i, e) = lazy_twiddle(pw[h_bitrev12((uint32_t)(units * m + i * m + k))], q);
+                // inverse pass 1: half length h = 16 2^l, place p = i + 16 k of it: psi^(-p N / h)
+                if (units == 16) at(inv, 16, i, e) = lazy_twiddle(pw[(2 * kN - (i + 16 * k) * (kN / (16 * m))) % (2 * kN)], q);
+            }
+        }
+    }
+    // inverse pass 2, thread u, input t: psi^(-2 u brv4(t)) psi^-u N^-1
+    for (int u = 0; u < 256; u++)
+        for (int t = 0; t < 16; t++) {
+            const int e = u * (2 * (int)(h_bitrev12((uint32_t)t) >> 8) + 1);   // below 256 * 31 < 2N
+            at(inv + kTwPass1, 256, u, t) = lazy_twiddle((uint64_t)pw[(2 * kN - e) % (2 * kN)] * ninv % q, q);
+        }
+}
+
 // every per-channel constant of c_dev (also written by the allocation-free set-up)
 DevConst make_dev_const() {
     DevConst dc{};
@@ -417,18 +455,23 @@ DevConst make_dev_const() {
         ChanConst& cc = dc.ch[ch];
         const uint32_t q = kChanQ[ch];
         cc.q = q;
-        cc.two_q = 2 * q;
+        cc.nq = 0u - q;
         cc.barrett = ~0ull / q;
-        cc.ninv = (uint32_t)h_invmod(kN, q);
-        cc.ninv_p = shoup32(cc.ninv, q);
-        // the last inverse layer's single twiddle is entry 1 of the inverse
-        // table: psi^-brv(1) = psi^-(N/2); folding N^-1 into it saves one
-        // multiplication per butterfly of that layer
-        const uint64_t iw1 = h_powmod(h_invmod(chan_root(ch), q), h_bitrev12(1), q);
-        cc.ninv_w = (uint32_t)(iw1 * cc.ninv % q);
-        cc.ninv_w_p = shoup32(cc.ninv_w, q);
+        cc.rq = (uint32_t)(((1ull << 33) / q + 1) / 2);
+        const uint64_t psi = chan_root(ch);
+        for (int k = 1; k < 16; k++) cc.fw[k] = lazy_twiddle(h_powmod(psi, h_bitrev12((uint32_t)k), q), q);
+        for (int k = 0; k < 8; k++) cc.iw[k] = lazy_twiddle(h_powmod(psi, 2 * kN - 2 * kN / 16 * k, q), q);
+        for (int t = 0; t < 16; t++) cc.ic[t] = lazy_twiddle(h_powmod(psi, 2 * kN - 256 * t, q), q);
+        uint32_t qi = q;   // q^-1 mod 2^32 by Newton's iteration (q q = 1 mod 8)
+        for (int i = 0; i < 4; i++) qi *= 2 - q * qi;
+        cc.qinv = qi;
+        const uint32_t r32 = (uint32_t)((1ull << 32) % q);
+        cc.kpos = r32;
+        cc.kneg = q - r32;
         cc.bsinv = ch < 2 ? (uint32_t)(kBsModInvCrt % q) : 0;
         cc.bsinv_p = shoup32(cc.bsinv, q);
+        cc.kbaby = ch < 2 ? (uint32_t)((uint64_t)cc.kneg * cc.bsinv % q) : cc.kneg;
+        cc.xs = cc.kbaby > q / 2 ? cc.kbaby - q : cc.kbaby;
     }
     dc.q1inv_mod_q2 = (uint32_t)h_invmod(kQ1 % kQ2, kQ2);
     dc.q1inv_mod_q2_p = shoup32(dc.q1inv_mod_q2, kQ2);
@@ -442,30 +485,20 @@ int init_constants(kspir_ctx* c) {
 
     // twiddles: crt channels use root_of_unity_crt (reference crt.h:81) reduced
     // per prime; bsMod and p use HEXL's minimal primitive root
-    uint64_t roots[CH_COUNT];
-    for (int ch = 0; ch < CH_COUNT; ch++) roots[ch] = chan_root(ch);
-    // per channel uint2 [2][N]: {psi^brv(k), Shoup} then {psi^-brv(k), Shoup}, k-major order
-    std::vector<uint32_t> tw((size_t)CH_COUNT * 4 * kN);
-    for (int ch = 0; ch < CH_COUNT; ch++) {
-        const uint64_t q = kChanQ[ch], psi = roots[ch], pinv = h_invmod(psi, q);
-        uint32_t* t = tw.data() + (size_t)ch * 4 * kN;
-        for (int k = 0; k < kN; k++) {
-            uint32_t e = h_bitrev12(k);
-            const uint32_t w = (uint32_t)h_powmod(psi, e, q), iw = (uint32_t)h_powmod(pinv, e, q);
-            const int pos = tw_layout_pos(k);   // the transforms read the k-major layout
-            t[2 * pos] = w;
-            t[2 * pos + 1] = shoup32(w, (uint32_t)q);
-            t[2 * kN + 2 * pos] = iw;
-            t[2 * kN + 2 * pos + 1] = shoup32(iw, (uint32_t)q);
-        }
-    }
-    KS_CUDA(c, cudaMalloc(&c->tw, tw.size() * 4));
-    KS_COPY(c, c->tw, tw.data(), tw.size() * 4, cudaMemcpyHostToDevice);
-    for (int ch = 0; ch < CH_COUNT; ch++) c->ntabs.tw[ch] = reinterpret_cast<const uint2*>(c->tw + (size_t)ch * 4 * kN);
+    std::vector<uint2> tw((size_t)CH_COUNT * kTwChannel);
+    for (int ch = 0; ch < CH_COUNT; ch++) build_twiddles(chan_root(ch), kChanQ[ch], tw.data() + (size_t)ch * kTwChannel);
+    KS_CUDA(c, cudaMalloc(&c->tw, tw.size() * sizeof(uint2)));
+    KS_COPY(c, c->tw, tw.data(), tw.size() * sizeof(uint2), cudaMemcpyHostToDevice);
+    for (int ch = 0; ch < CH_COUNT; ch++) c->ntabs.tw[ch] = c->tw + (size_t)ch * kTwChannel;
 
     std::vector<uint16_t> sb((size_t)c->N1h * kN), sg((size_t)std::max(1, c->N2 - 1) * kN);
-    for (int i = 0; i < c->N1h; i++) slot_permutation(pow5(i + 1), sb.data() + (size_t)i * kN);
-    for (int cc = 1; cc < c->N2; cc++) slot_permutation(pow5((uint32_t)(c->N1 * cc)), sg.data() + (size_t)(cc - 1) * kN);
+    std::vector<uint16_t> nat(kN);
+    auto lanes = [&](uint32_t g, uint16_t* out) {   // the slot permutation of X -> X^g, lane order
+        slot_permutation(g, nat.data());
+        for (int k = 0; k < kN; k++) out[lane_pos(k)] = nat[k];
+    };
+    for (int i = 0; i < c->N1h; i++) lanes(pow5(i + 1), sb.data() + (size_t)i * kN);
+    for (int cc = 1; cc < c->N2; cc++) lanes(pow5((uint32_t)(c->N1 * cc)), sg.data() + (size_t)(cc - 1) * kN);
     KS_CUDA(c, cudaMalloc(&c->sigma_baby, sb.size() * 2));
     KS_COPY(c, c->sigma_baby, sb.data(), sb.size() * 2, cudaMemcpyHostToDevice);
     KS_CUDA(c, cudaMalloc(&c->sigma_giant, sg.size() * 2));
@@ -487,15 +520,14 @@ int init_workspaces(kspir_ctx* c) {
     struct Part { void** dst; size_t bytes; };
     Workspace& w = c->ws0;
     std::vector<Part> parts = {
-        {(void**)&w.dig0, 9 * P},
-        {(void**)&w.qbn, 2 * P},
-        {(void**)&w.qbbs, P},
+        {(void**)&w.digraw, 3 * P},
+        {(void**)&w.dig0, 12 * P},
+        {(void**)&w.qb, 3 * P},
         {(void**)&w.col0, 4 * P},
         {(void**)&w.interA, 2 * P},
-        {(void**)&w.interB, 2 * P},
-        {(void**)&w.inter_bs, 2 * P},
+        {(void**)&w.inter_bs, P},
         {(void**)&w.inter_acoef, 2 * P},
-        {(void**)&w.dig1, 9 * P},
+        {(void**)&w.dig1, 12 * P},
         {(void**)&w.cipherbuf, (size_t)kN * N1 * 2 * 8},
         {(void**)&w.sout, (size_t)r * N2 * 4 * P},
         {(void**)&w.result, (size_t)r * 4 * P},
@@ -531,14 +563,14 @@ int init_workspaces(kspir_ctx* c) {
     auto add = [&](const uint32_t* src, uint32_t* dst, int ch, int stride) {
         NttJob j; j.src = src; j.dst = dst; j.ch = ch; j.dst_stride = stride; jobs.push_back(j);
     };
-    // query: dig0 (9), query b crt (2), modswitched query -> cipherbuf column 0 (4);
+    // query: dig0 (9 digits, 3 b), modswitched query -> cipherbuf column 0 (4);
     // a second copy writes column 0 of the rotation-major cipherbuf
     uint32_t* cb32 = reinterpret_cast<uint32_t*>(w.cipherbuf);
     for (int rm = 0; rm < 2; rm++) {
         (rm ? c->seg_q_rm : c->seg_q) = (int)jobs.size();
         for (int j = 0; j < 3; j++)
-            for (int ch = 0; ch < 3; ch++) add(w.dig0 + (j * 3 + ch) * kN, w.dig0 + (j * 3 + ch) * kN, ch, 1);
-        for (int ch = 0; ch < 2; ch++) add(w.qbn + ch * kN, w.qbn + ch * kN, ch, 1);
+            for (int ch = 0; ch < 3; ch++) add(w.digraw + j * kN, w.dig0 + (size_t)ch * 4 * kN + j, ch, 4);
+        for (int ch = 0; ch < 3; ch++) add(w.qb + ch * kN, w.dig0 + (size_t)ch * 4 * kN + 3, ch, 4);
         for (int comp = 0; comp < 2; comp++)
             for (int ch = 0; ch < 2; ch++) {
                 if (rm) add(w.col0 + (comp * 2 + ch) * kN, cb32 + cipherbuf_rm_idx(0, comp, ch, 0), ch, 1);
@@ -550,7 +582,7 @@ int init_workspaces(kspir_ctx* c) {
     for (int ch = 0; ch < 2; ch++) add(w.interA + ch * kN, w.inter_acoef + ch * kN, ch, 1);
     c->seg_dig1 = (int)jobs.size();
     for (int j = 0; j < 3; j++)
-        for (int ch = 0; ch < 3; ch++) add(w.dig1 + (j * 3 + ch) * kN, w.dig1 + (j * 3 + ch) * kN, ch, 1);
+        for (int ch = 0; ch < 3; ch++) add(w.digraw + j * kN, w.dig1 + (size_t)ch * 4 * kN + j, ch, 4);
     KS_CUDA(c, cudaMalloc(&c->jobs, jobs.size() * sizeof(NttJob)));
     KS_COPY(c, c->jobs, jobs.data(), jobs.size() * sizeof(NttJob), cudaMemcpyHostToDevice);
     return KSPIR_OK;
@@ -580,7 +612,19 @@ int init_key_slots(kspir_ctx* c) {
 
 inline int blocks_for(long n, int t) { return (int)((n + t - 1) / t); }
 
+constexpr int kBabySplitMaxBatch = 1;   // batches up to this size run one CTA per rotation and component
 constexpr int kPackSplitMaxBatch = 4;   // batches up to this size pack with the split (latency) kernels
+
+// converts one client's key words (device memory) into its key slot
+void launch_keys(const kspir_ctx* c, const uint64_t* baby, const uint64_t* giant, const uint64_t* packing,
+                 const uint64_t* rgsw, const ClientKeysDev& d, cudaStream_t st) {
+    const long ng = (long)(c->N2 - 1) * 2 * 2, np = (long)c->levels * 4 * 2;
+    const long polys = (long)c->N1h * 12 + ng + np + 8;
+    k_keys_from_words<<<blocks_for(polys * (kN / 4), 256), 256, 0, st>>>(
+        baby, giant, packing, rgsw, const_cast<uint32_t*>(d.baby_crt), const_cast<uint32_t*>(d.baby_bs),
+        const_cast<uint32_t*>(d.giant), const_cast<uint32_t*>(d.packing), const_cast<uint32_t*>(d.rgsw), c->N1h, (int)ng,
+        (int)np);
+}
 
 // ---------------------------------------------------------------------------
 // launch sequence of `nq` queries in workspace slots slot0 .. slot0 + nq - 1
@@ -623,30 +667,30 @@ void enqueue_baby(kspir_ctx* c, int slot0, int nq, bool rm, cudaStream_t st) {
     const Batch bt = batch_of(c, slot0);
     launch(c, false, k_query_prep, dim3(kN / 256, nq), 256, 0, st, w, c->gad.baby, bt, c->p.r * 4 * kN,
            giant_two_acc(c) ? 1 : 0);
-    launch(c, false, k_ntt_jobs<false>, dim3(c->n_q, nq), kNttThreads, kNttJobSmem, st,
+    launch(c, false, k_ntt_jobs<false>, dim3(c->n_q, nq), kNttGroup, kNttJobSmem, st,
            (const NttJob*)(c->jobs + (rm ? c->seg_q_rm : c->seg_q)), c->ntabs, bt);
     BabyArgs a1{};
     a1.cb_rm = rm ? 1 : 0;
-    a1.dig = w.dig0; a1.srcB = w.qbn; a1.srcBbs = w.qbbs; a1.perms = c->perms; a1.sigma = c->sigma_baby;
-    a1.cipherbuf = w.cipherbuf; a1.interA = w.interA; a1.interB = w.interB; a1.inter_bs = w.inter_bs;
+    a1.dig = w.dig0; a1.perms = c->perms; a1.sigma = c->sigma_baby;
+    a1.cipherbuf = w.cipherbuf; a1.interA = w.interA; a1.inter_dig = w.dig1; a1.inter_bs = w.inter_bs;
     a1.N1 = c->N1; a1.col_base = 1; a1.inter_idx = c->N1h - 2;
-    // one CTA per (rotation, component), also for a single query: with the
-    // minimum-form reductions its six transforms per rotation beat the
-    // four-CTA shape (eight transforms) on one answer (0.399 against
-    // 0.403 ms) and on overlapped answers (0.229 against 0.235 ms)
     auto rot = [&](const BabyArgs& args, int nrot) {
         if (nrot <= 0) return;
-        launch(c, false, k_baby_pair<3, 2>, dim3(nrot * 2, nq), kNttThreads, kBabyPairSmem, st, args, c->keys0, c->ntabs,
-               bt);
+        if (nq <= kBabySplitMaxBatch)
+            launch(c, false, k_baby_rot<1>, dim3(nrot * 2, nq), kNttThreads, kBabyPolys1 * kPadN * 4, st, args, c->keys0,
+                   c->ntabs, bt);
+        else
+            launch(c, false, k_baby_rot<2>, dim3(nrot, nq), kNttThreads, kBabyPolys2 * kPadN * 4, st, args, c->keys0,
+                   c->ntabs, bt);
     };
     rot(a1, c->N1h - 1);
-    launch(c, false, k_ntt_jobs<true>, dim3(2, nq), kNttThreads, kNttJobSmem, st, (const NttJob*)(c->jobs + c->seg_inter),
+    launch(c, false, k_ntt_jobs<true>, dim3(2, nq), kNttGroup, kNttJobSmem, st, (const NttJob*)(c->jobs + c->seg_inter),
            c->ntabs, bt);
     launch(c, false, k_inter_decomp, dim3(kN / 256, nq), 256, 0, st, w, c->gad.baby, bt);
-    launch(c, false, k_ntt_jobs<false>, dim3(9, nq), kNttThreads, kNttJobSmem, st, (const NttJob*)(c->jobs + c->seg_dig1),
+    launch(c, false, k_ntt_jobs<false>, dim3(9, nq), kNttGroup, kNttJobSmem, st, (const NttJob*)(c->jobs + c->seg_dig1),
            c->ntabs, bt);
     BabyArgs a2 = a1;
-    a2.dig = w.dig1; a2.srcB = w.interB; a2.srcBbs = w.inter_bs + kN;
+    a2.dig = w.dig1;
     a2.col_base = c->N1h; a2.inter_idx = -1;
     rot(a2, c->N1h);
 }
@@ -823,11 +867,11 @@ FaArgs fa_args(const kspir_ctx* c, int ring_slot) {
     A.gad = c->gad;
     BabyArgs a1{};
     a1.cb_rm = 0;
-    a1.dig = w.dig0; a1.srcB = w.qbn; a1.srcBbs = w.qbbs; a1.perms = c->perms; a1.sigma = c->sigma_baby;
-    a1.cipherbuf = w.cipherbuf; a1.interA = w.interA; a1.interB = w.interB; a1.inter_bs = w.inter_bs;
+    a1.dig = w.dig0; a1.perms = c->perms; a1.sigma = c->sigma_baby;
+    a1.cipherbuf = w.cipherbuf; a1.interA = w.interA; a1.inter_dig = w.dig1; a1.inter_bs = w.inter_bs;
     a1.N1 = c->N1; a1.col_base = 1; a1.inter_idx = c->N1h - 2;
     BabyArgs a2 = a1;
-    a2.dig = w.dig1; a2.srcB = w.interB; a2.srcBbs = w.inter_bs + kN;
+    a2.dig = w.dig1;
     a2.col_base = c->N1h; a2.inter_idx = -1;
     A.a1 = a1;
     A.a2 = a2;
@@ -1218,7 +1262,8 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     KS_CUDA(c.get(), cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device));
     c->scan_ctas = c->nsm;
     if (const char* e = getenv("KSPIR_SCAN_CTAS")) c->scan_ctas = std::max(1, std::min(c->nsm, atoi(e)));
-    KS_CUDA(c.get(), cudaFuncSetAttribute(k_baby_pair<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBabyPairSmem));
+    KS_CUDA(c.get(), cudaFuncSetAttribute(k_baby_rot<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBabyPolys1 * kPadN * 4));
+    KS_CUDA(c.get(), cudaFuncSetAttribute(k_baby_rot<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBabyPolys2 * kPadN * 4));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_client_query, cudaFuncAttributeMaxDynamicSharedMemorySize, kClientSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_client_decrypt, cudaFuncAttributeMaxDynamicSharedMemorySize, kClientSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_db_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDbRowsSmem));
@@ -1251,7 +1296,7 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     }
     rc = init_constants(c.get());
     if (rc) return rc;
-    KS_CUDA(c.get(), cudaMalloc(&c->perms, (size_t)p.N1 * kN * 4));
+    KS_CUDA(c.get(), cudaMalloc(&c->perms, (size_t)p.N1 * kN * 2));
     c->ring.resize(kTimingRing);
     c->ring_nq.assign(kTimingRing, 0);
     for (auto& evs : c->ring)
@@ -2048,7 +2093,9 @@ int kspir_perms_upload(kspir_ctx* c, const int32_t* perms, size_t count) {
     std::lock_guard<std::mutex> lk(c->mu);
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
-    KS_COPY(c, c->perms, perms, count * 4, cudaMemcpyHostToDevice);
+    std::vector<uint16_t> lanes(count);
+    for (size_t i = 0; i < count; i++) lanes[i / kN * kN + lane_pos((int)(i % kN))] = (uint16_t)perms[i];
+    KS_COPY(c, c->perms, lanes.data(), count * 2, cudaMemcpyHostToDevice);
     c->perms_loaded = true;
     return KSPIR_OK;
 }
@@ -2061,46 +2108,27 @@ int kspir_client_keys_upload(kspir_ctx* c, int client, const uint64_t* baby, con
     std::lock_guard<std::mutex> lk(c->mu);
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
-    const size_t nb_poly = (size_t)c->N1h * 3 * 2;                 // crt rows and bs rows each
-    const size_t ng_poly = (size_t)(c->N2 - 1) * 2 * 2;
-    const size_t np_poly = (size_t)c->levels * 4 * 2;
-    const size_t nr_poly = 4 * 2;
-    // split baby rows 0-2 (crtMod) and 3-5 (bsMod)
-    std::vector<uint64_t> crt_rows(nb_poly * kN), bs_rows(nb_poly * kN);
-    for (int i = 0; i < c->N1h; i++)
-        for (int j = 0; j < 6; j++)
-            for (int comp = 0; comp < 2; comp++) {
-                const uint64_t* src = baby + (((size_t)i * 6 + j) * 2 + comp) * kN;
-                uint64_t* dst = (j < 3 ? crt_rows.data() : bs_rows.data()) +
-                                (((size_t)i * 3 + (j % 3)) * 2 + comp) * kN;
-                memcpy(dst, src, kN * 8);
-            }
-    if (!canonical(crt_rows.data(), crt_rows.size(), kCrtMod) || !canonical(bs_rows.data(), bs_rows.size(), kBsMod) ||
-        (giant && !canonical(giant, ng_poly * kN, kCrtMod)) || (packing && !canonical(packing, np_poly * kN, kCrtMod)) ||
-        !canonical(rgsw, nr_poly * kN, kCrtMod))
+    const size_t nb = (size_t)c->N1h * 6 * 2 * kN, ng = (size_t)(c->N2 - 1) * 2 * 2 * kN;
+    const size_t np = (size_t)c->levels * 4 * 2 * kN, nr = (size_t)4 * 2 * kN;
+    for (size_t p = 0; p < nb / kN; p++)   // rows 0-2 of each baby key mod crtMod, 3-5 mod bsMod
+        if (!canonical(baby + p * kN, kN, ((p / 2) % 6) < 3 ? kCrtMod : (uint64_t)kBsMod))
+            return set_err(c, KSPIR_ERR_INVALID_ARG, "key word not canonical");
+    if ((giant && !canonical(giant, ng, kCrtMod)) || (packing && !canonical(packing, np, kCrtMod)) ||
+        !canonical(rgsw, nr, kCrtMod))
         return set_err(c, KSPIR_ERR_INVALID_ARG, "key word not canonical");
 
-    const ClientKeysDev keys = keys_host(c, client);
-    const size_t stage_words = std::max({nb_poly, ng_poly, np_poly, nr_poly}) * kN;
     uint64_t* stage = nullptr;
-    KS_CUDA(c, cudaMalloc(&stage, stage_words * 8));
-    auto split = [&](const uint64_t* h, size_t polys, const uint32_t* dst) -> int {
-        if (!polys) return KSPIR_OK;
-        KS_COPY(c, stage, h, polys * kN * 8, cudaMemcpyHostToDevice);
-        k_split_words<<<blocks_for((long)polys * kN, 256), 256, 0, c->stream>>>(stage, const_cast<uint32_t*>(dst),
-                                                                              (int)polys);
-        KS_CUDA(c, cudaStreamSynchronize(c->stream));
-        return KSPIR_OK;
-    };
+    KS_CUDA(c, cudaMalloc(&stage, (nb + ng + np + nr) * 8));
+    uint64_t *g = stage + nb, *pk = g + ng, *rg = pk + np;
     c->key_loaded[client] = 0;
-    int rc = split(crt_rows.data(), nb_poly, keys.baby_crt);
-    if (!rc) rc = split(giant, ng_poly, keys.giant);
-    if (!rc) rc = split(packing, np_poly, keys.packing);
-    if (!rc) rc = split(rgsw, nr_poly, keys.rgsw);
+    int rc = copy_sync(c, stage, baby, nb * 8, cudaMemcpyHostToDevice);
+    if (!rc && ng) rc = copy_sync(c, g, giant, ng * 8, cudaMemcpyHostToDevice);
+    if (!rc && np) rc = copy_sync(c, pk, packing, np * 8, cudaMemcpyHostToDevice);
+    if (!rc) rc = copy_sync(c, rg, rgsw, nr * 8, cudaMemcpyHostToDevice);
     if (!rc) {
-        std::vector<uint32_t> bs32(bs_rows.size());
-        for (size_t i = 0; i < bs_rows.size(); i++) bs32[i] = (uint32_t)bs_rows[i];
-        rc = copy_sync(c, const_cast<uint32_t*>(keys.baby_bs), bs32.data(), bs32.size() * 4, cudaMemcpyHostToDevice);
+        launch_keys(c, stage, g, pk, rg, keys_host(c, client), c->stream);
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
+            rc = set_err(c, KSPIR_ERR_CUDA, "key conversion");
     }
     cudaFree(stage);
     if (rc) return rc;
@@ -2571,43 +2599,15 @@ constexpr size_t kNaScratchWords = (size_t)kNoAllocMaxCount * kNaPerCt   // per-
 // Scratch shared by every call on a device; it keeps the previous call's
 // contents.  Twiddle tables of the no-allocation path live beside it.
 static __device__ __align__(256) uint32_t g_na_scratch[kNaScratchWords];
-static __device__ __align__(256) uint32_t g_na_tw[3 * 4 * kN];
+static __device__ __align__(256) uint2 g_na_tw[3 * kTwChannel];
 
 struct NaDevice {
     bool ready = false;
     uint32_t* scratch = nullptr;   // device address of g_na_scratch on this device
-    uint32_t* tw = nullptr;        // device address of g_na_tw on this device
+    uint2* tw = nullptr;           // device address of g_na_tw on this device
 };
 NaDevice g_na[64];
 std::mutex g_na_mutex;
-
-// twiddles psi^brv(k), psi^-brv(k) and Shoup companions, computed on the device
-__global__ void k_na_twiddles(uint32_t* tw, uint32_t q0, uint32_t q1, uint32_t q2, uint32_t p0, uint32_t p1,
-                              uint32_t p2) {
-    const int ch = blockIdx.y;
-    const uint32_t q = ch == 0 ? q0 : ch == 1 ? q1 : q2;
-    const uint32_t psi = ch == 0 ? p0 : ch == 1 ? p1 : p2;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kN; k += gridDim.x * blockDim.x) {
-        uint32_t e = __brev((uint32_t)k) >> (32 - kLogN);
-        auto pw = [&](uint32_t x) {
-            uint64_t r = 1, b = psi;
-            while (x) {
-                if (x & 1) r = r * b % q;
-                b = b * b % q;
-                x >>= 1;
-            }
-            return (uint32_t)r;
-        };
-        uint32_t w = pw(e);
-        uint32_t iw = pw((2 * kN - e) % (2 * kN));   // psi^(2N) = 1
-        uint32_t* t = tw + (size_t)ch * 4 * kN;   // uint2 [2][N], k-major layout
-        const int pos = tw_layout_pos(k);
-        t[2 * pos] = w;
-        t[2 * pos + 1] = (uint32_t)(((uint64_t)w << 32) / q);
-        t[2 * kN + 2 * pos] = iw;
-        t[2 * kN + 2 * pos + 1] = (uint32_t)(((uint64_t)iw << 32) / q);
-    }
-}
 
 // job list for count <= kNoAllocMaxCount: inverse transforms of the first
 // kNoAllocMaxCount*4 polynomials, then forward transforms of the digits
@@ -2660,9 +2660,10 @@ int na_setup(int device, cudaStream_t st) {
     const DevConst dc = make_dev_const();   // the same constants a context writes
     if (cudaMemcpyToSymbolAsync(c_dev, &dc, sizeof(dc), 0, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return KSPIR_ERR_CUDA;
-    const uint64_t root_crt = 3375402822066082ull;
-    k_na_twiddles<<<dim3(16, 3), 256, 0, st>>>(d.tw, kQ1, kQ2, kBsMod, (uint32_t)(root_crt % kQ1),
-                                              (uint32_t)(root_crt % kQ2), (uint32_t)h_min_root(kBsMod));
+    std::vector<uint2> tw(3 * (size_t)kTwChannel);
+    for (int ch = 0; ch < 3; ch++) build_twiddles(chan_root(ch), kChanQ[ch], tw.data() + (size_t)ch * kTwChannel);
+    if (cudaMemcpyAsync(d.tw, tw.data(), tw.size() * sizeof(uint2), cudaMemcpyHostToDevice, st) != cudaSuccess)
+        return KSPIR_ERR_CUDA;
     NaLayout L = na_layout(d.scratch);
     k_na_jobs<<<1, kNoAllocMaxCount * 12, 0, st>>>(L.jobs, L.fd_res, L.ecoef, L.edig);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return KSPIR_ERR_CUDA;
@@ -2689,7 +2690,7 @@ extern "C" int kspir_external_product_noalloc(int device, const uint64_t* d_rgsw
         const NaDevice& d = g_na[device];
         NaLayout L = na_layout(d.scratch);
         NttTables tabs;
-        for (int ch = 0; ch < 3; ch++) tabs.tw[ch] = reinterpret_cast<const uint2*>(d.tw + (size_t)ch * 4 * kN);
+        for (int ch = 0; ch < 3; ch++) tabs.tw[ch] = d.tw + (size_t)ch * kTwChannel;
         GadgetS g;
         g.ell = 2; g.base_bits = 20; g.gbits = 18;   // RGSW of test-pir.cpp:71
         const size_t n = (size_t)count * 2 * kN;
@@ -2700,9 +2701,9 @@ extern "C" int kspir_external_product_noalloc(int device, const uint64_t* d_rgsw
         k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(d_first_dim, L.fd_res, count * 2);
         k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(d_result, L.acc_res, count * 2);
         k_split_words<<<blocks_for(8L * kN, 256), 256, 0, st>>>(d_rgsw, L.rgsw, 8);
-        k_ntt_jobs<true><<<count * 4, kNttThreads, kNttJobSmem, st>>>(L.jobs, tabs, Batch{});
+        k_ntt_jobs<true><<<count * 4, kNttGroup, kNttJobSmem, st>>>(L.jobs, tabs, Batch{});
         k_ext_decomp<<<blocks_for((long)count * kN, 256), 256, 0, st>>>(L.ecoef, L.edig, count, g);
-        k_ntt_jobs<false><<<count * 8, kNttThreads, kNttJobSmem, st>>>(L.jobs + kNoAllocMaxCount * 4, tabs, Batch{});
+        k_ntt_jobs<false><<<count * 8, kNttGroup, kNttJobSmem, st>>>(L.jobs + kNoAllocMaxCount * 4, tabs, Batch{});
         k_ext_mac_intt<<<count * 4, kNttThreads, kMacSmem, st>>>(L.edig, L.rgsw, L.acc_res, L.ext, 4, tabs);
         int flag = 0;
         if (cudaGetLastError() != cudaSuccess ||

@@ -12,7 +12,9 @@
 
 namespace kspir {
 
-// Client key material, converted to residues at upload.
+// Client key material, converted at upload (k_keys_from_words): per channel the
+// centred residue of the word times -2^32 (rgsw: 2^32; baby_crt: -bsMod^-1 2^32),
+// each polynomial in lane order (ntt.cuh).
 //   baby_crt [N1/2][3][2 comp][2 ch][N]    (reference keyMap[5^i][0..2], lwe.h:381-466)
 //   baby_bs  [N1/2][3][2 comp][N]          (keyMap[5^i][3..5], mod bsMod)
 //   giant    [N2-1][2][2 comp][2 ch][N]    (keyMap[5^(N1 c)])
@@ -40,15 +42,14 @@ __host__ __device__ __forceinline__ size_t sout_idx(int row, int cv, int z, int 
 
 struct Workspace {
     uint64_t* q64;          // [4][N] query words: crt a, crt b, bs a, bs b (coefficient form)
-    uint32_t* dig0;         // [3][3 ch][N] decompose_bsgs(query a) digits -> NTT form
-    uint32_t* qbn;          // [2 ch][N] query b mod q1/q2 -> NTT form
-    uint32_t* qbbs;         // [N] query b mod bsMod, coefficient form
+    uint32_t* digraw;       // [3][N] decompose_bsgs digits, signed (the query's, then the intermediate's)
+    uint32_t* dig0;         // [3 ch][N][4] NTT form of the query's digits and b (crt: b * bsMod^-1)
+    uint32_t* qb;           // [3 ch][N] query b (crt: * bsMod^-1), coefficient form
     uint32_t* col0;         // [2 comp][2 ch][N] modswitched query, coefficient form (scratch)
     uint32_t* interA;       // [2 ch][N] rotation N1/2-1, a, before modswitch, NTT form
-    uint32_t* interB;       // [2 ch][N] rotation N1/2-1, b, NTT form of the coefficient-form sum
-    uint32_t* inter_bs;     // [2 comp][N] rotation N1/2-1 mod bsMod, coefficient form
+    uint32_t* inter_bs;     // [N] rotation N1/2-1, a mod bsMod, coefficient form
     uint32_t* inter_acoef;  // [2 ch][N] interA, coefficient form
-    uint32_t* dig1;         // [3][3 ch][N] digits of the intermediate -> NTT form
+    uint32_t* dig1;         // [3 ch][N][4] the same of the intermediate
     uint64_t* cipherbuf;    // [N][N1][2] reference reorientCipher layout (twosteps.cpp:1386)
     uint32_t* sout;         // DB-scan outputs, NTT form, layout of sout_idx (r * N2 rows)
     uint32_t* result;       // [r][2 comp][2 ch][N] first-dimension results, NTT form (the
@@ -88,12 +89,11 @@ __device__ __forceinline__ Workspace ws_at(Workspace w, const Batch& b) {
     const size_t off = (size_t)s * b.ws_bytes;
     w.q64 += (size_t)s * 4 * kN;
     w.resp64 += (size_t)s * 2 * kN;
+    w.digraw = shifted(w.digraw, off);
     w.dig0 = shifted(w.dig0, off);
-    w.qbn = shifted(w.qbn, off);
-    w.qbbs = shifted(w.qbbs, off);
+    w.qb = shifted(w.qb, off);
     w.col0 = shifted(w.col0, off);
     w.interA = shifted(w.interA, off);
-    w.interB = shifted(w.interB, off);
     w.inter_bs = shifted(w.inter_bs, off);
     w.inter_acoef = shifted(w.inter_acoef, off);
     w.dig1 = shifted(w.dig1, off);

@@ -126,12 +126,7 @@ int srv_upload(Srv& s, Srv::Lane& L, Srv::Client& cl) {
     if (s.kw_pack && cudaMemcpyAsync(pk, cl.packing, s.kw_pack * 8, cudaMemcpyHostToDevice, L.st) != cudaSuccess)
         return KSPIR_ERR_CUDA;
     if (cudaMemcpyAsync(rg, cl.rgsw, s.kw_rgsw * 8, cudaMemcpyHostToDevice, L.st) != cudaSuccess) return KSPIR_ERR_CUDA;
-    const ClientKeysDev d = keys_host(c, cl.slot);
-    const long polys = (long)(s.kw_baby + s.kw_giant + s.kw_pack + s.kw_rgsw) / kN;
-    k_keys_from_words<<<blocks_for(polys * kN, 256), 256, 0, L.st>>>(
-        b, g, pk, rg, const_cast<uint32_t*>(d.baby_crt), const_cast<uint32_t*>(d.baby_bs),
-        const_cast<uint32_t*>(d.giant), const_cast<uint32_t*>(d.packing), const_cast<uint32_t*>(d.rgsw), c->N1h,
-        (int)(s.kw_giant / kN), (int)(s.kw_pack / kN));
+    launch_keys(c, b, g, pk, rg, keys_host(c, cl.slot), L.st);
     if (cudaGetLastError() != cudaSuccess) return KSPIR_ERR_CUDA;
     if (cudaEventRecord(s.slot_ready[cl.slot], L.st) != cudaSuccess) return KSPIR_ERR_CUDA;
     cl.fresh = false;
