@@ -101,13 +101,6 @@ void slot_permutation(uint32_t g, uint16_t* sigma) {
 
 uint32_t pow5(uint32_t e) { return (uint32_t)h_powmod(5, e, 2 * kN); }
 
-// Gather table of the database preprocessing: row R = k N1 + i of the
-// rearranged database takes entry G_i[j] of its diagonal row, where
-// G_i = query_encode^-1 o perm[i] (reference twosteps.cpp:104-118).
-// query_encode[t] = brv((rot_t - 1) / 2) with rot_t = 5^t mod 2N for t < N/2
-// and rot_{N-1-t} = -5^t mod 2N (utils.cpp:1473-1512, :1657-1675); perm[i] is
-// the slot permutation of X -> X^(5^i) (compute_permutation_matrix,
-// utils.cpp:1585-1619).
 // query_encode[t] (utils.cpp:1657-1675): brv((rot_t - 1) / 2), rot_t = 5^t mod 2N
 // for t < N/2 and rot_{N-1-t} = -5^t mod 2N
 std::vector<int32_t> query_encode_table() {
@@ -120,19 +113,6 @@ std::vector<int32_t> query_encode_table() {
     return qe;
 }
 
-std::vector<uint16_t> db_gather_table(int N1) {
-    std::vector<uint16_t> inv_qe(kN), perm(kN), g((size_t)N1 * kN);
-    for (uint32_t t = 0; t < (uint32_t)kN / 2; t++) {
-        const uint32_t rot = pow5(t);
-        inv_qe[h_bitrev12((rot - 1) / 2)] = (uint16_t)t;
-        inv_qe[h_bitrev12((2 * kN - rot - 1) / 2)] = (uint16_t)(kN - 1 - t);
-    }
-    for (int i = 0; i < N1; i++) {
-        slot_permutation(pow5((uint32_t)i), perm.data());
-        for (int j = 0; j < kN; j++) g[(size_t)i * kN + j] = inv_qe[perm[j]];
-    }
-    return g;
-}
 uint32_t inv_mod_2n(uint32_t g) { return (uint32_t)h_powmod(g, 2047, 2 * kN); }   // group order | 2048
 
 int ilog2i(int v) { int l = 0; while ((1 << l) < v) l++; return l; }
@@ -212,7 +192,7 @@ struct kspir_ctx {
     uint64_t* db = nullptr;
     bool db_loaded = false;
     bool mma = false;                 // batched tensor-core scan enabled (N1 = 128, several slots)
-    uint16_t* dbg = nullptr;          // gather table of the database preprocessing [N1][N]
+    uint16_t* db_qenc = nullptr;      // query_encode, of the database preprocessing [N]
     int* dbflag = nullptr;            // its validation word
     // one-sub-database preprocessing calls (kspir_database_*): device raw,
     // rows and datacrt; pinned host staging and the last rows returned
@@ -1094,8 +1074,7 @@ int build_dbop(kspir_ctx* c) {
     if (!c->mma) return KSPIR_OK;
     const size_t bytes = (size_t)kN * 2 * c->G * kATile;
     if (!c->dbop) KS_CUDA(c, cudaMalloc(&c->dbop, bytes));
-    k_dbop_build<<<blocks_for((long)kN * 2 * c->G * 128 * 8, 256), 256, 0, c->stream>>>(c->db, c->dbop, c->p.r, c->N2,
-                                                                                        c->G);
+    k_dbop_build<<<blocks_for((long)kN * c->G * 32 * 8, 256), 256, 0, c->stream>>>(c->db, c->dbop, c->p.r, c->N2, c->G);
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, cudaStreamSynchronize(c->stream));
     return KSPIR_OK;
@@ -1208,6 +1187,13 @@ int init_fused(kspir_ctx* c) {
     return KSPIR_OK;
 }
 
+template <bool ROWS>
+void launch_db_rows(kspir_ctx* c, const uint64_t* raw, uint64_t* out, uint64_t* rows, int subs) {
+    auto kern = (uintptr_t)raw % 16 == 0 ? k_db_rows<ROWS, true> : k_db_rows<ROWS, false>;
+    kern<<<dim3(kN / 2 / kDbRowsPerCta, subs), kDbRowsThreads, kDbRowsSmem, c->stream>>>(raw, c->db_qenc, out, rows, c->N1,
+                                                                                         c->ntabs);
+}
+
 template <int BT>
 int mma_attr(kspir_ctx* c) {
     KS_CUDA(c, cudaFuncSetAttribute(k_scan_mma<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, MmaCfg<BT>::SMEM));
@@ -1266,8 +1252,8 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_baby_rot<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBabyPolys2 * kPadN * 4));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_client_query, cudaFuncAttributeMaxDynamicSharedMemorySize, kClientSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_client_decrypt, cudaFuncAttributeMaxDynamicSharedMemorySize, kClientSmem));
-    KS_CUDA(c.get(), cudaFuncSetAttribute(k_db_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDbRowsSmem));
-    KS_CUDA(c.get(), cudaFuncSetAttribute(k_db_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDbRowsSmem));
+    for (auto kern : {k_db_rows<false, false>, k_db_rows<false, true>, k_db_rows<true, false>, k_db_rows<true, true>})
+        KS_CUDA(c.get(), cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDbRowsSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_ntt_jobs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNttJobSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_ntt_jobs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNttJobSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_giant_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGiantSmem));
@@ -1349,7 +1335,7 @@ int kspir_ctx_destroy(kspir_ctx* c) {
     cudaFree(c->stage32);
     cudaFree(c->key_mem);
     cudaFree(c->db);
-    cudaFree(c->dbg);
+    cudaFree(c->db_qenc);
     cudaFree(c->dbflag);
     cudaFree(c->prep_dev);
     cudaFree(c->cl_qenc);
@@ -1389,21 +1375,28 @@ int kspir_db_upload(kspir_ctx* c, const uint64_t* datacrt, size_t words) {
 namespace {
 // Validates the raw database on the device, then overwrites the resident one
 // with its preprocessed form (k_db_rows), caller holds the lock.
-// the gather table of the context's N1 and the validation word, built once
+// the table of the preprocessing and the validation word, built once
 int ensure_db_tables(kspir_ctx* c) {
-    if (c->dbg) return KSPIR_OK;
-    const std::vector<uint16_t> g = db_gather_table(c->N1);
-    KS_CUDA(c, cudaMalloc(&c->dbflag, sizeof(int)));
-    KS_CUDA(c, cudaMalloc(&c->dbg, g.size() * 2));
-    KS_COPY(c, c->dbg, g.data(), g.size() * 2, cudaMemcpyHostToDevice);
+    if (c->db_qenc) return KSPIR_OK;
+    const std::vector<int32_t> q = query_encode_table();
+    const std::vector<uint16_t> g(q.begin(), q.end());
+    if (!c->dbflag) KS_CUDA(c, cudaMalloc(&c->dbflag, sizeof(int)));
+    uint16_t* d = nullptr;
+    KS_CUDA(c, cudaMalloc(&d, g.size() * 2));
+    if (int rc = copy_sync(c, d, g.data(), g.size() * 2, cudaMemcpyHostToDevice)) {
+        cudaFree(d);
+        return rc;
+    }
+    c->db_qenc = d;
     return KSPIR_OK;
 }
+
 
 // 1 when some of the n raw words is >= bsgsp (synchronises)
 int db_words_invalid(kspir_ctx* c, const uint64_t* d_raw, size_t n, int* bad) {
     cudaStream_t st = c->stream;
     KS_CUDA(c, cudaMemsetAsync(c->dbflag, 0, sizeof(int), st));
-    k_check_canonical<<<c->nsm * 8, 256, 0, st>>>(d_raw, n, kP, c->dbflag);
+    k_check_raw<<<c->nsm * 8, 256, 0, st>>>(d_raw, n, c->dbflag);
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, cudaMemcpyAsync(bad, c->dbflag, sizeof(int), cudaMemcpyDeviceToHost, st));
     KS_CUDA(c, cudaStreamSynchronize(st));
@@ -1431,8 +1424,7 @@ int db_preprocess_dev(kspir_ctx* c, const uint64_t* d_raw, float* device_ms) {
         return set_err(c, KSPIR_ERR_INVALID_ARG, "database entries must be below bsgsp = 65537");
     }
     c->db_loaded = false;
-    k_db_rows<false><<<dim3(kN / 2 / kDbRowsPerCta, r), kNttThreads, kDbRowsSmem, st>>>(d_raw, c->dbg, c->db,
-                                                                                          nullptr, c->N1, c->ntabs);
+    launch_db_rows<false>(c, d_raw, c->db, nullptr, r);
     KS_CUDA(c, cudaGetLastError());
     int rc = build_dbop(c);   // synchronises
     if (rc) return rc;
@@ -1506,8 +1498,7 @@ int kspir_database_tobsgsntt(kspir_ctx* c, const uint64_t* data, uint64_t* resul
     if (bad) return set_err(c, KSPIR_ERR_INVALID_ARG, "database entries must be below bsgsp = 65537");
     // the datacrt comes out of the same pass and stays on the device for a
     // database_tocrt of exactly these rows
-    k_db_rows<true><<<dim3(kN / 2 / kDbRowsPerCta, 1), kNttThreads, kDbRowsSmem, c->stream>>>(
-        d_raw, c->dbg, d_crt, d_rows, c->N1, c->ntabs);
+    launch_db_rows<true>(c, d_raw, d_crt, d_rows, 1);
     KS_CUDA(c, cudaGetLastError());
     KS_COPY(c, h_rows, d_rows, kSubWords * 8, cudaMemcpyDeviceToHost);
     memcpy(result, h_rows, kSubWords * 8);
