@@ -58,6 +58,16 @@ __global__ void k_compose_words(const uint32_t* __restrict__ res, uint64_t* __re
     words[idx] = crt_compose_res(r[k], r[kN + k]);
 }
 
+// words[comp][k] = canonical crtMod value of column 0 of a cipherbuf in the
+// reference layout ([N][N1][2] words of two residues): 64 KiB to copy out instead
+// of the whole cipherbuf (8 MiB at N1 = 128).
+__global__ void k_compose_column(const uint64_t* __restrict__ cipherbuf, uint64_t* __restrict__ words, int N1) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= 2 * kN) return;
+    const uint64_t v = cipherbuf[(size_t)(idx % kN) * N1 * 2 + idx / kN];
+    words[idx] = crt_compose_res((uint32_t)v, (uint32_t)(v >> 32));
+}
+
 // Response words of every query of a batch: resp64 of its slot = canonical
 // words of the two residue polynomials `res` (a workspace pointer of slot 0).
 __global__ void k_compose_resp(const uint32_t* __restrict__ res, Workspace w, Batch bt) {

@@ -2404,20 +2404,12 @@ int kspir_matrix_vector_mul_bsgs_rns_crt_large(kspir_ctx* c, int client, uint64_
     // result words, and the modswitched query (cipherbuf column 0) back into query1[0]
     uint64_t* words = reinterpret_cast<uint64_t*>(c->stage32);
     k_compose_words<<<blocks_for((long)c->p.r * 2 * kN, 256), 256, 0, st>>>(w.result, words, c->p.r * 2);
+    k_compose_column<<<2 * kN / 256, 256, 0, st>>>(w.cipherbuf, c->bresp, c->N1);
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, cudaMemcpyAsync(result, words, (size_t)c->p.r * 2 * kN * 8, cudaMemcpyDeviceToHost, st));
     rc = finish(c, 0, 1);
     if (rc) return rc;
-    std::vector<uint64_t> cb((size_t)kN * c->N1 * 2);
-    KS_COPY(c, cb.data(), w.cipherbuf, cb.size() * 8, cudaMemcpyDeviceToHost);
-    for (int comp = 0; comp < 2; comp++)
-        for (int k = 0; k < kN; k++) {
-            const uint64_t wv = cb[(size_t)k * c->N1 * 2 + comp];
-            const uint64_t r1 = (uint32_t)wv, r2 = wv >> 32;
-            // canonical value with these residues (Garner on the host)
-            const uint64_t t = (uint64_t)(((hu128)((r2 + kQ2 - r1 % kQ2) % kQ2) * h_invmod(kQ1, kQ2)) % kQ2);
-            query_inout[(size_t)comp * kN + k] = r1 + (uint64_t)kQ1 * t;
-        }
+    KS_COPY(c, query_inout, c->bresp, 2 * kN * 8, cudaMemcpyDeviceToHost);
     return KSPIR_OK;
 }
 
