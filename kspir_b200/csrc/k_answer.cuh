@@ -379,7 +379,7 @@ __device__ __forceinline__ FaShape fa_shape(const FaArgs& A) {
 
 __device__ __forceinline__ void fa_run(const FaArgs& A, const FaTask& t, uint8_t* smem) {
     switch (t.type) {
-        case FT_PREP: query_prep_one(ws_at(A.w, A.bt), A.gad.baby, t.b * kNttThreads + threadIdx.x); break;
+        case FT_PREP: query_prep_one(ws_at(A.w, A.bt).q64, ws_at(A.w, A.bt), A.gad.baby, t.b * kNttThreads + threadIdx.x); break;
         case FT_QNTT: fa_ntt_job<false>(A, A.jobs[A.seg_q + t.b], smem); break;
         case FT_ROT1: fa_rotation(A, A.a1, t.b, t.a, smem); break;
         case FT_INTER_NTT: fa_ntt_job<true>(A, A.jobs[A.seg_inter + t.b], smem); break;

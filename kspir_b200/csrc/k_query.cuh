@@ -15,10 +15,10 @@ namespace kspir {
 //    modswitched rotations), and mod bsMod;
 //  * the RNS modswitch of the query itself, (x_crt - x_bs) * bsMod^-1 mod
 //    crtMod (twosteps.cpp:1073-1086), as residues before its transform.
-// k < N; ws is already the query's workspace slot.
-__device__ __forceinline__ void query_prep_one(const Workspace& ws, const GadgetBsgs& g, int k) {
-    const uint64_t a_crt = ws.q64[k], b_crt = ws.q64[kN + k];
-    const uint32_t a_bs = (uint32_t)ws.q64[2 * kN + k], b_bs = (uint32_t)ws.q64[3 * kN + k];
+// k < N; q: the query's words [4][N]; ws is already the query's workspace slot.
+__device__ __forceinline__ void query_prep_one(const uint64_t* q, const Workspace& ws, const GadgetBsgs& g, int k) {
+    const uint64_t a_crt = q[k], b_crt = q[kN + k];
+    const uint32_t a_bs = (uint32_t)q[2 * kN + k], b_bs = (uint32_t)q[3 * kN + k];
     int32_t dig[kMaxEll];
     decompose_bsgs(a_crt, a_bs, g, dig);
     for (int j = 0; j < g.ell; j++) ws.digraw[j * kN + k] = (uint32_t)dig[j];
@@ -35,15 +35,25 @@ __device__ __forceinline__ void query_prep_one(const Workspace& ws, const Gadget
     ws.col0[3 * kN + k] = shoup_mul(submod(bq2, b_bs, kQ2), c2.bsinv, c2.bsinv_p, kQ2);
 }
 
-// Also zeroes the query's giant-step accumulators (acc_words u32 words of
-// ws.result, and of ws.ecoef when two_acc): the giant steps of this answer
-// add into them.
-__global__ void k_query_prep(Workspace ws, GadgetBsgs g, Batch bt, int acc_words, int two_acc) {
-    pdl_launch_dependents();
-    pdl_wait();
+// The key slots of a launch's queries.
+constexpr int kMaxBatch = 256;     // queries per launch
+struct ClientList {
+    int n;
+    int id[kMaxBatch];
+};
+
+// First kernel of an answer.  q: the queries' words [nq][4][N], in device memory
+// or in the pinned staging of a host-buffer answer (128 KiB read once, over
+// the bus).  Also sets the key slot of each query (read by the later kernels)
+// and zeroes the query's giant-step accumulators (acc_words u32 words of
+// ws.result, and of ws.ecoef when two_acc): the giant steps of this answer add
+// into them.
+__global__ void k_query_prep(const uint64_t* q, ClientList cl, int* client_of, Workspace ws, GadgetBsgs g, Batch bt,
+                             int acc_words, int two_acc) {
     ws = ws_at(ws, bt);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < kN) query_prep_one(ws, g, k);
+    if (k == 0) client_of[batch_slot(bt)] = cl.id[blockIdx.y];
+    if (k < kN) query_prep_one(q + (size_t)blockIdx.y * 4 * kN, ws, g, k);
     const uint4 z = make_uint4(0, 0, 0, 0);
     for (int i = 4 * k; i < acc_words; i += 4 * kN) {
         *reinterpret_cast<uint4*>(ws.result + i) = z;

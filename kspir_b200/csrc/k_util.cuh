@@ -68,16 +68,18 @@ __global__ void k_compose_column(const uint64_t* __restrict__ cipherbuf, uint64_
     words[idx] = crt_compose_res((uint32_t)v, (uint32_t)(v >> 32));
 }
 
-// Response words of every query of a batch: resp64 of its slot = canonical
-// words of the two residue polynomials `res` (a workspace pointer of slot 0).
-__global__ void k_compose_resp(const uint32_t* __restrict__ res, Workspace w, Batch bt) {
-    pdl_launch_dependents();
+// Last kernel of an answer: the response words [nq][2][N] of its queries, the
+// canonical words of the two residue polynomials `res` (a workspace pointer of
+// slot 0), into device memory or the pinned staging of a host-buffer answer;
+// err_out (or null) receives the error word of the launch's first slot.
+__global__ void k_compose_resp(const uint32_t* __restrict__ res, uint64_t* resp, const int* errs, int* err_out, Batch bt) {
     pdl_wait();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx == 0 && err_out) *err_out = *reinterpret_cast<const volatile int*>(errs + (size_t)bt.slot0 * kErrStride);
     if (idx >= 2 * kN) return;
     const uint32_t* r = shifted(res, ws_off(bt)) + (size_t)(idx / kN) * 2 * kN;
     const int k = idx % kN;
-    w.resp64[(size_t)batch_slot(bt) * 2 * kN + idx] = crt_compose_res(__ldcg(r + k), __ldcg(r + kN + k));
+    resp[(size_t)blockIdx.y * 2 * kN + idx] = crt_compose_res(__ldcg(r + k), __ldcg(r + kN + k));
 }
 
 // res[p][ch][k] = words[p][k] mod q_ch (ch = q1, q2) for `polys` polynomials.

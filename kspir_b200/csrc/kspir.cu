@@ -157,18 +157,9 @@ constexpr int kTimingRing = 512;   // event sets of recent launches kept for ksp
 #define KSPIR_SINGLE_SLOTS 8
 #endif
 constexpr int kSingleSlots = KSPIR_SINGLE_SLOTS;
-constexpr int kMaxBatch = 256;     // queries per launch
-
-struct ClientList {
-    int n;
-    int id[kMaxBatch];
-};
-
-// client_of[slot0 + i] = key slot of query i of a launch (read by the kernels)
-__global__ void k_set_clients(int* client_of, int slot0, ClientList cl) {
-    const int i = threadIdx.x;
-    if (i < cl.n) client_of[slot0 + i] = cl.id[i];
-}
+// client_of[slot] = the key slot of a staged call's client (an answer's first
+// kernel sets its queries' itself)
+__global__ void k_set_client(int* client_of, int slot, int client) { client_of[slot] = client; }
 
 // scan-stage residues back to the [row][comp][ch][N] polynomial layout
 __global__ void k_unblock_sout(const uint32_t* __restrict__ sout, uint32_t* __restrict__ out, int rows) {
@@ -271,7 +262,7 @@ struct kspir_ctx {
     // before reuse).  A host-buffer answer owns its slot (slot_busy) from its
     // enqueue until it has read its response, runs on the slot's stream and
     // waits for host_done outside the mutex; its error word lands in
-    // single_errs[slot] (pinned).
+    // single_errs[slot] (pinned), its words pass through single_io[slot].
     int single_slots = 1;
     int next_single = 0;
     std::vector<cudaEvent_t> slot_done;
@@ -281,6 +272,7 @@ struct kspir_ctx {
     std::vector<char> slot_busy;
     std::vector<cudaStream_t> slot_last_stream;   // stream of each slot's last answer
     int* single_errs = nullptr;
+    uint64_t* single_io = nullptr;    // [slots][query 4N + response 2N] pinned staging
     std::condition_variable slot_cv;
     std::mutex mu;            // serialises enqueues from several host threads
 };
@@ -641,12 +633,19 @@ void launch(const kspir_ctx* c, bool pdl, void (*kern)(KArgs...), dim3 grid, dim
 // the giant steps of a sub-database need a second u32 accumulator
 bool giant_two_acc(const kspir_ctx* c) { return c->N2 - 1 > kGiantTermsPerAcc; }
 
+// query words [nq][4][N] at q -> digits and residues; key slots of the queries
+void enqueue_prep(kspir_ctx* c, int slot0, int nq, const int* clients, const uint64_t* q, cudaStream_t st) {
+    ClientList cl;
+    cl.n = nq;
+    for (int i = 0; i < nq; i++) cl.id[i] = clients[i];
+    launch(c, false, k_query_prep, dim3(kN / 256, nq), 256, 0, st, q, cl, c->client_of, c->ws0, c->gad.baby,
+           batch_of(c, slot0), c->p.r * 4 * kN, giant_two_acc(c) ? 1 : 0);
+}
+
 // rm: write the cipherbuf rotation-major (the tensor-core scans read that one)
 void enqueue_baby(kspir_ctx* c, int slot0, int nq, bool rm, cudaStream_t st) {
     const Workspace& w = c->ws0;
     const Batch bt = batch_of(c, slot0);
-    launch(c, false, k_query_prep, dim3(kN / 256, nq), 256, 0, st, w, c->gad.baby, bt, c->p.r * 4 * kN,
-           giant_two_acc(c) ? 1 : 0);
     launch(c, false, k_ntt_jobs<false>, dim3(c->n_q, nq), kNttGroup, kNttJobSmem, st,
            (const NttJob*)(c->jobs + (rm ? c->seg_q_rm : c->seg_q)), c->ntabs, bt);
     BabyArgs a1{};
@@ -797,14 +796,20 @@ void enqueue_packing(kspir_ctx* c, int slot0, int nq, cudaStream_t st, uint32_t*
         }
         cur = out;
     }
-    launch(c, nq <= kPackSplitMaxBatch, k_compose_resp, dim3(2 * kN / 256, nq), 256, 0, st, cur, w, bt);
+}
+
+// the packed residues (the last level's output, or ext for r = 1) -> response words
+void enqueue_compose(kspir_ctx* c, int slot0, int nq, uint64_t* resp, int* err_out, cudaStream_t st) {
+    const uint32_t* res = c->levels & 1 ? c->ws0.ext2 : c->ws0.ext;
+    launch(c, false, k_compose_resp, dim3(2 * kN / 256, nq), 256, 0, st, res, resp, (const int*)c->errs, err_out,
+           batch_of(c, slot0));
 }
 
 // kernels launched by one enqueue_answer
 long answer_launches(const kspir_ctx* c, int kind, int nq) {
-    // clients 1, baby 7, scan, giant 2, external product 1, packing one or two per level + compose
+    // baby 7, scan, giant 2, external product 1, packing one or two per level + compose
     const int per_level = nq <= kPackSplitMaxBatch ? 2 : 1;
-    return 1 + 7 + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + per_level * c->levels + 1;
+    return 7 + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + per_level * c->levels + 1;
 }
 
 // Captures the four non-scan phases of (slot0, nq) as CUDA graphs (the scan
@@ -820,6 +825,7 @@ int build_graphs(kspir_ctx* c, int slot0, int nq, bool rm, kspir_ctx::PhaseGraph
     cudaStream_t cs = c->capture;
     for (int ph = 0; ph < 4; ph++) {
         cudaGraph_t g = nullptr;
+        if (ph == 3 && c->levels == 0) continue;   // nothing to pack
         KS_CUDA(c, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
         if (ph == 0) enqueue_baby(c, slot0, nq, rm, cs);
         else if (ph == 1) enqueue_giant(c, slot0, nq, cs);
@@ -900,8 +906,16 @@ int enqueue_fused(kspir_ctx* c, int client, cudaStream_t st, int ring_slot) {
 
 // allow_fused: a single answer of slot 0 through the public single-answer
 // calls may run as the fused kernel (batches and serving lanes never do)
+// io: where the queries are read and the responses (and the first slot's error
+// word) written; by default the slots' device words
+struct AnswerIo {
+    const uint64_t* q = nullptr;
+    uint64_t* resp = nullptr;
+    int* err = nullptr;
+};
+
 int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStream_t st, bool allow_fused = false,
-                   bool share = false) {
+                   bool share = false, AnswerIo io = AnswerIo()) {
     const int slot = (int)(c->enqueues % kTimingRing);
     auto& ev = c->ring[slot];
     if (allow_fused && c->fused && nq == 1 && slot0 == 0) {
@@ -919,10 +933,8 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         return KSPIR_OK;
     }
     c->ring_fused[slot] = 0;
-    ClientList cl;
-    cl.n = nq;
-    for (int i = 0; i < nq; i++) cl.id[i] = clients[i];
-    k_set_clients<<<1, kMaxBatch, 0, st>>>(c->client_of, slot0, cl);
+    if (!io.q) io.q = c->bq64 + (size_t)slot0 * 4 * kN;
+    if (!io.resp) io.resp = c->bresp + (size_t)slot0 * 2 * kN;
     const int kind = scan_kind_for(c, nq);
     c->last_kind = kind;
     if (c->use_graphs) {
@@ -930,6 +942,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         int rc = build_graphs(c, slot0, nq, kind != SCAN_CUDA, &pg);
         if (rc) return rc;
         cudaEventRecord(ev[0], st);
+        enqueue_prep(c, slot0, nq, clients, io.q, st);
         KS_CUDA(c, cudaGraphLaunch(pg->g[0], st));
         cudaEventRecord(ev[1], st);
         enqueue_scan(c, slot0, nq, kind, st, share);
@@ -938,10 +951,12 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         cudaEventRecord(ev[3], st);
         KS_CUDA(c, cudaGraphLaunch(pg->g[2], st));
         cudaEventRecord(ev[4], st);
-        KS_CUDA(c, cudaGraphLaunch(pg->g[3], st));
+        if (pg->g[3]) KS_CUDA(c, cudaGraphLaunch(pg->g[3], st));
+        enqueue_compose(c, slot0, nq, io.resp, io.err, st);
         cudaEventRecord(ev[5], st);
     } else {
         cudaEventRecord(ev[0], st);
+        enqueue_prep(c, slot0, nq, clients, io.q, st);
         enqueue_baby(c, slot0, nq, kind != SCAN_CUDA, st);
         cudaEventRecord(ev[1], st);
         enqueue_scan(c, slot0, nq, kind, st, share);
@@ -951,6 +966,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         enqueue_ext(c, slot0, nq, c->p.r, nullptr, nullptr, st);
         cudaEventRecord(ev[4], st);
         enqueue_packing(c, slot0, nq, st);
+        enqueue_compose(c, slot0, nq, io.resp, io.err, st);
         cudaEventRecord(ev[5], st);
     }
     c->ring_nq[slot] = nq;
@@ -1300,6 +1316,7 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
         KS_CUDA(c.get(), cudaStreamCreateWithFlags(&c->slot_stream[i], cudaStreamNonBlocking));
     }
     KS_CUDA(c.get(), cudaHostAlloc(&c->single_errs, (size_t)c->single_slots * 4, cudaHostAllocDefault));
+    KS_CUDA(c.get(), cudaHostAlloc(&c->single_io, (size_t)c->single_slots * 6 * kN * 8, cudaHostAllocDefault));
     rc = init_key_slots(c.get());
     if (rc) return rc;
     rc = init_workspaces(c.get());
@@ -1322,6 +1339,7 @@ int kspir_ctx_destroy(kspir_ctx* c) {
     for (auto& e : c->host_done) if (e) cudaEventDestroy(e);
     for (auto& st : c->slot_stream) if (st) cudaStreamDestroy(st);
     if (c->single_errs) cudaFreeHost(c->single_errs);
+    if (c->single_io) cudaFreeHost(c->single_io);
     for (auto& kv : c->graphs)
         for (auto& g : kv.second.g) if (g) cudaGraphExecDestroy(g);
     if (c->capture) cudaStreamDestroy(c->capture);
@@ -2172,27 +2190,43 @@ int kspir_answer(kspir_ctx* c, int client, const uint64_t* query, uint64_t* resp
     c->slot_busy[slot] = 1;
     SlotHold hold{c, slot};
     cudaStream_t st = c->slot_stream[slot];
+    // the words pass through the slot's pinned staging, which the answer's first
+    // and last kernels read and write themselves: no copy on the stream, and a
+    // caller with pageable buffers waits outside the mutex
+    uint64_t* hq = c->single_io + (size_t)slot * 6 * kN;
+    uint64_t* hr = hq + 4 * kN;
+    lk.unlock();
+    memcpy(hq, query, 4 * kN * 8);
+    lk.lock();
     const bool share = singles_beside(c, slot, st);
     if (c->slot_used[slot]) KS_CUDA(c, cudaStreamWaitEvent(st, c->slot_done[slot], 0));
-    KS_CUDA(c, cudaMemcpyAsync(c->bq64 + (size_t)slot * 4 * kN, query, 4 * kN * 8, cudaMemcpyHostToDevice, st));
-    rc = enqueue_answer(c, slot, 1, &client, st, true, share);
-    if (rc) return rc;
-    KS_CUDA(c, cudaGetLastError());
-    // the query is validated while the device answers it; a non-canonical one
-    // is reported before anything reaches the caller's response buffer
-    const bool ok = canonical(query, 2 * kN, kCrtMod) && canonical(query + 2 * kN, 2 * kN, kBsMod);
-    if (ok) {
-        KS_CUDA(c, cudaMemcpyAsync(response, c->bresp + (size_t)slot * 2 * kN, 2 * kN * 8, cudaMemcpyDeviceToHost, st));
+    if (c->fused) {
+        KS_CUDA(c, cudaMemcpyAsync(c->bq64 + (size_t)slot * 4 * kN, hq, 4 * kN * 8, cudaMemcpyHostToDevice, st));
+        rc = enqueue_answer(c, slot, 1, &client, st, true, share);
+        if (rc) return rc;
+        KS_CUDA(c, cudaMemcpyAsync(hr, c->bresp + (size_t)slot * 2 * kN, 2 * kN * 8, cudaMemcpyDeviceToHost, st));
         KS_CUDA(c, cudaMemcpyAsync(c->single_errs + slot, c->errs + (size_t)slot * kErrStride, 4,
                                    cudaMemcpyDeviceToHost, st));
+    } else {
+        AnswerIo io;
+        io.q = hq;
+        io.resp = hr;
+        io.err = c->single_errs + slot;
+        rc = enqueue_answer(c, slot, 1, &client, st, false, share, io);
+        if (rc) return rc;
     }
+    KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, cudaEventRecord(c->slot_done[slot], st));
     KS_CUDA(c, cudaEventRecord(c->host_done[slot], st));
     c->slot_used[slot] = 1;
     c->slot_last_stream[slot] = st;
-    // other host calls enqueue while this one waits for its answer
+    // other host calls enqueue while this one validates its query and waits for
+    // its answer; a non-canonical query is reported before anything reaches the
+    // caller's response buffer
     lk.unlock();
+    const bool ok = canonical(hq, 2 * kN, kCrtMod) && canonical(hq + 2 * kN, 2 * kN, kBsMod);
     const cudaError_t e = cudaEventSynchronize(c->host_done[slot]);
+    if (e == cudaSuccess && ok && !c->single_errs[slot]) memcpy(response, hr, 2 * kN * 8);
     lk.lock();
     if (e != cudaSuccess) return set_err(c, KSPIR_ERR_CUDA, cudaGetErrorString(e));
     if (!ok) return set_err(c, KSPIR_ERR_INVALID_ARG, "query word not canonical");
@@ -2397,7 +2431,7 @@ int kspir_matrix_vector_mul_bsgs_rns_crt_large(kspir_ctx* c, int client, uint64_
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
     KS_CUDA(c, cudaMemcpyAsync(c->bq64, query_inout, 4 * kN * 8, cudaMemcpyHostToDevice, st));
-    k_set_clients<<<1, 32, 0, st>>>(c->client_of, 0, ClientList{1, {client}});
+    enqueue_prep(c, 0, 1, &client, c->bq64, st);
     enqueue_baby(c, 0, 1, false, st);
     enqueue_scan(c, 0, 1, SCAN_CUDA, st);
     enqueue_giant(c, 0, 1, st);
@@ -2426,7 +2460,7 @@ int kspir_external_product(kspir_ctx* c, int client, uint64_t* result, uint64_t*
     cudaStream_t st = c->stream;
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
-    k_set_clients<<<1, 32, 0, st>>>(c->client_of, 0, ClientList{1, {client}});
+    k_set_client<<<1, 1, 0, st>>>(c->client_of, 0, client);
     uint64_t* words = reinterpret_cast<uint64_t*>(c->stage32);     // r*2*N u64 fit in r*4*N u32
     // first_dim -> ws.result residues; the caller's accumulators (NTT domain) -> ws.sout residues
     KS_CUDA(c, cudaMemcpyAsync(words, first_dim, n * 8, cudaMemcpyHostToDevice, st));
@@ -2459,7 +2493,7 @@ int kspir_packing_rlwes(kspir_ctx* c, int client, uint64_t* rlwes, uint64_t* res
     cudaStream_t st = c->stream;
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
-    k_set_clients<<<1, 32, 0, st>>>(c->client_of, 0, ClientList{1, {client}});
+    k_set_client<<<1, 1, 0, st>>>(c->client_of, 0, client);
     uint64_t* words = reinterpret_cast<uint64_t*>(c->stage32);
     KS_CUDA(c, cudaMemcpyAsync(words, rlwes, n * 8, cudaMemcpyHostToDevice, st));
     k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(words, w.ext, R * 2);
@@ -2467,6 +2501,7 @@ int kspir_packing_rlwes(kspir_ctx* c, int client, uint64_t* rlwes, uint64_t* res
     // the scan-output region, which the packing does not use)
     uint32_t* c2 = w.sout;
     enqueue_packing(c, 0, 1, st, c2);
+    enqueue_compose(c, 0, 1, c->bresp, nullptr, st);
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, cudaMemcpyAsync(response, c->bresp, 2 * kN * 8, cudaMemcpyDeviceToHost, st));
     if (R > 1) {
