@@ -63,6 +63,34 @@ __host__ __device__ __forceinline__ size_t cipherbuf_rm_idx(int col, int comp, i
     return ((size_t)(col * 2 + comp) * 2 + ch) * kN + z;
 }
 
+// Rotation-major columns into the reference layout ([z][col] of four words: a q1,
+// a q2, b q1, b q2), for the CUDA-core scan.  One CTA per 32 slots and 64 columns
+// (grid.z: query): 128-byte rows in, 1 KiB pieces out, through 32 KiB of shared
+// memory where slot z of column col sits at z ^ (col mod 32), so that both sides
+// touch 32 distinct banks.
+constexpr int kCbRowsZ = 32, kCbRowsCols = 64;
+__global__ void __launch_bounds__(256) k_cipherbuf_rows(const uint32_t* __restrict__ rm, uint64_t* __restrict__ cbuf,
+                                                        int N1, Batch bt) {
+    __shared__ uint32_t V[kCbRowsCols * 4 * kCbRowsZ];
+    const size_t wo = (size_t)(bt.slot0 + (int)blockIdx.z) * bt.ws_bytes;
+    rm = shifted(rm, wo);
+    uint4* out = reinterpret_cast<uint4*>(shifted(cbuf, wo));
+    const int z0 = blockIdx.x * kCbRowsZ, c0 = blockIdx.y * kCbRowsCols;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < kCbRowsCols * 4 / 8; i++) {
+        const int row = warp + 8 * i;   // col * 4 + comp * 2 + ch
+        V[row * kCbRowsZ + (lane ^ ((row >> 2) & 31))] = __ldcg(rm + ((size_t)c0 * 4 + row) * kN + z0 + lane);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kCbRowsZ * kCbRowsCols / 256; i++) {
+        const int t = threadIdx.x + 256 * i, col = t % kCbRowsCols, z = t / kCbRowsCols;
+        const uint32_t* v = V + col * 4 * kCbRowsZ + (z ^ (col & 31));
+        out[(size_t)(z0 + z) * N1 + c0 + col] = make_uint4(v[0], v[kCbRowsZ], v[2 * kCbRowsZ], v[3 * kCbRowsZ]);
+    }
+}
+
 constexpr int kBabyEll = 3;
 constexpr int kBabyPolys1 = 2, kBabyPolys2 = 4;   // padded polynomials: x2 of one or two components, per prime
 

@@ -220,7 +220,7 @@ struct kspir_ctx {
     int* client_of = nullptr;         // [slots]
     uint32_t* stage32 = nullptr;      // [r][4][N] residues for the staged entry points
     NttJob* jobs = nullptr;           // transform job lists of slot 0
-    int seg_q = 0, seg_q_rm = 0, n_q = 0, seg_inter = 0, seg_dig1 = 0;
+    int seg_q = 0, seg_q_rm = 0, seg_q_so = 0, n_q = 0, seg_inter = 0, seg_dig1 = 0;
     // client keys: key slot k is slot 0's layout shifted by k * key_bytes
     uint32_t* key_mem = nullptr;
     size_t key_bytes = 0;
@@ -501,7 +501,8 @@ int init_workspaces(kspir_ctx* c) {
         {(void**)&w.inter_acoef, 2 * P},
         {(void**)&w.dig1, 12 * P},
         {(void**)&w.cipherbuf, (size_t)kN * N1 * 2 * 8},
-        {(void**)&w.sout, (size_t)r * N2 * 4 * P},
+        // the scan output; before the scan, the rotations of a CUDA-core scan (enqueue_baby)
+        {(void**)&w.sout, std::max((size_t)r * N2 * 4 * P, (size_t)kN * N1 * 2 * 8)},
         {(void**)&w.result, (size_t)r * 4 * P},
         {(void**)&w.ecoef, (size_t)r * 4 * P},
         {(void**)&w.ext, (size_t)r * 4 * P},
@@ -536,19 +537,20 @@ int init_workspaces(kspir_ctx* c) {
         NttJob j; j.src = src; j.dst = dst; j.ch = ch; j.dst_stride = stride; jobs.push_back(j);
     };
     // query: dig0 (9 digits, 3 b), modswitched query -> cipherbuf column 0 (4);
-    // a second copy writes column 0 of the rotation-major cipherbuf
+    // further copies write column 0 rotation-major, in the cipherbuf (tensor-core
+    // scans) and in the scan output's region (CUDA-core scan)
     uint32_t* cb32 = reinterpret_cast<uint32_t*>(w.cipherbuf);
-    for (int rm = 0; rm < 2; rm++) {
-        (rm ? c->seg_q_rm : c->seg_q) = (int)jobs.size();
+    for (int rm = 0; rm < 3; rm++) {
+        (rm == 2 ? c->seg_q_so : rm ? c->seg_q_rm : c->seg_q) = (int)jobs.size();
         for (int j = 0; j < 3; j++)
             for (int ch = 0; ch < 3; ch++) add(w.digraw + j * kN, w.dig0 + (size_t)ch * 4 * kN + j, ch, 4);
         for (int ch = 0; ch < 3; ch++) add(w.qb + ch * kN, w.dig0 + (size_t)ch * 4 * kN + 3, ch, 4);
         for (int comp = 0; comp < 2; comp++)
             for (int ch = 0; ch < 2; ch++) {
-                if (rm) add(w.col0 + (comp * 2 + ch) * kN, cb32 + cipherbuf_rm_idx(0, comp, ch, 0), ch, 1);
+                if (rm) add(w.col0 + (comp * 2 + ch) * kN, (rm == 2 ? w.sout : cb32) + cipherbuf_rm_idx(0, comp, ch, 0), ch, 1);
                 else add(w.col0 + (comp * 2 + ch) * kN, cb32 + 2 * comp + ch, ch, 4 * N1);
             }
-        c->n_q = (int)jobs.size() - (rm ? c->seg_q_rm : c->seg_q);
+        if (!rm) c->n_q = (int)jobs.size() - c->seg_q;
     }
     c->seg_inter = (int)jobs.size();
     for (int ch = 0; ch < 2; ch++) add(w.interA + ch * kN, w.inter_acoef + ch * kN, ch, 1);
@@ -642,16 +644,21 @@ void enqueue_prep(kspir_ctx* c, int slot0, int nq, const int* clients, const uin
            batch_of(c, slot0), c->p.r * 4 * kN, giant_two_acc(c) ? 1 : 0);
 }
 
-// rm: write the cipherbuf rotation-major (the tensor-core scans read that one)
+// rm: leave the cipherbuf rotation-major (the tensor-core scans read that one).
+// Otherwise the rotations are written rotation-major into the scan output's
+// region, whose turn comes later, and transposed from there: 4-byte stores into
+// the reference layout, 2 KiB apart, took 23 of the 74 us of a single answer's
+// baby steps, the transpose takes 6.
 void enqueue_baby(kspir_ctx* c, int slot0, int nq, bool rm, cudaStream_t st) {
     const Workspace& w = c->ws0;
     const Batch bt = batch_of(c, slot0);
     launch(c, false, k_ntt_jobs<false>, dim3(c->n_q, nq), kNttGroup, kNttJobSmem, st,
-           (const NttJob*)(c->jobs + (rm ? c->seg_q_rm : c->seg_q)), c->ntabs, bt);
+           (const NttJob*)(c->jobs + (rm ? c->seg_q_rm : c->seg_q_so)), c->ntabs, bt);
     BabyArgs a1{};
-    a1.cb_rm = rm ? 1 : 0;
+    a1.cb_rm = 1;
     a1.dig = w.dig0; a1.perms = c->perms; a1.sigma = c->sigma_baby;
-    a1.cipherbuf = w.cipherbuf; a1.interA = w.interA; a1.inter_dig = w.dig1; a1.inter_bs = w.inter_bs;
+    a1.cipherbuf = rm ? w.cipherbuf : reinterpret_cast<uint64_t*>(w.sout);
+    a1.interA = w.interA; a1.inter_dig = w.dig1; a1.inter_bs = w.inter_bs;
     a1.N1 = c->N1; a1.col_base = 1; a1.inter_idx = c->N1h - 2;
     auto rot = [&](const BabyArgs& args, int nrot) {
         if (nrot <= 0) return;
@@ -672,6 +679,9 @@ void enqueue_baby(kspir_ctx* c, int slot0, int nq, bool rm, cudaStream_t st) {
     a2.dig = w.dig1;
     a2.col_base = c->N1h; a2.inter_idx = -1;
     rot(a2, c->N1h);
+    if (!rm)
+        launch(c, false, k_cipherbuf_rows, dim3(kN / kCbRowsZ, c->N1 / kCbRowsCols, nq), 256, 0, st,
+               (const uint32_t*)w.sout, w.cipherbuf, c->N1, bt);
 }
 
 int scan_kind_for(kspir_ctx* c, int nq) {
@@ -807,9 +817,9 @@ void enqueue_compose(kspir_ctx* c, int slot0, int nq, uint64_t* resp, int* err_o
 
 // kernels launched by one enqueue_answer
 long answer_launches(const kspir_ctx* c, int kind, int nq) {
-    // baby 7, scan, giant 2, external product 1, packing one or two per level + compose
+    // baby 7 (and the transpose of a CUDA-core scan's), scan, giant 2, external product 1, packing one or two per level + compose
     const int per_level = nq <= kPackSplitMaxBatch ? 2 : 1;
-    return 7 + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + per_level * c->levels + 1;
+    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + per_level * c->levels + 1;
 }
 
 // Captures the four non-scan phases of (slot0, nq) as CUDA graphs (the scan
