@@ -193,17 +193,18 @@ __device__ __forceinline__ uint64_t crt_compose_res(uint32_t r1, uint32_t r2) {
 // unsigned minimum for code compiled for the host as well
 __host__ __device__ __forceinline__ uint32_t min_u32(uint32_t a, uint32_t b) { return a < b ? a : b; }
 
-// x mod q, exact for every 64-bit x, q a prime in (2^27, 2^28); mu1 = 2^59 / q,
-// c32 = 2^32 mod q, mu2 = 2^57 / q.  Two Barrett steps with 32x32 products.
-__host__ __device__ __forceinline__ uint32_t mod28(uint64_t x, uint32_t q, uint32_t mu1, uint32_t c32, uint32_t mu2) {
-    const uint32_t xh = (uint32_t)(x >> 32), xl = (uint32_t)x;
-    // conditional subtractions as minima (x - m wraps above x when x < m)
-    uint32_t r = xh - (uint32_t)(((uint64_t)xh * mu1) >> 59) * q;   // in [0, 2q)
-    r = min_u32(r, r - q);
-    const uint64_t y = (uint64_t)r * c32 + xl;                       // < 2^57, same residue
-    const uint32_t qh = (uint32_t)(((y >> 26) * mu2) >> 31);
-    uint32_t t = (uint32_t)y - qh * q;                                // in [0, 3q)
-    t = min_u32(t, t - 2 * q);                                        // in [0, 2q)
+// x mod q, exact for every 64-bit x = xl + 2^32 xh, q one of the crt primes; c32 =
+// 2^32 mod q, mu = floor(2^59 / q).  The high word is brought below 2^29.1 with its
+// quotient by 2^28 (q is within 7 % of it), so y = (its residue) 2^32 + xl is below
+// 2^57.1; the estimate umulhi(y >> 27, mu) of y / q falls short by less than 1.8
+// (0.26 from mu, 0.54 from the shift, 1 from its floor), so one conditional
+// subtraction finishes.
+__host__ __device__ __forceinline__ uint32_t mod28(uint64_t x, uint32_t q, uint32_t c32, uint32_t mu) {
+    const uint32_t xh = (uint32_t)(x >> 32);
+    const uint32_t r = xh - (xh >> 28) * q;
+    const uint64_t y = (uint64_t)r * c32 + (uint32_t)x;
+    const uint32_t qh = (uint32_t)(((uint64_t)(uint32_t)(y >> 27) * mu) >> 32);
+    const uint32_t t = (uint32_t)y - qh * q;   // in [0, 1.8 q)
     return min_u32(t, t - q);
 }
 

@@ -27,15 +27,23 @@
 // engine, no multicast) at a 1 KiB-aligned stage.
 //
 // Work: a unit is (ZB consecutive NTT slots, prime, query tile); its ZB query
-// tiles stay resident while the database tiles stream through a ring in the
-// order (row group g, slot).  The epilogue keeps the ZB results of one
+// tiles stay resident while the database tiles stream through a ring, two row
+// groups at a time: (g, slot), (g + 1, slot), next slot.  The epilogue keeps the ZB results of one
 // (row, component, query) in registers and writes them as 16-byte pieces of
 // the blocked scan output (sout_idx), where the eight row lanes of a query
 // cover two 128-byte lines.
 //
 // Warp roles: warp 0 producer (one lane), warp 1 TMEM allocation and MMA issue
 // (one lane), warps 2.. epilogue (warp w reads TMEM lanes 32 (w % 4) .. and a
-// 1/PARTS share of the 16-column chunks).  Every wait is bounded; on a timeout
+// 1/PARTS share of the 16-column chunks).  What bounds a tile is the round trip
+// MMA - epilogue loads - accumulator given back, not a unit (without the
+// reductions it takes as long, without stores 0.07 ms less): so the epilogue
+// warps work in two sets, one per row-group parity, each with its own
+// accumulators, and one set's loads overlap the other's reductions.  Batch of 64
+// at r = 16, with the operand split: 0.98 ms with every warp on every tile and
+// per-store 64-bit addresses, 0.89 ms with TMEM addresses in uniform registers
+// and linear store addresses, 0.85 ms with the two sets; batch of 32 at r = 64:
+// 1.65, 1.52, 1.43 ms.  Every wait is bounded; on a timeout
 // the warp sets the error word and leaves its loop, the producer waits for its
 // own copies in flight, the MMA lane for its own MMAs, and TMEM is freed.
 #pragma once
@@ -69,13 +77,16 @@ struct MmaCfg {
     static constexpr int NA = NA_FIT < 6 ? NA_FIT : 6;  // database-tile ring
     static constexpr int SMEM = 1024 + ZB * BTILE + NA * kATile + BAR_BYTES;
     static constexpr int CHUNKS = N / 16;             // 16-column chunks = 4 query groups each
-    static constexpr int PARTS = CHUNKS < 4 ? CHUNKS : 4;   // epilogue warps per TMEM quarter
+    static constexpr int SETS = 2;                    // sets of epilogue warps: set s takes the row groups g % SETS = s
+    static constexpr int NTS = NTB / SETS;            // TMEM accumulators per set
+    static constexpr int PARTS = 2;                   // epilogue warps per TMEM quarter and set
     static constexpr int CPW = CHUNKS / PARTS;        // chunks (outputs per lane) per epilogue warp
     static constexpr int LDB = CPW < 2 ? CPW : 2;     // outputs whose TMEM loads share one wait
-    static constexpr int EPI = 4 * PARTS;             // epilogue warps
+    static constexpr int EPI = 4 * PARTS * SETS;      // epilogue warps
     static constexpr int THREADS = 32 * (2 + EPI);
     static_assert(NA >= 2 && SMEM <= kMmaSmemLimit, "shared memory budget");
     static_assert(NTB * N <= 512, "TMEM columns");
+    static_assert(4 * CPW <= BT, "an epilogue warp's chunks belong to one component");
 };
 
 // tile row of database row j (0..31) limb la, and of query group g limb lb
@@ -148,11 +159,12 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
     uint64_t* done = t_empty + C::NTB;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the warp index as a value known to be uniform: TMEM addresses stay in uniform registers
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < C::NA; s++) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
         for (int s = 0; s < C::ZB; s++) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
-        for (int s = 0; s < C::NTB; s++) { mbar_init(&t_full[s], 1); mbar_init(&t_empty[s], C::EPI); }
+        for (int s = 0; s < C::NTB; s++) { mbar_init(&t_full[s], 1); mbar_init(&t_empty[s], C::EPI / C::SETS); }
         mbar_init(done, 1);
         fence_mbar_init();
     }
@@ -178,10 +190,11 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, tu++) {
                 const int qt = u % QT, ch = (u / QT) & 1, z0 = (u / QT >> 1) * C::ZB;
-                for (int g = 0; g < G && ok; g++)
+                // the sets' row groups alternate tile by tile
+                for (int gp = 0; gp < G && ok; gp += C::SETS)
                     for (int zi = 0; zi < C::ZB && ok; zi++) {
                         const int z = z0 + zi;
-                        if (g == 0) {
+                        if (gp == 0) {
                             if (tu > 0 && !mbar_wait_bounded(&b_empty[zi], (uint32_t)((tu - 1) & 1), kMmaWaitNs)) {
                                 atomicOr(a.err, 8); ok = false; break;
                             }
@@ -190,14 +203,16 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                                      C::BTILE, &b_full[zi]);
                             bl[zi]++;
                         }
-                        const int sa = (int)(ia % C::NA);
-                        if (ia >= C::NA && !mbar_wait_bounded(&a_empty[sa], (uint32_t)((ia / C::NA - 1) & 1), kMmaWaitNs)) {
-                            atomicOr(a.err, 8); ok = false; break;
+                        for (int g = gp; g < gp + C::SETS && g < G; g++) {
+                            const int sa = (int)(ia % C::NA);
+                            if (ia >= C::NA && !mbar_wait_bounded(&a_empty[sa], (uint32_t)((ia / C::NA - 1) & 1), kMmaWaitNs)) {
+                                atomicOr(a.err, 8); ok = false; break;
+                            }
+                            mbar_arrive_expect_tx(&a_full[sa], kATile);
+                            bulk_g2s(atiles + sa * kATile, a.dbop + (((size_t)z * 2 + ch) * G + g) * kATile, kATile,
+                                     &a_full[sa]);
+                            ia++;
                         }
-                        mbar_arrive_expect_tx(&a_full[sa], kATile);
-                        bulk_g2s(atiles + sa * kATile, a.dbop + (((size_t)z * 2 + ch) * G + g) * kATile, kATile,
-                                 &a_full[sa]);
-                        ia++;
                     }
             }
             // never leave with copies in flight into shared memory
@@ -212,43 +227,49 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
         if (lane == 0) {
             const uint32_t idesc = mma_idesc_u8(C::N);
             const uint32_t abase = smem_addr(atiles), bbase = smem_addr(btiles);
-            long ia = 0, tc = 0;
+            long ia = 0, tc[C::SETS] = {};
             int tu = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, tu++) {
-                for (int g = 0; g < G && ok; g++)
-                    for (int zi = 0; zi < C::ZB; zi++) {
-                        if (g == 0 && !mbar_wait_bounded(&b_full[zi], (uint32_t)(tu & 1), kMmaWaitNs)) {
+                for (int gp = 0; gp < G && ok; gp += C::SETS)
+                    for (int zi = 0; zi < C::ZB && ok; zi++) {
+                        if (gp == 0 && !mbar_wait_bounded(&b_full[zi], (uint32_t)(tu & 1), kMmaWaitNs)) {
                             atomicOr(a.err, 32); ok = false; break;
                         }
-                        const int sa = (int)(ia % C::NA);
-                        if (!mbar_wait_bounded(&a_full[sa], (uint32_t)((ia / C::NA) & 1), kMmaWaitNs)) {
-                            atomicOr(a.err, 32); ok = false; break;
-                        }
-                        const int tb = (int)(tc % C::NTB);
-                        if (tc >= C::NTB &&
-                            !mbar_wait_bounded(&t_empty[tb], (uint32_t)((tc / C::NTB - 1) & 1), kMmaWaitNs)) {
-                            atomicOr(a.err, 32); ok = false; break;
-                        }
-                        tc_fence_after();
-                        const uint64_t ad = mma_sdesc_sw128(abase + sa * kATile);
-                        const uint64_t bd = mma_sdesc_sw128(bbase + zi * C::BTILE);
 #pragma unroll
-                        for (int kk = 0; kk < kMmaK / 32; kk++)
-                            mma_u8(tmem + tb * C::N, ad + 2 * kk, bd + 2 * kk, idesc, kk > 0);
-                        mma_commit(&a_empty[sa]);
-                        if (g == G - 1) mma_commit(&b_empty[zi]);
-                        mma_commit(&t_full[tb]);
-                        ia++;
-                        tc++;
+                        for (int s = 0; s < C::SETS; s++) {
+                            const int g = gp + s;
+                            if (g >= G || !ok) break;
+                            const int sa = (int)(ia % C::NA);
+                            if (!mbar_wait_bounded(&a_full[sa], (uint32_t)((ia / C::NA) & 1), kMmaWaitNs)) {
+                                atomicOr(a.err, 32); ok = false; break;
+                            }
+                            const int tb = s + C::SETS * (int)(tc[s] % C::NTS);
+                            if (tc[s] >= C::NTS &&
+                                !mbar_wait_bounded(&t_empty[tb], (uint32_t)((tc[s] / C::NTS - 1) & 1), kMmaWaitNs)) {
+                                atomicOr(a.err, 32); ok = false; break;
+                            }
+                            tc_fence_after();
+                            const uint64_t ad = mma_sdesc_sw128(abase + sa * kATile);
+                            const uint64_t bd = mma_sdesc_sw128(bbase + zi * C::BTILE);
+#pragma unroll
+                            for (int kk = 0; kk < kMmaK / 32; kk++)
+                                mma_u8(tmem + tb * C::N, ad + 2 * kk, bd + 2 * kk, idesc, kk > 0);
+                            mma_commit(&a_empty[sa]);
+                            if (g == G - 1) mma_commit(&b_empty[zi]);
+                            mma_commit(&t_full[tb]);
+                            ia++;
+                            tc[s]++;
+                        }
                     }
             }
             mma_commit(done);
             if (!mbar_wait_bounded(done, 0, kMmaWaitNs)) atomicOr(a.err, 64);
         }
     } else {
-        // epilogue: warp (quarter q, part p) owns TMEM lanes 32q.. and chunks p*CPW ..
-        const int quarter = warp & 3, part = (warp - 2) >> 2;
+        // epilogue: warp (quarter q, part p) of set s owns TMEM lanes 32q.. and
+        // chunks p*CPW .. of its set's tiles
+        const int quarter = warp & 3, part = ((warp - 2) >> 2) % C::PARTS, set = (warp - 2) / (4 * C::PARTS);
         const int j3 = lane >> 2, gq = lane & 3;
         const int jrow = 8 * quarter + j3;   // database row within the 32-row tile
         const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16) + part * C::CPW * 16;
@@ -258,15 +279,21 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             const int qt = u % QT, ch = (u / QT) & 1, z0 = (u / QT >> 1) * C::ZB;
             const uint32_t q = ch ? kQ2 : kQ1;
-            const uint32_t mu1 = ch ? (uint32_t)((1ull << 59) / kQ2) : (uint32_t)((1ull << 59) / kQ1);
+            const uint32_t mu = ch ? (uint32_t)((1ull << 59) / kQ2) : (uint32_t)((1ull << 59) / kQ1);
             const uint32_t c32 = ch ? (uint32_t)((1ull << 32) % kQ2) : (uint32_t)((1ull << 32) % kQ1);
-            const uint32_t mu2 = ch ? (uint32_t)((1ull << 57) / kQ2) : (uint32_t)((1ull << 57) / kQ1);
-            for (int g = 0; g < G && ok; g++) {
+            // this lane's first query (its chunks' queries are four apart, all of one
+            // component) and its place in that query's scan output: 32 rows
+            // (eight blocks of four) further for each row group
+            const int bq0 = qt * BT + (4 * part * C::CPW + gq) % BT;
+            const int cv = 4 * part * C::CPW / BT * 2 + ch;
+            char* so = reinterpret_cast<char*>(a.sout0 + sout_idx(32 * set + jrow, cv, z0, a.rows)) +
+                       (size_t)(a.slot0 + bq0) * a.ws_bytes;
+            for (int g = set; g < G && ok; g += C::SETS, so += sout_idx(32 * C::SETS, 0, 0, 0) * 4) {
 #pragma unroll
                 for (int zi = 0; zi < C::ZB; zi++) {
-                    const int tb = (int)(tc % C::NTB);
+                    const int tb = set + C::SETS * (int)(tc % C::NTS);
                     // warp-uniform outcome: tcgen05.ld below needs the whole warp
-                    const bool got = mbar_wait_bounded(&t_full[tb], (uint32_t)((tc / C::NTB) & 1), kMmaWaitNs);
+                    const bool got = mbar_wait_bounded(&t_full[tb], (uint32_t)((tc / C::NTS) & 1), kMmaWaitNs);
                     if (!__all_sync(0xffffffffu, got)) {
                         if (lane == 0) atomicOr(a.err, 128);
                         ok = false;
@@ -294,13 +321,13 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                             const uint32_t t3 = L[5] + L[6] + H[1] + H[2];
                             const uint32_t t4 = L[7] + H[4] + H[3];
                             const uint32_t t5 = H[5] + H[6];
-                            uint64_t x = L[0];
-                            mad_wide(x, t1, 1u << 8);
+                            // weights 1 and 2^8 stay below 2^32 (each limb product sums to at
+                            // most 128 * 255^2); weights 2^32.. wrap mod 2^64
+                            const uint32_t xl = L[0] + (t1 << 8), xh = t4 + (t5 << 8) + (H[7] << 16);
+                            uint64_t x = (uint64_t)xh << 32 | xl;
                             mad_wide(x, t2, 1u << 16);
                             mad_wide(x, t3, 1u << 24);
-                            const uint32_t xh = t4 + (t5 << 8) + (H[7] << 16);   // weights 2^32.. (mod 2^64)
-                            x += (uint64_t)xh << 32;
-                            ob[zi][c0 + c1] = mod28(x, q, mu1, c32, mu2);
+                            ob[zi][c0 + c1] = mod28(x, q, c32, mu);
                         }
                     }
                     tc_fence_before();
@@ -309,20 +336,16 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                     tc++;
                 }
                 if (!ok) break;
-                const int row = 32 * g + jrow;
-                if (row < a.rows) {
+                if (32 * g + jrow < a.rows) {
+                    char* o = so;
 #pragma unroll
-                    for (int c = 0; c < C::CPW; c++) {
-                        const int grp = 4 * (part * C::CPW + c) + gq;   // comp * BT + b
-                        const int comp = grp / BT, bq = qt * BT + grp % BT;
-                        if (bq < a.nq) {
-                            uint32_t* so = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(a.sout0) +
-                                                                       (size_t)(a.slot0 + bq) * a.ws_bytes);
+                    for (int c = 0; c < C::CPW; c++, o += 4 * a.ws_bytes) {
+                        if (bq0 + 4 * c < a.nq) {
                             // four consecutive slots per 16-byte store; the eight
                             // row lanes of this query cover two 128-byte lines
 #pragma unroll
                             for (int z4 = 0; z4 < C::ZB; z4 += 4)
-                                *reinterpret_cast<uint4*>(so + sout_idx(row, comp * 2 + ch, z0 + z4, a.rows)) =
+                                *reinterpret_cast<uint4*>(o + 4 * z4) =
                                     make_uint4(ob[z4][c], ob[z4 + 1][c], ob[z4 + 2][c], ob[z4 + 3][c]);
                         }
                     }

@@ -689,7 +689,12 @@ int scan_kind_for(kspir_ctx* c, int nq) {
     auto it = c->scan_choice.find(nq);
     if (it != c->scan_choice.end()) return it->second;
     if (nq == 1) return SCAN_CUDA;
-    return nq >= 16 ? SCAN_MMA16 : nq >= 8 ? SCAN_MMA8 : SCAN_MMA4;
+    // the smallest query tile that holds the batch in one pass over the database,
+    // else the largest (fewest passes); r = 16, scan with its operand split, us:
+    // n = 4: 221 (tile 4), 235 (8); n = 8: 244 (8), 275 (16); n = 13: 468 (8), 294
+    // (16), 342 (32); n = 17: 690, 540, 358; n = 40: 1196, 846, 829; n = 64: 1895,
+    // 1173, 879.  (At r = 2 tiles of 16 are 10 % faster for 33 to 48 queries.)
+    return nq > 16 ? SCAN_MMA32 : nq > 8 ? SCAN_MMA16 : nq > 4 ? SCAN_MMA8 : SCAN_MMA4;
 }
 
 long scan_launches(const kspir_ctx* c, int kind, int nq) { return kind == SCAN_CUDA ? nq : 2; }
