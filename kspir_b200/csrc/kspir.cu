@@ -784,11 +784,24 @@ void enqueue_giant(kspir_ctx* c, int slot0, int nq, cudaStream_t st) {
 void enqueue_ext(kspir_ctx* c, int slot0, int nq, int count, const uint32_t* init, uint32_t* coef_out,
                  cudaStream_t st) {
     const Workspace& w = c->ws0;
-    launch(c, false, k_ext_fused<2>, dim3(count * 2, nq), kNttThreads, kExtSmem, st, (const uint32_t*)w.result,
+    // more ciphertexts than SMs: fewer transforms; else two SMs per ciphertext (k_ext_wide)
+    if ((long)count * nq > c->nsm)
+        launch(c, false, k_ext_wide<2>, dim3(count, nq), kExtWideThreads, kExtWideSmem, st, (const uint32_t*)w.result,
+               (const uint32_t*)c->keys0.rgsw, init, w.ext, coef_out, c->ntabs, c->gad.ext, batch_of(c, slot0));
+    else
+        launch(c, false, k_ext_fused<2>, dim3(count * 2, nq), kNttThreads, kExtSmem, st, (const uint32_t*)w.result,
            (const uint32_t*)c->keys0.rgsw, init, w.ext, coef_out, c->ntabs, c->gad.ext, batch_of(c, slot0));
 }
 
-// c2out (or null; split kernels only): receives each merge's X^I c + r, the
+// Whether a packing level of I merges runs on the split kernels (one transform
+// per CTA, latency) rather than whole merges per CTA pair (throughput): few
+// queries and few merges.  One query, us per level: I = 32 and 16 together 70 split, 45
+// fused; I <= 8: 12 to 16 split, 18 to 20 fused.  c2out only the split kernels write.
+bool pack_split(const kspir_ctx*, int nq, int I, const uint32_t* c2out) {
+    return c2out || (nq <= kPackSplitMaxBatch && nq * I < 16);
+}
+
+// c2out (or null): receives each merge's X^I c + r, the
 // words the reference's packingRLWEs leaves in rlwes[I + j]
 void enqueue_packing(kspir_ctx* c, int slot0, int nq, cudaStream_t st, uint32_t* c2out = nullptr) {
     const Workspace& w = c->ws0;
@@ -800,7 +813,7 @@ void enqueue_packing(kspir_ctx* c, int slot0, int nq, cudaStream_t st, uint32_t*
         const uint32_t ginv = inv_mod_2n((uint32_t)(kN / I + 1));
         uint32_t* out = (cur == w.ext) ? w.ext2 : w.ext;
         const uint32_t* key = c->keys0.packing + (size_t)lv * pe * 4 * kN;
-        if (nq <= kPackSplitMaxBatch) {   // latency: one transform per CTA
+        if (pack_split(c, nq, I, c2out)) {   // latency: one transform per CTA
             launch(c, true, k_pack_split_fwd<4>, dim3(I * 2 * 5, nq), kNttThreads, kPackSplitSmem, st, cur, w.pkpart, key, I,
                    ginv, c->ntabs, c->gad.pack, bt);
             launch(c, true, k_pack_split_inv<4>, dim3(I * 4, nq), kNttThreads, kPackSplitSmem, st, cur,
@@ -823,8 +836,9 @@ void enqueue_compose(kspir_ctx* c, int slot0, int nq, uint64_t* resp, int* err_o
 // kernels launched by one enqueue_answer
 long answer_launches(const kspir_ctx* c, int kind, int nq) {
     // baby 7 (and the transpose of a CUDA-core scan's), scan, giant 2, external product 1, packing one or two per level + compose
-    const int per_level = nq <= kPackSplitMaxBatch ? 2 : 1;
-    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + per_level * c->levels + 1;
+    long packing = 0;
+    for (int lv = 0; lv < c->levels; lv++) packing += pack_split(c, nq, 1 << lv, nullptr) ? 2 : 1;
+    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + packing + 1;
 }
 
 // Captures the four non-scan phases of (slot0, nq) as CUDA graphs (the scan
@@ -1288,6 +1302,7 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_ntt_jobs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNttJobSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_ntt_jobs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNttJobSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_giant_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGiantSmem));
+    KS_CUDA(c.get(), cudaFuncSetAttribute(k_ext_wide<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExtWideSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_ext_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExtSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_pack_fused<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPackSmem));
     KS_CUDA(c.get(), cudaFuncSetAttribute(k_pack_split_fwd<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPackSplitSmem));
