@@ -684,6 +684,8 @@ void enqueue_baby(kspir_ctx* c, int slot0, int nq, bool rm, cudaStream_t st) {
                (const uint32_t*)w.sout, w.cipherbuf, c->N1, bt);
 }
 
+int smallest_tile(int nq) { return nq > 16 ? SCAN_MMA32 : nq > 8 ? SCAN_MMA16 : nq > 4 ? SCAN_MMA8 : SCAN_MMA4; }
+
 int scan_kind_for(kspir_ctx* c, int nq) {
     if (!c->mma) return SCAN_CUDA;
     auto it = c->scan_choice.find(nq);
@@ -694,10 +696,23 @@ int scan_kind_for(kspir_ctx* c, int nq) {
     // n = 4: 221 (tile 4), 235 (8); n = 8: 244 (8), 275 (16); n = 13: 468 (8), 294
     // (16), 342 (32); n = 17: 690, 540, 358; n = 40: 1196, 846, 829; n = 64: 1895,
     // 1173, 879.  (At r = 2 tiles of 16 are 10 % faster for 33 to 48 queries.)
-    return nq > 16 ? SCAN_MMA32 : nq > 8 ? SCAN_MMA16 : nq > 4 ? SCAN_MMA8 : SCAN_MMA4;
+    return smallest_tile(nq);
 }
 
-long scan_launches(const kspir_ctx* c, int kind, int nq) { return kind == SCAN_CUDA ? nq : 2; }
+// With tiles of 32, the queries of a batch's last tile that run on a smaller tile
+// (0: none): up to 16 after at least one full tile.  Two tiles of 32
+// cost twice one whatever they hold; scan with its operand split, ms, one kind of
+// tile -> with the smaller last one: r = 16: n = 33: 0.80 -> 0.65, 40: 0.80 -> 0.68, 48:
+// 0.84 -> 0.74; r = 64, n = 40: 2.78 -> 2.28; r = 2, n = 40: 0.286 -> 0.246.  (A
+// tail after tiles of 16 or 8 gains nothing: their tiles cost nearly as much.)
+int scan_tail(int kind, int nq) {
+    const int rem = nq % 32;
+    return kind == SCAN_MMA32 && nq > 32 && rem <= 16 ? rem : 0;
+}
+
+long scan_launches(const kspir_ctx*, int kind, int nq) {
+    return kind == SCAN_CUDA ? nq : scan_tail(kind, nq) ? 4 : 2;
+}
 
 // Query-operand region of a launch starting at workspace slot slot0: 8 MiB per
 // slot, so launches on disjoint 32-aligned slot ranges (serving lanes) never
@@ -705,7 +720,7 @@ long scan_launches(const kspir_ctx* c, int kind, int nq) { return kind == SCAN_C
 uint8_t* qop_at(kspir_ctx* c, int slot0) { return c->qop + (size_t)slot0 * kN * 2 * 8 * kMmaK; }
 
 template <int BT>
-void launch_scan_mma(kspir_ctx* c, int slot0, int nq, cudaStream_t st) {
+void launch_scan_mma(kspir_ctx* c, int slot0, int nq, int* err, cudaStream_t st) {
     using C = MmaCfg<BT>;
     const int QT = (nq + BT - 1) / BT;
     uint8_t* qop = qop_at(c, slot0);
@@ -722,7 +737,7 @@ void launch_scan_mma(kspir_ctx* c, int slot0, int nq, cudaStream_t st) {
     a.QT = QT;
     a.G = c->G;
     a.rows = c->p.r * c->N2;
-    a.err = c->errs + (size_t)slot0 * kErrStride;
+    a.err = err;
     const int units = (kN / C::ZB) * 2 * QT;
     k_scan_mma<BT><<<std::min(c->nsm, units), C::THREADS, C::SMEM, st>>>(a);
 }
@@ -753,12 +768,18 @@ void enqueue_scan(kspir_ctx* c, int slot0, int nq, int kind, cudaStream_t st, bo
         }
         return;
     }
-    switch (scan_bt(kind)) {
-        case 4: launch_scan_mma<4>(c, slot0, nq, st); break;
-        case 8: launch_scan_mma<8>(c, slot0, nq, st); break;
-        case 16: launch_scan_mma<16>(c, slot0, nq, st); break;
-        default: launch_scan_mma<32>(c, slot0, nq, st); break;
-    }
+    int* err = c->errs + (size_t)slot0 * kErrStride;   // the batch's error word
+    auto tiles = [&](int kind, int slot, int n) {
+        switch (kind) {
+            case SCAN_MMA4: launch_scan_mma<4>(c, slot, n, err, st); break;
+            case SCAN_MMA8: launch_scan_mma<8>(c, slot, n, err, st); break;
+            case SCAN_MMA16: launch_scan_mma<16>(c, slot, n, err, st); break;
+            default: launch_scan_mma<32>(c, slot, n, err, st); break;
+        }
+    };
+    const int tail = scan_tail(kind, nq);
+    tiles(kind, slot0, nq - tail);
+    if (tail) tiles(smallest_tile(tail), slot0 + nq - tail, tail);
 }
 
 // The giant steps add into result (and, past kGiantTermsPerAcc steps per
