@@ -129,28 +129,46 @@ constexpr int kGiantSmem = kGiantPolys * kPadN * 4;
 
 // The key switch of output row `row` (= r N2 + c) into acc ([comp][prime][N] of
 // sub-database r), by 512 threads.  Each 256-thread group runs one prime: its
-// inverse transform of a, and, after both have met for the decomposition,
-// the transforms of the two digits (one set of twiddle loads for both) and
-// the key products.  Bounded by the multiply pipe and instruction issue (57 and
-// 54 % busy at 2 CTAs per SM; the six transforms alone take 0.75 of the 1.18 ms
-// of a batch of 64 at r = 16, which was 1.56 ms with conditional-subtraction
-// radix-8 transforms and 64-bit Barrett reductions).
+// inverse transform of a (read from global memory by the first pass), and, after
+// both have met for the decomposition, the transforms of the two digits (one
+// set of twiddle loads for both) and the key products.  X -> X^g keeps
+// coefficients u + 256 t in column u, the column that a thread's last inverse and
+// first forward pass hold, so the digits reach the transform in registers and only
+// the other prime's half crosses shared memory.  Bounded by issue, the multiply pipe
+// and shared-memory wavefronts together (each 55 to 60 % busy at 2 CTAs per SM;
+// without the decomposition, the b gather and the accumulation 0.99 ms remain of
+// 1.16).  Batch of 64 at r = 16: 1.56 ms with conditional-subtraction radix-8
+// transforms and 64-bit Barrett reductions, 1.18 ms with the digits written
+// twice to shared memory and read back, 1.16 ms; batch of 32 at r = 64: 2.37 -> 2.31.
 template <int ELL, class Sync>
 __device__ __forceinline__ void giant_body(uint32_t* P, const uint32_t* __restrict__ sout, uint32_t* acc,
                                            const uint32_t* __restrict__ gkeys, const uint16_t* __restrict__ gsigma,
                                            int N1, const NttTables& tabs, const GadgetB& g, int row, int c, int rows) {
-    static_assert(2 * ELL <= kGiantPolys, "shared-memory polynomials");
+    static_assert(ELL == 2 && 2 * ELL <= kGiantPolys, "shared-memory polynomials");
     const int ch = thread_group(), u = threadIdx.x & (kNttGroup - 1);
 
     // a of output[c] on this group's prime, to coefficient form
+    auto load_a = [&](int, uint32_t* x) {
 #pragma unroll
-    for (int k = u; k < kN / 4; k += kNttGroup)
-        *reinterpret_cast<uint4*>(P + ch * kPadN + pidx(4 * k)) =
-            __ldcg(reinterpret_cast<const uint4*>(sout + sout_idx(row, 0 * 2 + ch, 4 * k, rows)));
-    GroupSync::sync();
-    group_ntt_inverse<1, GroupSync>(P + ch * kPadN, kPadN, tabs, ch, u);
+        for (int v = 0; v < 2; v++) {
+            const uint32_t* src = sout + sout_idx(row, 0 * 2 + ch, 16 * u + 8 * v, rows);
+            if constexpr (std::is_same<Sync, CtaSync>::value) {
+                ldg_256(src, x + 8 * v);
+            } else {   // written by other CTAs of this launch: through L2
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                    const uint4 t = __ldcg(reinterpret_cast<const uint4*>(src + i));
+                    x[8 * v + i] = t.x; x[8 * v + i + 1] = t.y; x[8 * v + i + 2] = t.z; x[8 * v + i + 3] = t.w;
+                }
+            }
+        }
+    };
+    uint32_t* D = P + ch * ELL * kPadN;              // this group's polynomials
+    uint32_t* O = P + (1 - ch) * ELL * kPadN;        // the other's
+    auto keep = [&](int, int t, uint32_t v) { D[kPadN + pidx(u) + t * kPadGroupStep] = v; };
+    group_ntt_inverse<1, GroupSync>(D, kPadN, tabs, ch, u, keep, load_a);
     Sync::sync();
-    // X -> X^g, g = 5^(N1 c), then the digits (registers first: P is overwritten).
+    // X -> X^g, g = 5^(N1 c), then the digits of half of the coefficients in each group.
     // g = 1 mod 256 (N1 >= 64), so coefficient u + 256 t comes from u + 256 h with
     // h = (u g^-1 >> 8) + t g^-1 mod 32, negated when h >= 16.
     const uint32_t e = (uint32_t)(N1 * c) & 2047u;
@@ -158,25 +176,38 @@ __device__ __forceinline__ void giant_body(uint32_t* P, const uint32_t* __restri
     while (x) { if (x & 1) ginv = (ginv * b5) & (2 * kN - 1); b5 = (b5 * b5) & (2 * kN - 1); x >>= 1; }
     int32_t dres[kPerThreadG][ELL];
     uint32_t h = ((u * ginv) >> 8) + 8 * ch * ginv;
-    const uint32_t* Pu = P + pidx(u);
+    const uint32_t* Pu = P + kPadN + pidx(u);
 #pragma unroll
     for (int it = 0; it < kPerThreadG; it++) {   // coefficient u + 256 (8 ch + it)
         const uint32_t* src = Pu + (h & 15) * kPadGroupStep;
-        decompose_b_res<ELL>(src[0], src[kPadN], h & 16, g, dres[it]);
+        decompose_b_res<ELL>(src[0], src[ELL * kPadN], h & 16, g, dres[it]);
         h += ginv;
     }
+    // A digit is a small signed word, the same for both primes: each group hands its half
+    // to the other, column u to the thread that transforms column u, through the
+    // other's first polynomial (free since its inverse transform; this group's half of
+    // the second digit takes the places of the other's half of the first).  Only
+    // the two threads of column u touch it until the first pass has stored it.
+#pragma unroll
+    for (int it = 0; it < kPerThreadG; it++) {
+        O[pidx(u) + (8 * ch + it) * kPadGroupStep] = (uint32_t)dres[it][0];
+        O[pidx(u) + (8 * (1 - ch) + it) * kPadGroupStep] = (uint32_t)dres[it][1];
+    }
     Sync::sync();
-    // a digit is a small signed word, the same for both primes
+    uint32_t ex[ELL][kPerThreadG];
 #pragma unroll
-    for (int it = 0; it < kPerThreadG; it++)
+    for (int it = 0; it < kPerThreadG; it++) {
+        ex[0][it] = D[pidx(u) + (8 * (1 - ch) + it) * kPadGroupStep];
+        ex[1][it] = D[pidx(u) + (8 * ch + it) * kPadGroupStep];
+    }
+    auto digits = [&](int m, uint32_t* x) {
 #pragma unroll
-        for (int j = 0; j < ELL; j++)
-#pragma unroll
-            for (int p = 0; p < 2; p++)
-                P[(p * ELL + j) * kPadN + pidx(u) + (8 * ch + it) * kPadGroupStep] = (uint32_t)dres[it][j];
-    uint32_t* D = P + ch * ELL * kPadN;
-    Sync::sync();
-    group_ntt_forward<ELL, GroupSync, true>(D, kPadN, tabs, ch, u);   // signed, below 6.7 q
+        for (int it = 0; it < kPerThreadG; it++) {
+            x[it] = ch ? ex[m][it] : (uint32_t)dres[it][m];
+            x[8 + it] = ch ? (uint32_t)dres[it][m] : ex[m][it];
+        }
+    };
+    group_ntt_forward<ELL, GroupSync, true>(D, kPadN, tabs, ch, u, digits);   // signed, below 6.7 q
     const uint32_t q = c_dev.ch[ch].q;
     const uint4* key = reinterpret_cast<const uint4*>(gkeys + (size_t)(c - 1) * ELL * 4 * kN + (size_t)ch * kN);
     const uint16_t* sig = gsigma + (size_t)(c - 1) * kN;

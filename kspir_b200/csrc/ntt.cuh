@@ -250,14 +250,17 @@ __device__ __forceinline__ void inv_twiddles(const uint4* __restrict__ tab, int 
 // within +-q (signed words).  Ranges, in q, with B' = 1.03125 B + 1 per layer: 5.3 after
 // pass 0; the summands folded to 3: 7.7 after pass 1; folded to 2: 6.7 after
 // pass 2.  LAZY: the last pass leaves those signed words instead of canonical.
-template <int P, int M, bool LAZY>
-__device__ __forceinline__ void fwd_pass(uint32_t* s, int stride, const uint2* w, int ch, int u) {
+// The first pass takes its inputs from `in(m, x)` if there is one.
+struct NoSource {};
+template <int P, int M, bool LAZY, class In = NoSource>
+__device__ __forceinline__ void fwd_pass(uint32_t* s, int stride, const uint2* w, int ch, int u, const In& in = In()) {
     const ChanConst& cc = c_dev.ch[ch];
     uint32_t* b = s + unit_base<P>(u);
 #pragma unroll
     for (int m = 0; m < M; m++) {
         uint32_t x[16];
-        unit_load<P>(b + m * stride, x);
+        if constexpr (P == 0 && !std::is_same<In, NoSource>::value) in(m, x);
+        else unit_load<P>(b + m * stride, x);
         if (P > 0) {
 #pragma unroll
             for (int t = 0; t < 8; t++) x[t] = P == 1 ? fold6(x[t], cc.q) : fold8(x[t], cc.q);
@@ -274,9 +277,12 @@ __device__ __forceinline__ void fwd_pass(uint32_t* s, int stride, const uint2* w
 // One inverse pass, in the order P = 0 (contiguous), 1 (stride 16: inputs below
 // 5.2 q, the summands folded to 3, 7.7 q after it), 2 (stride 256; canonical
 // outputs, handed to `out(m, t, value)` if there is one, else stored in place).
+// The first pass takes its inputs, places 16 u .. 16 u + 15, from `in(m, x)` if there
+// is one.
 struct NoSink {};
-template <int P, int M, class Out = NoSink>
-__device__ __forceinline__ void inv_pass(uint32_t* s, int stride, const uint2* w, int ch, int u, const Out& out = Out()) {
+template <int P, int M, class Out = NoSink, class In = NoSource>
+__device__ __forceinline__ void inv_pass(uint32_t* s, int stride, const uint2* w, int ch, int u, const Out& out = Out(),
+                                         const In& in = In()) {
     const ChanConst& cc = c_dev.ch[ch];
     const uint32_t q = cc.q, nq = cc.nq;
     constexpr int F = 2 - P;   // the forward pass of the same strides
@@ -284,7 +290,8 @@ __device__ __forceinline__ void inv_pass(uint32_t* s, int stride, const uint2* w
 #pragma unroll
     for (int m = 0; m < M; m++) {
         uint32_t x[16];
-        unit_load<F>(b + m * stride, x);
+        if constexpr (P == 0 && !std::is_same<In, NoSource>::value) in(m, x);
+        else unit_load<F>(b + m * stride, x);
         if (P == 0) {
             unit_dft16<true>(x, cc);
         } else if (P == 1) {
@@ -312,12 +319,13 @@ __device__ __forceinline__ void inv_pass(uint32_t* s, int stride, const uint2* w
 // s + m * stride of channel ch.  The caller has synchronised their inputs; ends
 // with a barrier.  Each pass's twiddle loads are issued before the barrier
 // that precedes it.
-template <int M, class Sync, bool LAZY>
-__device__ __forceinline__ void group_ntt_forward(uint32_t* s, int stride, const NttTables& tabs, int ch, int u) {
+template <int M, class Sync, bool LAZY, class In = NoSource>
+__device__ __forceinline__ void group_ntt_forward(uint32_t* s, int stride, const NttTables& tabs, int ch, int u,
+                                                  const In& in = In()) {
     const uint4* tab = twiddle_table(tabs, ch, NTT_FWD);
     uint2 w[16];
     fwd_twiddles<0>(tab, ch, u, w);
-    if (M) fwd_pass<0, M, LAZY>(s, stride, w, ch, u);
+    if (M) fwd_pass<0, M, LAZY>(s, stride, w, ch, u, in);
     if (M) fwd_twiddles<1>(tab, ch, u, w);
     Sync::sync();
     if (M) fwd_pass<1, M, LAZY>(s, stride, w, ch, u);
@@ -329,12 +337,12 @@ __device__ __forceinline__ void group_ntt_forward(uint32_t* s, int stride, const
 
 // Inverse transforms by one group; canonical inputs (synchronised by the
 // caller) and outputs; ends with a barrier unless the outputs go to `out`.
-template <int M, class Sync, class Out = NoSink>
+template <int M, class Sync, class Out = NoSink, class In = NoSource>
 __device__ __forceinline__ void group_ntt_inverse(uint32_t* s, int stride, const NttTables& tabs, int ch, int u,
-                                                  const Out& out = Out()) {
+                                                  const Out& out = Out(), const In& in = In()) {
     const uint4* tab = twiddle_table(tabs, ch, NTT_INV);
     uint2 w[16];
-    if (M) inv_pass<0, M>(s, stride, w, ch, u);
+    if (M) inv_pass<0, M>(s, stride, w, ch, u, NoSink(), in);
     if (M) inv_twiddles<1>(tab, u, w);
     Sync::sync();
     if (M) inv_pass<1, M>(s, stride, w, ch, u);

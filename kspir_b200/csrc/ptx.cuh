@@ -91,6 +91,13 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst_smem, const void* src_gm
         : "memory");
 }
 
+// 32 bytes of read-only global memory, 32-byte aligned, without an L1 line
+__device__ __forceinline__ void ldg_256(const uint32_t* p, uint32_t* x) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7])
+                 : "l"(p));
+}
+
 // Programmatic dependent launch (sm_90+).  A kernel launched with the
 // programmatic-serialization attribute may start while the previous kernel in
 // its stream still runs: it does its independent prologue (staging
