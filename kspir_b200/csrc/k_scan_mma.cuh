@@ -128,6 +128,11 @@ __device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld_16x256b_x1(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -363,6 +368,217 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
     }
 }
 
+// The scan of one query on the tensor cores, for single answers that run beside
+// others: the same sums of the same operand tiles as k_scan_mma, streamed once at the
+// memory's rate by six warps that hardly use the issue slots and the multiply pipe,
+// which the key switches of the answers beside it need (the CUDA-core scan keeps
+// both busy: its time and theirs add up).  32 answers on eight streams at r =
+// 16: 225 us an answer beside CUDA-core scans, 202 with this one (189 to 203 for rings of
+// 3 to 6 tiles: beside a longer ring fewer key-switch CTAs fit, a shorter one is
+// slower where few answers overlap).  The memory traffic of an answer is 165 to 175 us.
+//
+// Query tile: 16 rows of two slots, n = 8 (z % 2) + 4 comp + lb, so the eight slots of
+// a unit are one 8 KiB copy (qop1[ch][z][4 comp + lb][128]) and every MMA (M = 128, N = 16)
+// reads a whole pair; of its 16 columns the eight of its own slot are used.  A
+// TMEM stage holds the eight slots of one row group.  In the 16x256b load shape a
+// thread gets the 4 x 2 products of one row, component and half of the query limbs
+// (columns 2 (t % 4), + 1): it folds them, swaps half of the slots with its
+// neighbour t ^ 1 and finishes four consecutive slots, one 16-byte store.
+struct Mma1Cfg {
+    static constexpr int N = 16;
+    static constexpr int ZB = 8;                          // NTT slots per unit
+    static constexpr int BUNIT = ZB * 8 * kMmaK;          // query operand of a unit
+    static constexpr int NB = 2;                          // units of it in flight
+    static constexpr int NA = 4;                          // database-tile ring
+    static constexpr int NTB = 2;                         // TMEM stages
+    static constexpr int TCOLS = NTB * ZB * N;            // 256
+    static constexpr int SMEM = 1024 + NB * BUNIT + NA * kATile + 256;
+    static constexpr int THREADS = 32 * 6;
+    static_assert((2 * NA + 2 * NB + 2 * NTB + 1) * 8 + 4 <= 256, "barriers");
+};
+
+__global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t* __restrict__ dbop,
+                                                                 const uint8_t* __restrict__ qop1,
+                                                                 uint32_t* __restrict__ sout, int G, int rows,
+                                                                 int* __restrict__ err) {
+    using C = Mma1Cfg;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* btiles = smem;                           // [NB][BUNIT]
+    uint8_t* atiles = smem + C::NB * C::BUNIT;        // [NA][kATile]
+    uint64_t* a_full = reinterpret_cast<uint64_t*>(atiles + C::NA * kATile);
+    uint64_t* a_empty = a_full + C::NA;
+    uint64_t* b_full = a_empty + C::NA;
+    uint64_t* b_empty = b_full + C::NB;
+    uint64_t* t_full = b_empty + C::NB;
+    uint64_t* t_empty = t_full + C::NTB;
+    uint64_t* done = t_empty + C::NTB;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < C::NA; s++) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
+        for (int s = 0; s < C::NB; s++) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
+        for (int s = 0; s < C::NTB; s++) { mbar_init(&t_full[s], 1); mbar_init(&t_empty[s], 4); }
+        mbar_init(done, 1);
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                     "n"(C::TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    constexpr int units = (kN / C::ZB) * 2;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint64_t pol_db = l2_policy_evict_first();
+            long ia = 0, ib = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ib++) {
+                const int ch = u & 1, z0 = (u >> 1) * C::ZB;
+                const int sb = (int)(ib % C::NB);
+                if (ib >= C::NB && !mbar_wait_bounded(&b_empty[sb], (uint32_t)((ib / C::NB - 1) & 1), kMmaWaitNs)) {
+                    atomicOr(err, 8);
+                    break;
+                }
+                mbar_arrive_expect_tx(&b_full[sb], C::BUNIT);
+                bulk_g2s(btiles + sb * C::BUNIT, qop1 + ((size_t)ch * kN + z0) * 8 * kMmaK, C::BUNIT, &b_full[sb]);
+                for (int g = 0; g < G && ok; g++)
+                    for (int zi = 0; zi < C::ZB; zi++) {
+                        const int sa = (int)(ia % C::NA);
+                        if (ia >= C::NA && !mbar_wait_bounded(&a_empty[sa], (uint32_t)((ia / C::NA - 1) & 1), kMmaWaitNs)) {
+                            atomicOr(err, 8);
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect_tx(&a_full[sa], kATile);
+                        bulk_g2s_hint(atiles + sa * kATile, dbop + (((size_t)(z0 + zi) * 2 + ch) * G + g) * kATile, kATile,
+                                      &a_full[sa], pol_db);
+                        ia++;
+                    }
+            }
+            // never leave with copies in flight into shared memory (ib counts the units
+            // whose query operand was asked for, but for one that was given up)
+            for (long j = ia > C::NA ? ia - C::NA : 0; j < ia; j++)
+                if (!mbar_wait_bounded(&a_full[j % C::NA], (uint32_t)((j / C::NA) & 1), kMmaWaitNs)) atomicOr(err, 16);
+            for (long j = ib > C::NB ? ib - C::NB : 0; j < ib; j++)
+                if (!mbar_wait_bounded(&b_full[j % C::NB], (uint32_t)((j / C::NB) & 1), kMmaWaitNs)) atomicOr(err, 16);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = mma_idesc_u8(C::N);
+            const uint32_t abase = smem_addr(atiles), bbase = smem_addr(btiles);
+            long ia = 0, ib = 0, tc = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ib++) {
+                const int sb = (int)(ib % C::NB);
+                if (!mbar_wait_bounded(&b_full[sb], (uint32_t)((ib / C::NB) & 1), kMmaWaitNs)) {
+                    atomicOr(err, 32);
+                    break;
+                }
+                for (int g = 0; g < G && ok; g++, tc++) {
+                    const int tb = (int)(tc % C::NTB);
+                    if (tc >= C::NTB && !mbar_wait_bounded(&t_empty[tb], (uint32_t)((tc / C::NTB - 1) & 1), kMmaWaitNs)) {
+                        atomicOr(err, 32);
+                        ok = false;
+                        break;
+                    }
+                    for (int zi = 0; zi < C::ZB; zi++, ia++) {
+                        const int sa = (int)(ia % C::NA);
+                        if (!mbar_wait_bounded(&a_full[sa], (uint32_t)((ia / C::NA) & 1), kMmaWaitNs)) {
+                            atomicOr(err, 32);
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint64_t ad = mma_sdesc_sw128(abase + sa * kATile);
+                        const uint64_t bd = mma_sdesc_sw128(bbase + sb * C::BUNIT + (zi >> 1) * C::N * kMmaK);
+#pragma unroll
+                        for (int kk = 0; kk < kMmaK / 32; kk++)
+                            mma_u8(tmem + (tb * C::ZB + zi) * C::N, ad + 2 * kk, bd + 2 * kk, idesc, kk > 0);
+                        mma_commit(&a_empty[sa]);
+                    }
+                    if (!ok) break;
+                    if (g == G - 1) mma_commit(&b_empty[sb]);
+                    mma_commit(&t_full[tb]);
+                }
+            }
+            mma_commit(done);
+            if (!mbar_wait_bounded(done, 0, kMmaWaitNs)) atomicOr(err, 64);
+        }
+    } else {
+        const int quarter = warp & 3;
+        const int half = lane & 1, comp = (lane >> 1) & 1;
+        const int jrow = 8 * quarter + (lane >> 2);   // database row within the 32-row tile
+        const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16);
+        long tc = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            const int ch = u & 1, z0 = (u >> 1) * C::ZB;
+            const uint32_t q = ch ? kQ2 : kQ1;
+            const uint32_t mu = ch ? (uint32_t)((1ull << 59) / kQ2) : (uint32_t)((1ull << 59) / kQ1);
+            const uint32_t c32 = ch ? (uint32_t)((1ull << 32) % kQ2) : (uint32_t)((1ull << 32) % kQ1);
+            for (int g = 0; g < G; g++, tc++) {
+                const int tb = (int)(tc % C::NTB);
+                // warp-uniform outcome: tcgen05.ld below needs the whole warp
+                const bool got = mbar_wait_bounded(&t_full[tb], (uint32_t)((tc / C::NTB) & 1), kMmaWaitNs);
+                if (!__all_sync(0xffffffffu, got)) {
+                    if (lane == 0) atomicOr(err, 128);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                uint64_t x[C::ZB];
+#pragma unroll
+                for (int z4 = 0; z4 < C::ZB; z4 += 4) {
+                    uint32_t L[4][4], H[4][4];   // limbs la 0, 1 and la 2, 3
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const uint32_t col = tq + (tb * C::ZB + z4 + i) * C::N + 8 * (i & 1);
+                        tmem_ld_16x256b_x1(col, L[i]);
+                        tmem_ld_16x256b_x1(col + (16u << 16), H[i]);
+                    }
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        // weights 1, 2^8 (below 2^32 together: limb products sum to at most
+                        // 128 * 255^2), 2^16, 2^24, 2^32 of limbs la + lb % 2
+                        uint64_t v = (uint64_t)H[i][3] << 32 | (L[i][0] + ((L[i][1] + L[i][2]) << 8));
+                        mad_wide(v, L[i][3] + H[i][0], 1u << 16);
+                        mad_wide(v, H[i][1] + H[i][2], 1u << 24);
+                        x[z4 + i] = half ? v << 16 : v;   // mod 2^64, as the reference's sums
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&t_empty[tb]);
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const uint64_t other = __shfl_xor_sync(0xffffffffu, half ? x[i] : x[4 + i], 1);
+                    o[i] = mod28((half ? x[4 + i] : x[i]) + other, q, c32, mu);
+                }
+                if (32 * g + jrow < rows)
+                    *reinterpret_cast<uint4*>(sout + sout_idx(32 * g + jrow, comp * 2 + ch, z0 + 4 * half, rows)) =
+                        make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(C::TCOLS));
+    }
+}
+
 // word lb of the 4 x 4 byte transpose of v[0..3]: bytes lb of the four words
 __device__ __forceinline__ void byte_transpose4(const uint32_t* v, uint32_t& l0, uint32_t& l1, uint32_t& l2, uint32_t& l3) {
     const uint32_t t0 = __byte_perm(v[0], v[1], 0x5140), t1 = __byte_perm(v[0], v[1], 0x7362);
@@ -392,7 +608,6 @@ constexpr int kSplitSmem = kMmaK * 4 * kSplitZ * 4;   // 64 KiB
 template <int BT>
 __global__ void __launch_bounds__(kSplitThreads) k_qop_split_rm(const uint32_t* __restrict__ cb0, size_t ws_bytes,
                                                                int slot0, int nq, int QT, uint8_t* __restrict__ qop) {
-    using C = MmaCfg<BT>;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint32_t* V = reinterpret_cast<uint32_t*>(smem_raw);   // [512 rows][32 columns]
     const int z0 = blockIdx.x * kSplitZ;
@@ -427,10 +642,11 @@ __global__ void __launch_bounds__(kSplitThreads) k_qop_split_rm(const uint32_t* 
             }
             byte_transpose4(v, w[0][g], w[1][g], w[2][g], w[3][g]);
         }
-        uint8_t* tile = qop + (((size_t)z * 2 + ch) * QT + qt) * C::BTILE;
+        // BT = 1 (k_scan_mma1): the rows of one slot, slots of a prime in order
+        uint8_t* tile = qop + (BT == 1 ? (size_t)ch * kN + z : ((size_t)z * 2 + ch) * QT + qt) * (8 * BT * kMmaK);
 #pragma unroll
         for (int lb = 0; lb < 4; lb++)
-            *reinterpret_cast<uint4*>(tile + sw128_off(mma_brow(comp * BT + b, lb), 16 * c)) =
+            *reinterpret_cast<uint4*>(tile + sw128_off(BT == 1 ? 4 * comp + lb : mma_brow(comp * BT + b, lb), 16 * c)) =
                 make_uint4(w[lb][0], w[lb][1], w[lb][2], w[lb][3]);
     }
 }

@@ -170,7 +170,8 @@ __global__ void k_unblock_sout(const uint32_t* __restrict__ sout, uint32_t* __re
 }
 
 // database-scan variants (chosen per batch size by kspir_tune_batch)
-enum ScanKind { SCAN_CUDA = 0, SCAN_MMA4 = 1, SCAN_MMA8 = 2, SCAN_MMA16 = 3, SCAN_MMA32 = 4, SCAN_KINDS = 5 };
+enum ScanKind { SCAN_CUDA = 0, SCAN_MMA4 = 1, SCAN_MMA8 = 2, SCAN_MMA16 = 3, SCAN_MMA32 = 4, SCAN_KINDS = 5,
+                SCAN_ONE = 5 };   // one query on the tensor cores (k_scan_mma1): chosen by enqueue_answer only
 int scan_bt(int kind) { return kind == SCAN_MMA4 ? 4 : kind == SCAN_MMA8 ? 8 : kind == SCAN_MMA16 ? 16 : 32; }
 
 }  // namespace
@@ -233,7 +234,7 @@ struct kspir_ctx {
     bool use_graphs = true;
     bool use_pdl = true;              // programmatic dependent launch inside the phases
     std::map<int, int> scan_choice;   // queries per launch -> ScanKind
-    int last_kind = 0;                // scan variant of the last answer launch
+    std::vector<char> slot_rm;        // the slot's last launch wrote its cipherbuf rotation-major (tensor-core scans)
     // events of recent launches: ring[i][0..5] brackets baby / scan / giant / ext / packing
     std::vector<std::array<cudaEvent_t, 6>> ring;
     std::vector<int> ring_nq;
@@ -769,6 +770,14 @@ void enqueue_scan(kspir_ctx* c, int slot0, int nq, int kind, cudaStream_t st, bo
         return;
     }
     int* err = c->errs + (size_t)slot0 * kErrStride;   // the batch's error word
+    if (kind == SCAN_ONE) {
+        const Workspace w = ws_host(c, slot0);
+        uint8_t* qop = qop_at(c, slot0);
+        k_qop_split_rm<1><<<dim3(kN / kSplitZ, 1), kSplitThreads, kSplitSmem, st>>>(
+            reinterpret_cast<const uint32_t*>(c->ws0.cipherbuf), c->ws_bytes, slot0, 1, 1, qop);
+        k_scan_mma1<<<c->scan_ctas, Mma1Cfg::THREADS, Mma1Cfg::SMEM, st>>>(c->dbop, qop, w.sout, c->G, R * c->N2, w.err);
+        return;
+    }
     auto tiles = [&](int kind, int slot, int n) {
         switch (kind) {
             case SCAN_MMA4: launch_scan_mma<4>(c, slot, n, err, st); break;
@@ -954,8 +963,21 @@ int enqueue_fused(kspir_ctx* c, int client, cudaStream_t st, int ring_slot) {
     return KSPIR_OK;
 }
 
+// Whether the scan of a single answer with `beside` others in flight runs on the
+// tensor cores (k_scan_mma1): from two others and two 32-row tiles on, unless
+// the caller chose a variant for n = 1 or an injected failure waits for a CUDA-core
+// scan.  us per answer, CUDA cores -> tensor cores: 32 answers on eight streams, r =
+// 16: 225 -> 202, r = 4: 73.6 -> 69.2; 4 answers, r = 16: 261 -> 250, r = 4: 113 -> 112;
+// 8 answers 226 -> 226 (217 with three others), 89 -> 86.  r = 2: 53 to 58 either
+// way, r = 1: 47 -> 50 (half of the tile is padding).
+constexpr int kOneMinBeside = 2, kOneMinRows = 64;
+bool one_on_tensor_cores(const kspir_ctx* c, int beside) {
+    return c->mma && beside >= kOneMinBeside && c->p.r * c->N2 >= kOneMinRows && !c->scan_choice.count(1) && c->scan_skip < 0;
+}
+
 // allow_fused: a single answer of slot 0 through the public single-answer
 // calls may run as the fused kernel (batches and serving lanes never do)
+// beside: single answers of other slots that may run beside this one
 // io: where the queries are read and the responses (and the first slot's error
 // word) written; by default the slots' device words
 struct AnswerIo {
@@ -965,11 +987,11 @@ struct AnswerIo {
 };
 
 int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStream_t st, bool allow_fused = false,
-                   bool share = false, AnswerIo io = AnswerIo()) {
+                   int beside = 0, AnswerIo io = AnswerIo()) {
     const int slot = (int)(c->enqueues % kTimingRing);
     auto& ev = c->ring[slot];
     if (allow_fused && c->fused && nq == 1 && slot0 == 0) {
-        c->last_kind = SCAN_CUDA;
+        c->slot_rm[0] = 0;
         cudaEventRecord(ev[0], st);
         int rc = enqueue_fused(c, clients[0], st, slot);
         if (rc) return rc;
@@ -985,8 +1007,9 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
     c->ring_fused[slot] = 0;
     if (!io.q) io.q = c->bq64 + (size_t)slot0 * 4 * kN;
     if (!io.resp) io.resp = c->bresp + (size_t)slot0 * 2 * kN;
-    const int kind = scan_kind_for(c, nq);
-    c->last_kind = kind;
+    int kind = scan_kind_for(c, nq);
+    if (nq == 1 && one_on_tensor_cores(c, beside)) kind = SCAN_ONE;
+    std::fill_n(c->slot_rm.begin() + slot0, nq, (char)(kind != SCAN_CUDA));
     if (c->use_graphs) {
         kspir_ctx::PhaseGraphs* pg = nullptr;
         int rc = build_graphs(c, slot0, nq, kind != SCAN_CUDA, &pg);
@@ -995,7 +1018,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         enqueue_prep(c, slot0, nq, clients, io.q, st);
         KS_CUDA(c, cudaGraphLaunch(pg->g[0], st));
         cudaEventRecord(ev[1], st);
-        enqueue_scan(c, slot0, nq, kind, st, share);
+        enqueue_scan(c, slot0, nq, kind, st, beside > 0);
         cudaEventRecord(ev[2], st);
         KS_CUDA(c, cudaGraphLaunch(pg->g[1], st));
         cudaEventRecord(ev[3], st);
@@ -1009,7 +1032,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         enqueue_prep(c, slot0, nq, clients, io.q, st);
         enqueue_baby(c, slot0, nq, kind != SCAN_CUDA, st);
         cudaEventRecord(ev[1], st);
-        enqueue_scan(c, slot0, nq, kind, st, share);
+        enqueue_scan(c, slot0, nq, kind, st, beside > 0);
         cudaEventRecord(ev[2], st);
         enqueue_giant(c, slot0, nq, st);
         cudaEventRecord(ev[3], st);
@@ -1123,16 +1146,18 @@ struct SlotHold {
     }
 };
 
-// Whether a single answer in another slot, on another stream, may still be
-// running when this one (slot `self`, stream `st`) starts: then the scan takes
-// the sharing ring shape.  Answers on the same stream run one after another
+// How many single answers in other slots, on other streams, may still be running
+// when this one (slot `self`, stream `st`) starts: beside one, the CUDA-core scan takes
+// the sharing ring shape; beside more, the scan may run on the tensor cores
+// (one_on_tensor_cores).  Answers on the same stream run one after another
 // and keep the streaming shape.
-bool singles_beside(kspir_ctx* c, int self, cudaStream_t st) {
+int singles_beside(kspir_ctx* c, int self, cudaStream_t st) {
+    int n = 0;
     for (int i = 0; i < c->single_slots; i++) {
         if (i == self || !c->slot_used[i] || c->slot_last_stream[i] == st) continue;
-        if (c->slot_busy[i] || cudaEventQuery(c->slot_done[i]) == cudaErrorNotReady) return true;
+        if (c->slot_busy[i] || cudaEventQuery(c->slot_done[i]) == cudaErrorNotReady) n++;
     }
-    return false;
+    return n;
 }
 
 // the tensor-core database operand, rebuilt from the resident database
@@ -1339,6 +1364,8 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
 #undef KS_ATTR
     int rc = KSPIR_OK;
     if (c->mma) {
+        KS_CUDA(c.get(), cudaFuncSetAttribute(k_qop_split_rm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem));
+        KS_CUDA(c.get(), cudaFuncSetAttribute(k_scan_mma1, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma1Cfg::SMEM));
         if (!rc) rc = mma_attr<4>(c.get());
         if (!rc) rc = mma_attr<8>(c.get());
         if (!rc) rc = mma_attr<16>(c.get());
@@ -1350,6 +1377,7 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     rc = init_constants(c.get());
     if (rc) return rc;
     KS_CUDA(c.get(), cudaMalloc(&c->perms, (size_t)p.N1 * kN * 2));
+    c->slot_rm.assign(p.max_inflight, 0);
     c->ring.resize(kTimingRing);
     c->ring_nq.assign(kTimingRing, 0);
     for (auto& evs : c->ring)
@@ -2204,10 +2232,10 @@ int kspir_answer_device(kspir_ctx* c, int client, const uint64_t* d_query, uint6
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     KS_CUDA(c, cudaSetDevice(c->device));
     const int slot = pick_slot(c, lk, false);
-    const bool share = singles_beside(c, slot, st);
+    const int beside = singles_beside(c, slot, st);
     if (c->slot_used[slot]) KS_CUDA(c, cudaStreamWaitEvent(st, c->slot_done[slot], 0));
     KS_CUDA(c, cudaMemcpyAsync(c->bq64 + (size_t)slot * 4 * kN, d_query, 4 * kN * 8, cudaMemcpyDeviceToDevice, st));
-    rc = enqueue_answer(c, slot, 1, &client, st, true, share);
+    rc = enqueue_answer(c, slot, 1, &client, st, true, beside);
     if (rc) return rc;
     KS_CUDA(c, cudaMemcpyAsync(d_response, c->bresp + (size_t)slot * 2 * kN, 2 * kN * 8, cudaMemcpyDeviceToDevice, st));
     KS_CUDA(c, cudaEventRecord(c->slot_done[slot], st));
@@ -2249,11 +2277,11 @@ int kspir_answer(kspir_ctx* c, int client, const uint64_t* query, uint64_t* resp
     lk.unlock();
     memcpy(hq, query, 4 * kN * 8);
     lk.lock();
-    const bool share = singles_beside(c, slot, st);
+    const int beside = singles_beside(c, slot, st);
     if (c->slot_used[slot]) KS_CUDA(c, cudaStreamWaitEvent(st, c->slot_done[slot], 0));
     if (c->fused) {
         KS_CUDA(c, cudaMemcpyAsync(c->bq64 + (size_t)slot * 4 * kN, hq, 4 * kN * 8, cudaMemcpyHostToDevice, st));
-        rc = enqueue_answer(c, slot, 1, &client, st, true, share);
+        rc = enqueue_answer(c, slot, 1, &client, st, true, beside);
         if (rc) return rc;
         KS_CUDA(c, cudaMemcpyAsync(hr, c->bresp + (size_t)slot * 2 * kN, 2 * kN * 8, cudaMemcpyDeviceToHost, st));
         KS_CUDA(c, cudaMemcpyAsync(c->single_errs + slot, c->errs + (size_t)slot * kErrStride, 4,
@@ -2263,7 +2291,7 @@ int kspir_answer(kspir_ctx* c, int client, const uint64_t* query, uint64_t* resp
         io.q = hq;
         io.resp = hr;
         io.err = c->single_errs + slot;
-        rc = enqueue_answer(c, slot, 1, &client, st, false, share, io);
+        rc = enqueue_answer(c, slot, 1, &client, st, false, beside, io);
         if (rc) return rc;
     }
     KS_CUDA(c, cudaGetLastError());
@@ -2483,6 +2511,7 @@ int kspir_matrix_vector_mul_bsgs_rns_crt_large(kspir_ctx* c, int client, uint64_
     if (int wrc = wait_singles(c, c->stream)) return wrc;
     KS_CUDA(c, cudaMemcpyAsync(c->bq64, query_inout, 4 * kN * 8, cudaMemcpyHostToDevice, st));
     enqueue_prep(c, 0, 1, &client, c->bq64, st);
+    c->slot_rm[0] = 0;
     enqueue_baby(c, 0, 1, false, st);
     enqueue_scan(c, 0, 1, SCAN_CUDA, st);
     enqueue_giant(c, 0, 1, st);
@@ -2591,7 +2620,7 @@ int kspir_fetch_stage_slot(kspir_ctx* c, int slot, int stage, uint64_t* out, siz
         const size_t n = (size_t)kN * c->N1 * 2;
         if (words != n) return set_err(c, KSPIR_ERR_INVALID_ARG, "size mismatch");
         KS_COPY(c, out, w.cipherbuf, n * 8, cudaMemcpyDeviceToHost);
-        if (c->last_kind != SCAN_CUDA) {
+        if (c->slot_rm[slot]) {
             // the tensor-core scans' launches write it rotation-major: back to [N][N1][2]
             std::vector<uint32_t> rm(2 * n);
             memcpy(rm.data(), out, n * 8);
