@@ -43,7 +43,12 @@
 // at r = 16, with the operand split: 0.98 ms with every warp on every tile and
 // per-store 64-bit addresses, 0.89 ms with TMEM addresses in uniform registers
 // and linear store addresses, 0.85 ms with the two sets; batch of 32 at r = 64:
-// 1.65, 1.52, 1.43 ms.  Every wait is bounded; on a timeout
+// 1.65, 1.52, 1.43 ms.  The threads that issue copies and MMAs count ring stages
+// and laps in 32 bits (a 64-bit tile count modulo the ring's length cost more
+// than the copy it addressed), and a TMEM stage holds up to four slots of a row group, so
+// that small tiles hand over once for four: r = 16 with the operand split, batch of 4:
+// 0.221 -> 0.208 ms, 8: 0.244 -> 0.230, 13: 0.292 -> 0.281, 64: 0.85 -> 0.83; r = 64, batch of 4:
+// 0.80 -> 0.71, 8: 0.87 -> 0.77.  Every wait is bounded; on a timeout
 // the warp sets the error word and leaves its loop, the producer waits for its
 // own copies in flight, the MMA lane for its own MMAs, and TMEM is freed.
 #pragma once
@@ -71,21 +76,22 @@ struct MmaCfg {
     static constexpr int N = 8 * BT;                  // MMA N = TMEM columns per accumulator
     static constexpr int ZB = BT == 32 ? 4 : 8;       // NTT slots per unit
     static constexpr int BTILE = N * kMmaK;
-    static constexpr int NTB = N >= 256 ? 2 : 4;      // TMEM accumulators (512 columns allocated)
+    static constexpr int TPS = N >= 256 ? 1 : N >= 128 ? 2 : 4;   // tiles (slots of one row group) per TMEM stage
+    static constexpr int NTB = N >= 64 ? 2 : 4;       // TMEM stages (512 columns allocated)
     static constexpr int BAR_BYTES = 512;
     static constexpr int NA_FIT = (kMmaSmemLimit - 1024 - BAR_BYTES - ZB * BTILE) / kATile;
     static constexpr int NA = NA_FIT < 6 ? NA_FIT : 6;  // database-tile ring
     static constexpr int SMEM = 1024 + ZB * BTILE + NA * kATile + BAR_BYTES;
     static constexpr int CHUNKS = N / 16;             // 16-column chunks = 4 query groups each
     static constexpr int SETS = 2;                    // sets of epilogue warps: set s takes the row groups g % SETS = s
-    static constexpr int NTS = NTB / SETS;            // TMEM accumulators per set
+    static constexpr int NTS = NTB / SETS;            // TMEM stages per set
     static constexpr int PARTS = 2;                   // epilogue warps per TMEM quarter and set
     static constexpr int CPW = CHUNKS / PARTS;        // chunks (outputs per lane) per epilogue warp
-    static constexpr int LDB = CPW < 2 ? CPW : 2;     // outputs whose TMEM loads share one wait
+    static constexpr int LDB = TPS * CPW < 2 ? TPS * CPW : 2;   // outputs whose TMEM loads share one wait
     static constexpr int EPI = 4 * PARTS * SETS;      // epilogue warps
     static constexpr int THREADS = 32 * (2 + EPI);
     static_assert(NA >= 2 && SMEM <= kMmaSmemLimit, "shared memory budget");
-    static_assert(NTB * N <= 512, "TMEM columns");
+    static_assert(NTB * TPS * N <= 512 && ZB % TPS == 0 && TPS * CPW % LDB == 0, "TMEM columns");
     static_assert(4 * CPW <= BT, "an epilogue warp's chunks belong to one component");
 };
 
@@ -188,7 +194,8 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
     if (warp == 0) {
         // producer
         if (lane == 0) {
-            long ia = 0;
+            int sa = 0, na = 0;      // ring stage and lap parity, tiles asked for (up to NA)
+            uint32_t pa = 0;
             int tu = 0;
             int bl[C::ZB];   // query-tile copies issued per slot
             for (int zi = 0; zi < C::ZB; zi++) bl[zi] = 0;
@@ -209,20 +216,23 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                             bl[zi]++;
                         }
                         for (int g = gp; g < gp + C::SETS && g < G; g++) {
-                            const int sa = (int)(ia % C::NA);
-                            if (ia >= C::NA && !mbar_wait_bounded(&a_empty[sa], (uint32_t)((ia / C::NA - 1) & 1), kMmaWaitNs)) {
+                            // (the parity before the first lap counts as complete)
+                            if (!mbar_wait_bounded(&a_empty[sa], pa ^ 1, kMmaWaitNs)) {
                                 atomicOr(a.err, 8); ok = false; break;
                             }
                             mbar_arrive_expect_tx(&a_full[sa], kATile);
                             bulk_g2s(atiles + sa * kATile, a.dbop + (((size_t)z * 2 + ch) * G + g) * kATile, kATile,
                                      &a_full[sa]);
-                            ia++;
+                            if (na < C::NA) na++;
+                            if (++sa == C::NA) { sa = 0; pa ^= 1; }
                         }
                     }
             }
-            // never leave with copies in flight into shared memory
-            for (long j = ia > C::NA ? ia - C::NA : 0; j < ia; j++)
-                if (!mbar_wait_bounded(&a_full[j % C::NA], (uint32_t)((j / C::NA) & 1), kMmaWaitNs)) atomicOr(a.err, 16);
+            // never leave with copies in flight into shared memory: the last lap's
+            for (; na > 0; na--) {
+                if (sa == 0) { sa = C::NA; pa ^= 1; }
+                if (!mbar_wait_bounded(&a_full[--sa], pa, kMmaWaitNs)) atomicOr(a.err, 16);
+            }
             for (int zi = 0; zi < C::ZB; zi++)
                 if (bl[zi] > 0 && !mbar_wait_bounded(&b_full[zi], (uint32_t)((bl[zi] - 1) & 1), kMmaWaitNs))
                     atomicOr(a.err, 16);
@@ -232,8 +242,8 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
         if (lane == 0) {
             const uint32_t idesc = mma_idesc_u8(C::N);
             const uint32_t abase = smem_addr(atiles), bbase = smem_addr(btiles);
-            long ia = 0, tc[C::SETS] = {};
-            int tu = 0;
+            int sa = 0, tu = 0;
+            uint32_t pa = 0, tc[C::SETS] = {};
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, tu++) {
                 for (int gp = 0; gp < G && ok; gp += C::SETS)
@@ -245,13 +255,12 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                         for (int s = 0; s < C::SETS; s++) {
                             const int g = gp + s;
                             if (g >= G || !ok) break;
-                            const int sa = (int)(ia % C::NA);
-                            if (!mbar_wait_bounded(&a_full[sa], (uint32_t)((ia / C::NA) & 1), kMmaWaitNs)) {
+                            if (!mbar_wait_bounded(&a_full[sa], pa, kMmaWaitNs)) {
                                 atomicOr(a.err, 32); ok = false; break;
                             }
                             const int tb = s + C::SETS * (int)(tc[s] % C::NTS);
-                            if (tc[s] >= C::NTS &&
-                                !mbar_wait_bounded(&t_empty[tb], (uint32_t)((tc[s] / C::NTS - 1) & 1), kMmaWaitNs)) {
+                            if (zi % C::TPS == 0 && tc[s] >= C::NTS &&
+                                !mbar_wait_bounded(&t_empty[tb], (tc[s] / C::NTS - 1) & 1, kMmaWaitNs)) {
                                 atomicOr(a.err, 32); ok = false; break;
                             }
                             tc_fence_after();
@@ -259,12 +268,14 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                             const uint64_t bd = mma_sdesc_sw128(bbase + zi * C::BTILE);
 #pragma unroll
                             for (int kk = 0; kk < kMmaK / 32; kk++)
-                                mma_u8(tmem + tb * C::N, ad + 2 * kk, bd + 2 * kk, idesc, kk > 0);
+                                mma_u8(tmem + (tb * C::TPS + zi % C::TPS) * C::N, ad + 2 * kk, bd + 2 * kk, idesc, kk > 0);
                             mma_commit(&a_empty[sa]);
                             if (g == G - 1) mma_commit(&b_empty[zi]);
-                            mma_commit(&t_full[tb]);
-                            ia++;
-                            tc[s]++;
+                            if (++sa == C::NA) { sa = 0; pa ^= 1; }
+                            if (zi % C::TPS == C::TPS - 1) {
+                                mma_commit(&t_full[tb]);
+                                tc[s]++;
+                            }
                         }
                     }
             }
@@ -278,7 +289,7 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
         const int j3 = lane >> 2, gq = lane & 3;
         const int jrow = 8 * quarter + j3;   // database row within the 32-row tile
         const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16) + part * C::CPW * 16;
-        long tc = 0;
+        uint32_t tc = 0;
         bool ok = true;
         uint32_t ob[C::ZB][C::CPW];
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
@@ -295,10 +306,10 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                        (size_t)(a.slot0 + bq0) * a.ws_bytes;
             for (int g = set; g < G && ok; g += C::SETS, so += sout_idx(32 * C::SETS, 0, 0, 0) * 4) {
 #pragma unroll
-                for (int zi = 0; zi < C::ZB; zi++) {
+                for (int zi = 0; zi < C::ZB; zi += C::TPS) {
                     const int tb = set + C::SETS * (int)(tc % C::NTS);
                     // warp-uniform outcome: tcgen05.ld below needs the whole warp
-                    const bool got = mbar_wait_bounded(&t_full[tb], (uint32_t)((tc / C::NTS) & 1), kMmaWaitNs);
+                    const bool got = mbar_wait_bounded(&t_full[tb], (tc / C::NTS) & 1, kMmaWaitNs);
                     if (!__all_sync(0xffffffffu, got)) {
                         if (lane == 0) atomicOr(a.err, 128);
                         ok = false;
@@ -306,12 +317,13 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                     }
                     tc_fence_after();
 #pragma unroll
-                    for (int c0 = 0; c0 < C::CPW; c0 += C::LDB) {
-                        // LDB outputs per wait: their loads overlap
+                    for (int e0 = 0; e0 < C::TPS * C::CPW; e0 += C::LDB) {
+                        // LDB outputs (slot e / CPW, chunk e % CPW) per wait: their loads overlap
                         uint32_t lo[C::LDB][8], hi[C::LDB][8];   // limbs la 0,1 and la 2,3
 #pragma unroll
                         for (int c1 = 0; c1 < C::LDB; c1++) {
-                            const uint32_t col = tq + tb * C::N + (c0 + c1) * 16;
+                            const int e = e0 + c1;
+                            const uint32_t col = tq + (tb * C::TPS + e / C::CPW) * C::N + e % C::CPW * 16;
                             tmem_ld_16x256b_x2(col, lo[c1]);
                             tmem_ld_16x256b_x2(col + (16u << 16), hi[c1]);
                         }
@@ -332,7 +344,7 @@ __global__ void __launch_bounds__(MmaCfg<BT>::THREADS, 1) k_scan_mma(ScanMmaArgs
                             uint64_t x = (uint64_t)xh << 32 | xl;
                             mad_wide(x, t2, 1u << 16);
                             mad_wide(x, t3, 1u << 24);
-                            ob[zi][c0 + c1] = mod28(x, q, c32, mu);
+                            ob[zi + (e0 + c1) / C::CPW][(e0 + c1) % C::CPW] = mod28(x, q, c32, mu);
                         }
                     }
                     tc_fence_before();
@@ -437,7 +449,7 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
     if (warp == 0) {
         if (lane == 0) {
             const uint64_t pol_db = l2_policy_evict_first();
-            long ia = 0, ib = 0;
+            uint32_t ia = 0, ib = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ib++) {
                 const int ch = u & 1, z0 = (u >> 1) * C::ZB;
@@ -464,16 +476,16 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
             }
             // never leave with copies in flight into shared memory (ib counts the units
             // whose query operand was asked for, but for one that was given up)
-            for (long j = ia > C::NA ? ia - C::NA : 0; j < ia; j++)
+            for (uint32_t j = ia > C::NA ? ia - C::NA : 0; j < ia; j++)
                 if (!mbar_wait_bounded(&a_full[j % C::NA], (uint32_t)((j / C::NA) & 1), kMmaWaitNs)) atomicOr(err, 16);
-            for (long j = ib > C::NB ? ib - C::NB : 0; j < ib; j++)
+            for (uint32_t j = ib > C::NB ? ib - C::NB : 0; j < ib; j++)
                 if (!mbar_wait_bounded(&b_full[j % C::NB], (uint32_t)((j / C::NB) & 1), kMmaWaitNs)) atomicOr(err, 16);
         }
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = mma_idesc_u8(C::N);
             const uint32_t abase = smem_addr(atiles), bbase = smem_addr(btiles);
-            long ia = 0, ib = 0, tc = 0;
+            uint32_t ia = 0, ib = 0, tc = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ib++) {
                 const int sb = (int)(ib % C::NB);
@@ -516,7 +528,7 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
         const int half = lane & 1, comp = (lane >> 1) & 1;
         const int jrow = 8 * quarter + (lane >> 2);   // database row within the 32-row tile
         const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16);
-        long tc = 0;
+        uint32_t tc = 0;
         bool ok = true;
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             const int ch = u & 1, z0 = (u >> 1) * C::ZB;

@@ -694,16 +694,16 @@ int scan_kind_for(kspir_ctx* c, int nq) {
     if (nq == 1) return SCAN_CUDA;
     // the smallest query tile that holds the batch in one pass over the database,
     // else the largest (fewest passes); r = 16, scan with its operand split, us:
-    // n = 4: 221 (tile 4), 235 (8); n = 8: 244 (8), 275 (16); n = 13: 468 (8), 294
-    // (16), 342 (32); n = 17: 690, 540, 358; n = 40: 1196, 846, 829; n = 64: 1895,
-    // 1173, 879.  (At r = 2 tiles of 16 are 10 % faster for 33 to 48 queries.)
+    // n = 4: 208 (tile 4), 217 (8); n = 8: 230 (8), 260 (16); n = 13: 400 (8), 281
+    // (16), 330 (32); n = 40: 1004, 770, 656 (with the smaller last tile of
+    // scan_tail); n = 64: 1630, 1084, 838.
     return smallest_tile(nq);
 }
 
 // With tiles of 32, the queries of a batch's last tile that run on a smaller tile
 // (0: none): up to 16 after at least one full tile.  Two tiles of 32
 // cost twice one whatever they hold; scan with its operand split, ms, one kind of
-// tile -> with the smaller last one: r = 16: n = 33: 0.80 -> 0.65, 40: 0.80 -> 0.68, 48:
+// tile -> with the smaller last one: r = 16: n = 33: 0.80 -> 0.65, 40: 0.80 -> 0.66, 48:
 // 0.84 -> 0.74; r = 64, n = 40: 2.78 -> 2.28; r = 2, n = 40: 0.286 -> 0.246.  (A
 // tail after tiles of 16 or 8 gains nothing: their tiles cost nearly as much.)
 int scan_tail(int kind, int nq) {
