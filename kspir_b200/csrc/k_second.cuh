@@ -116,8 +116,8 @@ namespace kspir {
 //   INTT(a) per prime -> compose -> X -> X^g -> decompose (ell digits)
 //   -> digit transforms -> -sum_j d_j * key[j]  and  b[sigma_g] - sum_j d_j * key[j]
 // and adds both, canonical, into the sub-database's accumulator (u32 words
-// in L2; the scan output is only read).  k_giant_finish then adds output[0]
-// and reduces.  A u32 word holds at most kGiantTermsPerAcc terms below
+// in L2; the scan output is only read).  k_giant_finish, or the external product
+// itself, then adds output[0] and reduces (giant_sum4).  A u32 word holds at most kGiantTermsPerAcc terms below
 // q1 (16 (q1 - 1) < 2^32); with more giant steps per sub-database (N1 = 64:
 // 31) rows c odd go to acc0 and rows c even to acc1.
 constexpr int kGiantTermsPerAcc = 16;
@@ -246,30 +246,63 @@ __global__ void __launch_bounds__(kNttThreads, 2)
                              shifted(gkeys, key_off(bt)), gsigma, N1, tabs, g, r * N2 + c, c, R * N2);
 }
 
-// result[r][comp][ch][k] = (output[0] + the giant-step accumulators) mod q,
-// in place over acc0 (= result).  One thread per four consecutive slots.
-__global__ void k_giant_finish(const uint32_t* __restrict__ sout, uint32_t* result, const uint32_t* acc1, int R,
-                               int N2, Batch bt) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long)R * 4 * (kN / 4)) return;
-    sout = shifted(sout, ws_off(bt));
-    result = shifted(result, ws_off(bt));
-    const int z = (int)(idx % (kN / 4)) * 4;
-    const int cc_ = (int)((idx / (kN / 4)) % 4);      // comp * 2 + ch
-    const int r = (int)(idx / (4 * (kN / 4)));
-    const ChanConst q = c_dev.ch[cc_ & 1];
-    uint4* res = reinterpret_cast<uint4*>(result + ((size_t)r * 4 + cc_) * kN + z);
-    const uint4 a = __ldcg(res);
-    const uint4 w = __ldcg(reinterpret_cast<const uint4*>(sout + sout_idx(r * N2, cc_, z, R * N2)));
+// Where the external product finds output[0] and the second accumulator of its
+// first-dimension results (slot-0 addresses).  sout null: the residues given are
+// final.
+struct GiantSums {
+    const uint32_t* sout;
+    const uint32_t* acc1;   // or null
+    int N2, rows;           // rows = R N2
+};
+
+// (output[0] + the giant-step accumulators) mod q of slots z .. z + 3, polynomial cv =
+// comp * 2 + prime of sub-database r; fd points at the polynomial of the accumulator
+// acc0, wo is the query's workspace offset
+__device__ __forceinline__ uint4 giant_sum4(const GiantSums& g, size_t wo, const uint32_t* fd, int r, int cv, int z) {
+    const ChanConst& q = c_dev.ch[cv & 1];
+    const uint4 a = __ldcg(reinterpret_cast<const uint4*>(fd + z));
+    const uint4 w = __ldcg(reinterpret_cast<const uint4*>(shifted(g.sout, wo) + sout_idx(r * g.N2, cv, z, g.rows)));
     uint64_t v0 = (uint64_t)a.x + w.x, v1 = (uint64_t)a.y + w.y, v2 = (uint64_t)a.z + w.z, v3 = (uint64_t)a.w + w.w;
-    if (acc1) {
-        const uint4 b = __ldcg(reinterpret_cast<const uint4*>(shifted(acc1, ws_off(bt)) + ((size_t)r * 4 + cc_) * kN + z));
+    if (g.acc1) {
+        const uint4 b = __ldcg(reinterpret_cast<const uint4*>(shifted(g.acc1, wo) + ((size_t)r * 4 + cv) * kN + z));
         v0 += b.x; v1 += b.y; v2 += b.z; v3 += b.w;
     }
-    *res = make_uint4(reduce64(v0, q.q, q.barrett), reduce64(v1, q.q, q.barrett), reduce64(v2, q.q, q.barrett),
+    return make_uint4(reduce64(v0, q.q, q.barrett), reduce64(v1, q.q, q.barrett), reduce64(v2, q.q, q.barrett),
                       reduce64(v3, q.q, q.barrett));
+}
+
+// The first-dimension results [r][comp][ch][k] from their accumulators acc0, in place
+// or (one query) into out, for the external products that do not add it up themselves
+// (first_dim_to_smem), the staged calls and diagnostics.  One thread per four
+// consecutive slots.
+__global__ void k_giant_finish(GiantSums g, uint32_t* acc0, uint32_t* out, int R, Batch bt) {
+    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long)R * 4 * (kN / 4)) return;
+    const size_t wo = ws_off(bt);
+    const int z = (int)(idx % (kN / 4)) * 4;
+    const int cv = (int)((idx / (kN / 4)) % 4);
+    const int r = (int)(idx / (4 * (kN / 4)));
+    const size_t at = ((size_t)r * 4 + cv) * kN;
+    acc0 = shifted(acc0, wo);
+    *reinterpret_cast<uint4*>((out ? out : acc0) + at + z) = giant_sum4(g, wo, acc0 + at, r, cv, z);
+}
+
+// Polynomial cv of first-dimension result r (at fd) into shared memory, by T threads.
+// With the sums here instead of in k_giant_finish, which writes every result once
+// more to be read back: batch of 64 at r = 16 3.484 -> 3.447 ms, of 32 at r = 64
+// 5.648 -> 5.582 ms.  Where a CTA per prime reads all of first_dim (k_ext_fused) the
+// longer load costs what the launch did (r = 1: 168.9 -> 170.2 us, r = 16: 383.9 ->
+// 383.0), so that one keeps the kernel.
+template <int T = kNttThreads>
+__device__ __forceinline__ void first_dim_to_smem(uint32_t* s, const uint32_t* fd, const GiantSums& g, size_t wo, int r,
+                                                  int cv) {
+    if (!g.sout) {
+        poly_to_smem<T>(s, fd);
+        return;
+    }
+#pragma unroll
+    for (int k = threadIdx.x % T; k < kN / 4; k += T)
+        *reinterpret_cast<uint4*>(s + pidx(4 * k)) = giant_sum4(g, wo, fd, r, cv, 4 * k);
 }
 
 }  // namespace kspir
@@ -643,8 +676,8 @@ constexpr int kExtWideSmem = 8 * kPadN * 4;   // two primes x four digits
 
 template <int ELL>
 __global__ void __launch_bounds__(kExtWideThreads, 1)
-    k_ext_wide(const uint32_t* __restrict__ first_dim, const uint32_t* __restrict__ rgsw, const uint32_t* __restrict__ init,
-               uint32_t* __restrict__ ext, uint32_t* __restrict__ coef_out, NttTables tabs, GadgetS g, Batch bt) {
+    k_ext_wide(const uint32_t* __restrict__ first_dim, GiantSums sums, const uint32_t* __restrict__ rgsw,
+               const uint32_t* __restrict__ init, uint32_t* __restrict__ ext, uint32_t* __restrict__ coef_out, NttTables tabs, GadgetS g, Batch bt) {
     static_assert(ELL == 2, "four digits, two per group and prime");
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint32_t* P = reinterpret_cast<uint32_t*>(smem_raw);
@@ -656,7 +689,7 @@ __global__ void __launch_bounds__(kExtWideThreads, 1)
     pdl_wait();   // the first-dimension results come from the previous kernel
     {
         uint32_t* S = P + grp * kPadN;   // polynomial grp = comp * 2 + prime
-        poly_to_smem<kNttGroup>(S, fd + (size_t)grp * kN);
+        first_dim_to_smem<kNttGroup>(S, fd + (size_t)grp * kN, sums, wo, r, grp);
         GroupSync::sync();
         uint32_t* co = coef_out ? shifted(coef_out, wo) + ((size_t)r * 4 + grp) * kN + u : nullptr;
         auto keep = [&](int, int t, uint32_t x) {

@@ -235,6 +235,7 @@ struct kspir_ctx {
     bool use_pdl = true;              // programmatic dependent launch inside the phases
     std::map<int, int> scan_choice;   // queries per launch -> ScanKind
     std::vector<char> slot_rm;        // the slot's last launch wrote its cipherbuf rotation-major (tensor-core scans)
+    std::vector<char> slot_sums;      // the slot's result holds the giant steps' accumulators (giant_sums), not final words
     // events of recent launches: ring[i][0..5] brackets baby / scan / giant / ext / packing
     std::vector<std::array<cudaEvent_t, 6>> ring;
     std::vector<int> ring_nq;
@@ -791,36 +792,48 @@ void enqueue_scan(kspir_ctx* c, int slot0, int nq, int kind, cudaStream_t st, bo
     if (tail) tiles(smallest_tile(tail), slot0 + nq - tail, tail);
 }
 
+// where the sums over the giant steps of slot 0 are
+GiantSums giant_sums(const kspir_ctx* c) {
+    return GiantSums{c->ws0.sout, giant_two_acc(c) ? c->ws0.ecoef : nullptr, c->N2, c->p.r * c->N2};
+}
+
+// More ciphertexts than SMs: one CTA per ciphertext with fewer transforms, which in an
+// answer adds the giant steps up itself; else two SMs per ciphertext (k_ext_wide)
+bool ext_wide(const kspir_ctx* c, int count, int nq) { return (long)count * nq > c->nsm; }
+
+// The first-dimension results from their accumulators, in place, or of one slot into `out`
+void enqueue_giant_finish(kspir_ctx* c, int slot0, int nq, uint32_t* out, cudaStream_t st) {
+    launch(c, false, k_giant_finish, dim3(blocks_for((long)c->p.r * 4 * (kN / 4), 256), nq), 256, 0, st, giant_sums(c),
+           c->ws0.result, out, c->p.r, batch_of(c, slot0));
+}
+
 // The giant steps add into result (and, past kGiantTermsPerAcc steps per
 // sub-database, ecoef as the second accumulator), which the answer's
-// k_query_prep (enqueue_baby) has zeroed.
-void enqueue_giant(kspir_ctx* c, int slot0, int nq, cudaStream_t st) {
+// k_query_prep (enqueue_baby) has zeroed.  finish: result then holds the sums.
+void enqueue_giant(kspir_ctx* c, int slot0, int nq, bool finish, cudaStream_t st) {
     const Workspace& w = c->ws0;
-    const Batch bt = batch_of(c, slot0);
     const int R = c->p.r;
-    uint32_t* acc1 = giant_two_acc(c) ? w.ecoef : nullptr;
-    if (c->N2 > 1)
-        launch(c, false, k_giant_fused<2>, dim3(R * (c->N2 - 1), nq), kNttThreads, kGiantSmem, st,
-               (const uint32_t*)w.sout, w.result, acc1, (const uint32_t*)c->keys0.giant,
-               (const uint16_t*)c->sigma_giant, c->N1, c->ntabs, c->gad.giant, R, bt);
-    launch(c, false, k_giant_finish, dim3(blocks_for((long)R * 4 * (kN / 4), 256), nq), 256, 0, st, (const uint32_t*)w.sout,
-           w.result, (const uint32_t*)acc1, R, c->N2, bt);
+    launch(c, false, k_giant_fused<2>, dim3(R * (c->N2 - 1), nq), kNttThreads, kGiantSmem, st, (const uint32_t*)w.sout,
+           w.result, giant_two_acc(c) ? w.ecoef : nullptr, (const uint32_t*)c->keys0.giant,
+           (const uint16_t*)c->sigma_giant, c->N1, c->ntabs, c->gad.giant, R, batch_of(c, slot0));
+    if (finish) enqueue_giant_finish(c, slot0, nq, nullptr, st);
 }
 
 // external products of `count` first-dimension results (result -> ext);
 // `init` holds NTT-domain accumulators ([count][2][2][N], slot-0 workspace
 // address) or is null for zero; coef_out (or null) receives the
-// first-dimension results in coefficient form
-void enqueue_ext(kspir_ctx* c, int slot0, int nq, int count, const uint32_t* init, uint32_t* coef_out,
+// first-dimension results in coefficient form; sums: result holds the giant steps'
+// accumulators (ext_wide only)
+void enqueue_ext(kspir_ctx* c, int slot0, int nq, int count, bool sums, const uint32_t* init, uint32_t* coef_out,
                  cudaStream_t st) {
     const Workspace& w = c->ws0;
-    // more ciphertexts than SMs: fewer transforms; else two SMs per ciphertext (k_ext_wide)
-    if ((long)count * nq > c->nsm)
+    if (ext_wide(c, count, nq))
         launch(c, false, k_ext_wide<2>, dim3(count, nq), kExtWideThreads, kExtWideSmem, st, (const uint32_t*)w.result,
-               (const uint32_t*)c->keys0.rgsw, init, w.ext, coef_out, c->ntabs, c->gad.ext, batch_of(c, slot0));
+               sums ? giant_sums(c) : GiantSums{}, (const uint32_t*)c->keys0.rgsw, init, w.ext, coef_out, c->ntabs,
+               c->gad.ext, batch_of(c, slot0));
     else
         launch(c, false, k_ext_fused<2>, dim3(count * 2, nq), kNttThreads, kExtSmem, st, (const uint32_t*)w.result,
-           (const uint32_t*)c->keys0.rgsw, init, w.ext, coef_out, c->ntabs, c->gad.ext, batch_of(c, slot0));
+               (const uint32_t*)c->keys0.rgsw, init, w.ext, coef_out, c->ntabs, c->gad.ext, batch_of(c, slot0));
 }
 
 // Whether a packing level of I merges runs on the split kernels (one transform
@@ -865,10 +878,12 @@ void enqueue_compose(kspir_ctx* c, int slot0, int nq, uint64_t* resp, int* err_o
 
 // kernels launched by one enqueue_answer
 long answer_launches(const kspir_ctx* c, int kind, int nq) {
-    // baby 7 (and the transpose of a CUDA-core scan's), scan, giant 2, external product 1, packing one or two per level + compose
+    // baby 7 (and the transpose of a CUDA-core scan's), scan, giant 1 or 2, external product 1, packing one or
+    // two per level + compose
     long packing = 0;
     for (int lv = 0; lv < c->levels; lv++) packing += pack_split(c, nq, 1 << lv, nullptr) ? 2 : 1;
-    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(c, kind, nq) + (c->N2 > 1 ? 2 : 1) + 1 + packing + 1;
+    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(c, kind, nq) + (ext_wide(c, c->p.r, nq) ? 1 : 2) + 1 +
+           packing + 1;
 }
 
 // Captures the four non-scan phases of (slot0, nq) as CUDA graphs (the scan
@@ -887,8 +902,8 @@ int build_graphs(kspir_ctx* c, int slot0, int nq, bool rm, kspir_ctx::PhaseGraph
         if (ph == 3 && c->levels == 0) continue;   // nothing to pack
         KS_CUDA(c, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
         if (ph == 0) enqueue_baby(c, slot0, nq, rm, cs);
-        else if (ph == 1) enqueue_giant(c, slot0, nq, cs);
-        else if (ph == 2) enqueue_ext(c, slot0, nq, c->p.r, nullptr, nullptr, cs);
+        else if (ph == 1) enqueue_giant(c, slot0, nq, !ext_wide(c, c->p.r, nq), cs);
+        else if (ph == 2) enqueue_ext(c, slot0, nq, c->p.r, ext_wide(c, c->p.r, nq), nullptr, nullptr, cs);
         else enqueue_packing(c, slot0, nq, cs);
         KS_CUDA(c, cudaStreamEndCapture(cs, &g));
         cudaError_t e = cudaGraphInstantiate(&pg.g[ph], g, 0);
@@ -992,6 +1007,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
     auto& ev = c->ring[slot];
     if (allow_fused && c->fused && nq == 1 && slot0 == 0) {
         c->slot_rm[0] = 0;
+        c->slot_sums[0] = 0;
         cudaEventRecord(ev[0], st);
         int rc = enqueue_fused(c, clients[0], st, slot);
         if (rc) return rc;
@@ -1010,6 +1026,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
     int kind = scan_kind_for(c, nq);
     if (nq == 1 && one_on_tensor_cores(c, beside)) kind = SCAN_ONE;
     std::fill_n(c->slot_rm.begin() + slot0, nq, (char)(kind != SCAN_CUDA));
+    std::fill_n(c->slot_sums.begin() + slot0, nq, (char)ext_wide(c, c->p.r, nq));
     if (c->use_graphs) {
         kspir_ctx::PhaseGraphs* pg = nullptr;
         int rc = build_graphs(c, slot0, nq, kind != SCAN_CUDA, &pg);
@@ -1034,9 +1051,9 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         cudaEventRecord(ev[1], st);
         enqueue_scan(c, slot0, nq, kind, st, beside > 0);
         cudaEventRecord(ev[2], st);
-        enqueue_giant(c, slot0, nq, st);
+        enqueue_giant(c, slot0, nq, !ext_wide(c, c->p.r, nq), st);
         cudaEventRecord(ev[3], st);
-        enqueue_ext(c, slot0, nq, c->p.r, nullptr, nullptr, st);
+        enqueue_ext(c, slot0, nq, c->p.r, ext_wide(c, c->p.r, nq), nullptr, nullptr, st);
         cudaEventRecord(ev[4], st);
         enqueue_packing(c, slot0, nq, st);
         enqueue_compose(c, slot0, nq, io.resp, io.err, st);
@@ -1378,6 +1395,7 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     if (rc) return rc;
     KS_CUDA(c.get(), cudaMalloc(&c->perms, (size_t)p.N1 * kN * 2));
     c->slot_rm.assign(p.max_inflight, 0);
+    c->slot_sums.assign(p.max_inflight, 0);
     c->ring.resize(kTimingRing);
     c->ring_nq.assign(kTimingRing, 0);
     for (auto& evs : c->ring)
@@ -2512,9 +2530,10 @@ int kspir_matrix_vector_mul_bsgs_rns_crt_large(kspir_ctx* c, int client, uint64_
     KS_CUDA(c, cudaMemcpyAsync(c->bq64, query_inout, 4 * kN * 8, cudaMemcpyHostToDevice, st));
     enqueue_prep(c, 0, 1, &client, c->bq64, st);
     c->slot_rm[0] = 0;
+    c->slot_sums[0] = 0;
     enqueue_baby(c, 0, 1, false, st);
     enqueue_scan(c, 0, 1, SCAN_CUDA, st);
-    enqueue_giant(c, 0, 1, st);
+    enqueue_giant(c, 0, 1, true, st);
     // result words, and the modswitched query (cipherbuf column 0) back into query1[0]
     uint64_t* words = reinterpret_cast<uint64_t*>(c->stage32);
     k_compose_words<<<blocks_for((long)c->p.r * 2 * kN, 256), 256, 0, st>>>(w.result, words, c->p.r * 2);
@@ -2545,10 +2564,11 @@ int kspir_external_product(kspir_ctx* c, int client, uint64_t* result, uint64_t*
     // first_dim -> ws.result residues; the caller's accumulators (NTT domain) -> ws.sout residues
     KS_CUDA(c, cudaMemcpyAsync(words, first_dim, n * 8, cudaMemcpyHostToDevice, st));
     k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(words, w.result, count * 2);
+    c->slot_sums[0] = 0;
     uint32_t* acc = w.sout;   // r*N2*4*N >= count*4*N residues
     KS_CUDA(c, cudaMemcpyAsync(words, result, n * 8, cudaMemcpyHostToDevice, st));
     k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(words, acc, count * 2);
-    enqueue_ext(c, 0, 1, count, acc, w.ecoef, st);
+    enqueue_ext(c, 0, 1, count, false, acc, w.ecoef, st);
     k_compose_words<<<blocks_for((long)n, 256), 256, 0, st>>>(w.ext, words, count * 2);
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, cudaMemcpyAsync(result, words, n * 8, cudaMemcpyDeviceToHost, st));
@@ -2643,10 +2663,12 @@ int kspir_fetch_stage_slot(kspir_ctx* c, int slot, int stage, uint64_t* out, siz
     uint32_t* flat = nullptr;
     KS_CUDA(c, cudaMalloc(&tmp, words * 8));
     cudaError_t e = cudaSuccess;
-    if (stage == KSPIR_STAGE_SCAN) {
+    const bool sums = stage == KSPIR_STAGE_RESULT && c->slot_sums[slot];
+    if (stage == KSPIR_STAGE_SCAN || sums) {
         e = cudaMalloc(&flat, words * 8);
         if (e == cudaSuccess) {
-            k_unblock_sout<<<blocks_for((long)R * c->N2 * 4 * kN, 256), 256, 0, st>>>(src, flat, R * c->N2);
+            if (sums) enqueue_giant_finish(c, slot, 1, flat, st);
+            else k_unblock_sout<<<blocks_for((long)R * c->N2 * 4 * kN, 256), 256, 0, st>>>(src, flat, R * c->N2);
             src = flat;
         }
     }
