@@ -227,8 +227,10 @@ struct kspir_ctx {
     size_t key_bytes = 0;
     ClientKeysDev keys0{};
     std::vector<char> key_loaded;
-    // CUDA graphs of the four non-scan phases per (slot0, queries)
-    struct PhaseGraphs { cudaGraphExec_t g[4] = {nullptr, nullptr, nullptr, nullptr}; };
+    // CUDA graphs of the four non-scan phases per (slot0, queries); baby steps [rotation-major cipherbuf or not]
+    struct PhaseGraphs {
+        cudaGraphExec_t baby[2] = {nullptr, nullptr}, giant = nullptr, ext = nullptr, packing = nullptr;
+    };
     std::map<std::pair<int, int>, PhaseGraphs> graphs;
     cudaStream_t capture = nullptr;
     bool use_graphs = true;
@@ -891,28 +893,32 @@ long answer_launches(const kspir_ctx* c, int kind, int nq) {
 // events).  Pointers are fixed for the context's lifetime and the key slot of
 // each query is read from client_of at run time, so the graphs stay valid for
 // any clients and across key or database uploads.
+// A slot's answers may read either cipherbuf layout (one_on_tensor_cores): only
+// the baby steps are captured for each, when first needed.
 int build_graphs(kspir_ctx* c, int slot0, int nq, bool rm, kspir_ctx::PhaseGraphs** out) {
-    auto key = std::make_pair(slot0, nq * 2 + (rm ? 1 : 0));
-    auto it = c->graphs.find(key);
-    if (it != c->graphs.end()) { *out = &it->second; return KSPIR_OK; }
-    kspir_ctx::PhaseGraphs pg;
+    kspir_ctx::PhaseGraphs& pg = c->graphs[std::make_pair(slot0, nq)];
+    *out = &pg;
     cudaStream_t cs = c->capture;
-    for (int ph = 0; ph < 4; ph++) {
+    const bool wide = ext_wide(c, c->p.r, nq);
+    auto captured = [&](cudaGraphExec_t& exec, auto&& enqueue) -> int {
+        if (exec) return KSPIR_OK;
         cudaGraph_t g = nullptr;
-        if (ph == 3 && c->levels == 0) continue;   // nothing to pack
         KS_CUDA(c, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        if (ph == 0) enqueue_baby(c, slot0, nq, rm, cs);
-        else if (ph == 1) enqueue_giant(c, slot0, nq, !ext_wide(c, c->p.r, nq), cs);
-        else if (ph == 2) enqueue_ext(c, slot0, nq, c->p.r, ext_wide(c, c->p.r, nq), nullptr, nullptr, cs);
-        else enqueue_packing(c, slot0, nq, cs);
+        enqueue();
         KS_CUDA(c, cudaStreamEndCapture(cs, &g));
-        cudaError_t e = cudaGraphInstantiate(&pg.g[ph], g, 0);
+        cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
-        if (e != cudaSuccess) return set_err(c, KSPIR_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    }
-    auto res = c->graphs.emplace(key, pg);
-    *out = &res.first->second;
-    return KSPIR_OK;
+        if (e != cudaSuccess) {
+            exec = nullptr;
+            return set_err(c, KSPIR_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+        }
+        return KSPIR_OK;
+    };
+    int rc = captured(pg.baby[rm], [&] { enqueue_baby(c, slot0, nq, rm, cs); });
+    if (!rc) rc = captured(pg.giant, [&] { enqueue_giant(c, slot0, nq, !wide, cs); });
+    if (!rc) rc = captured(pg.ext, [&] { enqueue_ext(c, slot0, nq, c->p.r, wide, nullptr, nullptr, cs); });
+    if (!rc && c->levels) rc = captured(pg.packing, [&] { enqueue_packing(c, slot0, nq, cs); });
+    return rc;
 }
 
 // The fused single answer of workspace slot 0 (k_answer.cuh): reset of its
@@ -1033,15 +1039,15 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
         if (rc) return rc;
         cudaEventRecord(ev[0], st);
         enqueue_prep(c, slot0, nq, clients, io.q, st);
-        KS_CUDA(c, cudaGraphLaunch(pg->g[0], st));
+        KS_CUDA(c, cudaGraphLaunch(pg->baby[kind != SCAN_CUDA], st));
         cudaEventRecord(ev[1], st);
         enqueue_scan(c, slot0, nq, kind, st, beside > 0);
         cudaEventRecord(ev[2], st);
-        KS_CUDA(c, cudaGraphLaunch(pg->g[1], st));
+        KS_CUDA(c, cudaGraphLaunch(pg->giant, st));
         cudaEventRecord(ev[3], st);
-        KS_CUDA(c, cudaGraphLaunch(pg->g[2], st));
+        KS_CUDA(c, cudaGraphLaunch(pg->ext, st));
         cudaEventRecord(ev[4], st);
-        if (pg->g[3]) KS_CUDA(c, cudaGraphLaunch(pg->g[3], st));
+        if (pg->packing) KS_CUDA(c, cudaGraphLaunch(pg->packing, st));
         enqueue_compose(c, slot0, nq, io.resp, io.err, st);
         cudaEventRecord(ev[5], st);
     } else {
@@ -1438,7 +1444,8 @@ int kspir_ctx_destroy(kspir_ctx* c) {
     if (c->single_errs) cudaFreeHost(c->single_errs);
     if (c->single_io) cudaFreeHost(c->single_io);
     for (auto& kv : c->graphs)
-        for (auto& g : kv.second.g) if (g) cudaGraphExecDestroy(g);
+        for (cudaGraphExec_t g : {kv.second.baby[0], kv.second.baby[1], kv.second.giant, kv.second.ext, kv.second.packing})
+            if (g) cudaGraphExecDestroy(g);
     if (c->capture) cudaStreamDestroy(c->capture);
     cudaFree(c->ws_mem);
     cudaFree(c->jobs);
