@@ -14,7 +14,7 @@
 //
 // Data movement: one 16 KiB slab DB[r][z] (N2 x N1 words) plus the 16*N1-byte
 // cipherbuf row z per work item, brought in by 1-D bulk copies (TMA engine,
-// no multicast) into an NST-deep shared-memory ring (12 stages at N1 = 128);
+// no multicast) into an NST-deep shared-memory ring (8 stages at N1 = 128);
 // one producer warp issues, CONS consumer warps each take one item at a time.
 //
 // Consumer mapping (one warp per slab): lane = 8 * r + c covers rows

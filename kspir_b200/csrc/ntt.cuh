@@ -35,7 +35,7 @@
 // own.
 //
 // 4096-point forward and inverse transforms of a batch of 64 (r = 16), giant
-// steps included: see the figures at k_giant_fused and k_baby_pair.
+// steps included: see the figures at k_giant_fused and k_baby.cuh.
 //
 // Shared-memory layout.  A polynomial occupies kPadN words: coefficient (or
 // slot) i sits at pidx(i) = i + 4 (i / 32) + 16 (i / 256).  With that padding
