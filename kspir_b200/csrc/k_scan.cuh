@@ -42,11 +42,12 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;     // 2 s per bounded wait
 // Ring shapes of the single-query scan, measured on B200 with a 1 GiB
 // database (consumer warps x stages of 18 KiB, 148 CTAs): 4 x 8 0.156 ms
 // (6.9 TB/s), 6 x 6 0.176 ms, 6 x 12 0.176 ms, 4 x 4 0.214 ms.  The default
-// (streaming) shape is 4 x 8: 148 KiB of shared memory, which leaves room on
-// the SM for a baby-step or transform CTA of a concurrent answer.  The sharing
-// shape (ScanShare) is 6 x 6: 110 KiB, slower alone but leaving room for a
-// giant-step or external-product CTA (107 KiB) beside it, which pays when
-// several answers are in flight.
+// (streaming) shape is 4 x 8: 145 KiB of shared memory, which leaves 82 KiB of the
+// SM to key-switch CTAs (19 to 76 KiB each) of a concurrent answer.  The sharing shape
+// (ScanShare) is 6 x 6: 109 KiB, slower alone but leaving 118, which pays at N1 = 128 when
+// other answers are in flight: us for 16 answers on eight streams at r = 1 619
+// (streaming) -> 598, for 32 at r = 2 1611 -> 1561, two at r = 64 1467 -> 1451.  At N1 =
+// 64 it does not: 32 answers at r = 8 4160 -> 4421, three 390 -> 416.
 template <int N1, int CONS_ = 4, int NST_ = 8>
 struct ScanCfg {
     static constexpr int N2 = kN / 2 / N1;
@@ -68,9 +69,9 @@ struct ScanCfg {
 };
 
 template <int N1>
-struct ScanShare {   // 6 x 6 where a 107 KiB CTA still fits beside it (N1 <= 128)
-    static constexpr int CONS = N1 <= 128 ? 6 : 4;
-    static constexpr int NST = N1 <= 128 ? 6 : 8;
+struct ScanShare {   // 6 x 6 at N1 = 128, else the streaming shape
+    static constexpr int CONS = N1 == 128 ? 6 : 4;
+    static constexpr int NST = N1 == 128 ? 6 : 8;
     using Cfg = ScanCfg<N1, CONS, NST>;
 };
 
