@@ -809,6 +809,17 @@ void enqueue_giant_finish(kspir_ctx* c, int slot0, int nq, uint32_t* out, cudaSt
            c->ws0.result, out, c->p.r, batch_of(c, slot0));
 }
 
+// Before the scan outputs of slots slot0 .. slot0 + nq - 1 are used for something else:
+// where a launch left sums to be added up from them (slot_sums), the results in
+// place
+void settle_sums(kspir_ctx* c, int slot0, int nq, cudaStream_t st) {
+    for (int s = slot0; s < slot0 + nq; s++)
+        if (c->slot_sums[s]) {
+            enqueue_giant_finish(c, s, 1, nullptr, st);
+            c->slot_sums[s] = 0;
+        }
+}
+
 // The giant steps add into result (and, past kGiantTermsPerAcc steps per
 // sub-database, ecoef as the second accumulator), which the answer's
 // k_query_prep (enqueue_baby) has zeroed.  finish: result then holds the sums.
@@ -2396,6 +2407,7 @@ int kspir_tune_batch(kspir_ctx* c, int n, int* kind_out, float* ms_out) {
     std::lock_guard<std::mutex> lk(c->mu);
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
+    settle_sums(c, 0, n, c->stream);   // each scan below overwrites their scan outputs
     cudaEvent_t e0, e1;
     KS_CUDA(c, cudaEventCreate(&e0));
     KS_CUDA(c, cudaEventCreate(&e1));
@@ -2566,12 +2578,12 @@ int kspir_external_product(kspir_ctx* c, int client, uint64_t* result, uint64_t*
     cudaStream_t st = c->stream;
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
+    settle_sums(c, 0, 1, st);   // count < r leaves some of the results as they are
     k_set_client<<<1, 1, 0, st>>>(c->client_of, 0, client);
     uint64_t* words = reinterpret_cast<uint64_t*>(c->stage32);     // r*2*N u64 fit in r*4*N u32
     // first_dim -> ws.result residues; the caller's accumulators (NTT domain) -> ws.sout residues
     KS_CUDA(c, cudaMemcpyAsync(words, first_dim, n * 8, cudaMemcpyHostToDevice, st));
     k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(words, w.result, count * 2);
-    c->slot_sums[0] = 0;
     uint32_t* acc = w.sout;   // r*N2*4*N >= count*4*N residues
     KS_CUDA(c, cudaMemcpyAsync(words, result, n * 8, cudaMemcpyHostToDevice, st));
     k_split_words<<<blocks_for((long)n, 256), 256, 0, st>>>(words, acc, count * 2);
@@ -2600,6 +2612,7 @@ int kspir_packing_rlwes(kspir_ctx* c, int client, uint64_t* rlwes, uint64_t* res
     cudaStream_t st = c->stream;
     KS_CUDA(c, cudaSetDevice(c->device));
     if (int wrc = wait_singles(c, c->stream)) return wrc;
+    settle_sums(c, 0, 1, st);
     k_set_client<<<1, 1, 0, st>>>(c->client_of, 0, client);
     uint64_t* words = reinterpret_cast<uint64_t*>(c->stage32);
     KS_CUDA(c, cudaMemcpyAsync(words, rlwes, n * 8, cudaMemcpyHostToDevice, st));
