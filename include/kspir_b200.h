@@ -245,10 +245,15 @@ int kspir_answer_batch_device(kspir_ctx* ctx, int n, const int32_t* clients, con
  * returns it; ms_out ([5] or NULL) receives each variant's scan time (1e30 for
  * variants not tried).  Do not call while answers are in flight: it uses the
  * workspaces.  kspir_set_scan_kind forces a variant (-1 = back to the
- * default), kspir_get_scan_kind reports the one in use. */
+ * default), kspir_get_scan_kind reports the one in use.  A single answer with
+ * two others or more in flight may run on the tensor cores although
+ * kspir_get_scan_kind(1) says 0: kspir_slot_scan_kind reports the variant of
+ * the last launch in a workspace slot, 5 for this one (KSPIR_ERR_NOT_READY
+ * before the first). */
 int kspir_tune_batch(kspir_ctx* ctx, int n, int* kind_out, float* ms_out);
 int kspir_set_scan_kind(kspir_ctx* ctx, int n, int kind);
 int kspir_get_scan_kind(kspir_ctx* ctx, int n);
+int kspir_slot_scan_kind(kspir_ctx* ctx, int slot);
 
 /* Reference matrix_vector_mul_bsgs_rns_crt_large (twosteps.h:55-57,
  * twosteps.cpp:1527-1579) for one client: query_inout is modswitched in place

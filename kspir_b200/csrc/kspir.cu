@@ -236,7 +236,8 @@ struct kspir_ctx {
     bool use_graphs = true;
     bool use_pdl = true;              // programmatic dependent launch inside the phases
     std::map<int, int> scan_choice;   // queries per launch -> ScanKind
-    std::vector<char> slot_rm;        // the slot's last launch wrote its cipherbuf rotation-major (tensor-core scans)
+    std::vector<signed char> slot_kind;   // scan variant of the slot's last launch (all but SCAN_CUDA read their
+                                          // cipherbuf rotation-major), or -1
     std::vector<char> slot_sums;      // the slot's result holds the giant steps' accumulators (giant_sums), not final words
     // events of recent launches: ring[i][0..5] brackets baby / scan / giant / ext / packing
     std::vector<std::array<cudaEvent_t, 6>> ring;
@@ -1023,7 +1024,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
     const int slot = (int)(c->enqueues % kTimingRing);
     auto& ev = c->ring[slot];
     if (allow_fused && c->fused && nq == 1 && slot0 == 0) {
-        c->slot_rm[0] = 0;
+        c->slot_kind[0] = SCAN_CUDA;
         c->slot_sums[0] = 0;
         cudaEventRecord(ev[0], st);
         int rc = enqueue_fused(c, clients[0], st, slot);
@@ -1042,7 +1043,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
     if (!io.resp) io.resp = c->bresp + (size_t)slot0 * 2 * kN;
     int kind = scan_kind_for(c, nq);
     if (nq == 1 && one_on_tensor_cores(c, beside)) kind = SCAN_ONE;
-    std::fill_n(c->slot_rm.begin() + slot0, nq, (char)(kind != SCAN_CUDA));
+    std::fill_n(c->slot_kind.begin() + slot0, nq, (signed char)kind);
     std::fill_n(c->slot_sums.begin() + slot0, nq, (char)ext_wide(c, c->p.r, nq));
     if (c->use_graphs) {
         kspir_ctx::PhaseGraphs* pg = nullptr;
@@ -1411,7 +1412,7 @@ int kspir_ctx_create(int device, const kspir_params* params, kspir_ctx** out) {
     rc = init_constants(c.get());
     if (rc) return rc;
     KS_CUDA(c.get(), cudaMalloc(&c->perms, (size_t)p.N1 * kN * 2));
-    c->slot_rm.assign(p.max_inflight, 0);
+    c->slot_kind.assign(p.max_inflight, -1);
     c->slot_sums.assign(p.max_inflight, 0);
     c->ring.resize(kTimingRing);
     c->ring_nq.assign(kTimingRing, 0);
@@ -2449,6 +2450,12 @@ int kspir_set_scan_kind(kspir_ctx* c, int n, int kind) {
 
 int kspir_get_scan_kind(kspir_ctx* c, int n) { return c ? scan_kind_for(c, n) : KSPIR_ERR_INVALID_ARG; }
 
+int kspir_slot_scan_kind(kspir_ctx* c, int slot) {
+    if (!c || slot < 0 || slot >= c->p.max_inflight) return KSPIR_ERR_INVALID_ARG;
+    std::lock_guard<std::mutex> lk(c->mu);
+    return c->slot_kind[slot] < 0 ? KSPIR_ERR_NOT_READY : c->slot_kind[slot];
+}
+
 namespace {
 // Phase split of a fused answer from its device timestamps: the segments of its
 // critical path (query side up to the scan start or the last rotation, the
@@ -2548,7 +2555,7 @@ int kspir_matrix_vector_mul_bsgs_rns_crt_large(kspir_ctx* c, int client, uint64_
     if (int wrc = wait_singles(c, c->stream)) return wrc;
     KS_CUDA(c, cudaMemcpyAsync(c->bq64, query_inout, 4 * kN * 8, cudaMemcpyHostToDevice, st));
     enqueue_prep(c, 0, 1, &client, c->bq64, st);
-    c->slot_rm[0] = 0;
+    c->slot_kind[0] = SCAN_CUDA;
     c->slot_sums[0] = 0;
     enqueue_baby(c, 0, 1, false, st);
     enqueue_scan(c, 0, 1, SCAN_CUDA, st);
@@ -2660,7 +2667,7 @@ int kspir_fetch_stage_slot(kspir_ctx* c, int slot, int stage, uint64_t* out, siz
         const size_t n = (size_t)kN * c->N1 * 2;
         if (words != n) return set_err(c, KSPIR_ERR_INVALID_ARG, "size mismatch");
         KS_COPY(c, out, w.cipherbuf, n * 8, cudaMemcpyDeviceToHost);
-        if (c->slot_rm[slot]) {
+        if (c->slot_kind[slot] > SCAN_CUDA) {
             // the tensor-core scans' launches write it rotation-major: back to [N][N1][2]
             std::vector<uint32_t> rm(2 * n);
             memcpy(rm.data(), out, n * 8);

@@ -77,6 +77,7 @@ SIGNATURES = {
     "kspir_tune_batch": (_i, [_vp, _i, _vp, _vp]),
     "kspir_set_scan_kind": (_i, [_vp, _i, _i]),
     "kspir_get_scan_kind": (_i, [_vp, _i]),
+    "kspir_slot_scan_kind": (_i, [_vp, _i]),
     "kspir_fetch_stage_slot": (_i, [_vp, _i, _i, _vp, _sz]),
     "kspir_client_key_bytes": (_sz, [_vp]),
     "kspir_debug_scan_fault": (_i, [_vp, ctypes.c_int64, ctypes.c_long]),
@@ -100,8 +101,9 @@ SCAN_MMA4 = 1
 SCAN_MMA8 = 2
 SCAN_MMA16 = 3
 SCAN_MMA32 = 4
+SCAN_ONE = 5   # one query on the tensor cores: only reported (Context.slot_scan_kind)
 SCAN_NAMES = {SCAN_CUDA: "cuda-core", SCAN_MMA4: "tcgen05-bt4", SCAN_MMA8: "tcgen05-bt8",
-              SCAN_MMA16: "tcgen05-bt16", SCAN_MMA32: "tcgen05-bt32"}
+              SCAN_MMA16: "tcgen05-bt16", SCAN_MMA32: "tcgen05-bt32", SCAN_ONE: "tcgen05-one"}
 
 
 class Params(ctypes.Structure):
@@ -434,6 +436,13 @@ class Context:
 
     def scan_kind(self, n: int) -> int:
         return self.lib.kspir_get_scan_kind(self._h, n)
+
+    def slot_scan_kind(self, slot: int = 0) -> int:
+        """Scan variant (SCAN_*) of the last launch in a workspace slot."""
+        kind = self.lib.kspir_slot_scan_kind(self._h, slot)
+        if kind < 0:
+            self._check(kind)
+        return kind
 
     def last_timing(self):
         tot = ctypes.c_float()

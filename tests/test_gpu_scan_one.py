@@ -1,0 +1,62 @@
+"""The tensor-core database scan of one query: that the answers meant to run on it
+do, and their words.  Eight answers are issued on four streams that a sleeping
+kernel holds up, so that how many others each finds in flight is known: none and
+one for the first two (CUDA cores), two or three for the rest (tensor cores from 64
+database rows on).  Word for word against the same queries alone and the oracle,
+also with every database half at 2^32 - 1 (sums that wrap modulo 2^64)."""
+import numpy as np
+import pytest
+import torch
+
+import kspir_b200 as kb
+from kspir_b200 import serving
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+N = po.N
+N1, ANSWERS = 128, 8   # one per workspace slot of the single answers
+
+
+def context(r, db, keys):
+    ctx = kb.Context(r, N1, max_clients=1, max_inflight=8)
+    ctx.upload_db(db)
+    ctx.upload_perms(keys["perms"])
+    ctx.upload_client(0, keys["baby"], keys["giant"], keys["packing"], keys["rgsw"])
+    return ctx
+
+
+def database(r, fill):
+    return np.full(r * N * N // 2, np.uint64(0xFFFFFFFFFFFFFFFF)) if fill == "ones" else po.gen_db(701, r, N1)
+
+
+def issue(ctx, q):
+    """Responses of the queries issued side by side, and each one's scan variant."""
+    d_q = torch.from_numpy(q.view(np.int64)).cuda()
+    d_r = torch.zeros((ANSWERS, 2 * N), dtype=torch.int64, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    torch.cuda.synchronize()
+    for s in streams:
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(200_000_000)   # a tenth of a second
+    for i in range(ANSWERS):
+        ctx.answer_device(0, d_q[i].data_ptr(), d_r[i].data_ptr(), streams[i % 4].cuda_stream)
+    kinds = [ctx.slot_scan_kind(i) for i in range(ANSWERS)]
+    ctx.sync()
+    return d_r.cpu().numpy().view(np.uint64), kinds
+
+
+@pytest.mark.parametrize("r,fill", [(2, "words"), (4, "words"), (4, "ones"), (8, "words"), (16, "ones")])
+def test_answers_beside_others(r, fill):
+    db, keys = database(r, fill), po.gen_client(710, r, N1)
+    q = serving.random_queries(np.random.default_rng(r), ANSWERS)
+    q[3] = 0
+    with context(r, db, keys) as ctx:
+        alone = [ctx.answer(0, q[i]) for i in range(ANSWERS)]
+        assert [ctx.slot_scan_kind(i) for i in range(ANSWERS)] == [kb.SCAN_CUDA] * ANSWERS
+        got, kinds = issue(ctx, q)
+        beside = kb.SCAN_ONE if r * (N // 2 // N1) >= 64 else kb.SCAN_CUDA
+        assert kinds == [kb.SCAN_CUDA] * 2 + [beside] * (ANSWERS - 2)
+        for i in range(ANSWERS):
+            assert np.array_equal(got[i], alone[i]), i
+        for i in (2, 3, 7):
+            assert np.array_equal(got[i], po.answer(db, r, N1, dict(keys, query=q[i]))), i
