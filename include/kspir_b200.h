@@ -239,7 +239,8 @@ int kspir_answer_batch_device(kspir_ctx* ctx, int n, const int32_t* clients, con
 
 /* Database-scan variant used for a batch of n queries:
  *   0 CUDA-core scan, one database pass per query
- *   1..4 tensor-core scan with query tiles of 4, 8, 16, 32 queries
+ *   1..4 tensor-core scan with query tiles of 4, 8, 16, 32 queries (n = 1: the
+ *        tensor-core scan of one query, whichever is given)
  * kspir_tune_batch times every variant on the resident database (results are
  * identical by construction; only speed differs), keeps the fastest for n and
  * returns it; ms_out ([5] or NULL) receives each variant's scan time (1e30 for
@@ -248,8 +249,8 @@ int kspir_answer_batch_device(kspir_ctx* ctx, int n, const int32_t* clients, con
  * default), kspir_get_scan_kind reports the one in use.  A single answer with
  * two others or more in flight may run on the tensor cores although
  * kspir_get_scan_kind(1) says 0: kspir_slot_scan_kind reports the variant of
- * the last launch in a workspace slot, 5 for this one (KSPIR_ERR_NOT_READY
- * before the first). */
+ * the last launch in a workspace slot, 5 for the tensor-core scan of one query
+ * (KSPIR_ERR_NOT_READY before the first). */
 int kspir_tune_batch(kspir_ctx* ctx, int n, int* kind_out, float* ms_out);
 int kspir_set_scan_kind(kspir_ctx* ctx, int n, int kind);
 int kspir_get_scan_kind(kspir_ctx* ctx, int n);

@@ -171,7 +171,7 @@ __global__ void k_unblock_sout(const uint32_t* __restrict__ sout, uint32_t* __re
 
 // database-scan variants (chosen per batch size by kspir_tune_batch)
 enum ScanKind { SCAN_CUDA = 0, SCAN_MMA4 = 1, SCAN_MMA8 = 2, SCAN_MMA16 = 3, SCAN_MMA32 = 4, SCAN_KINDS = 5,
-                SCAN_ONE = 5 };   // one query on the tensor cores (k_scan_mma1): chosen by enqueue_answer only
+                SCAN_ONE = 5 };   // one query on the tensor cores (k_scan_mma1): every launch of one query but SCAN_CUDA's
 int scan_bt(int kind) { return kind == SCAN_MMA4 ? 4 : kind == SCAN_MMA8 ? 8 : kind == SCAN_MMA16 ? 16 : 32; }
 
 }  // namespace
@@ -721,7 +721,9 @@ long scan_launches(const kspir_ctx*, int kind, int nq) {
 
 // Query-operand region of a launch starting at workspace slot slot0: 8 MiB per
 // slot, so launches on disjoint 32-aligned slot ranges (serving lanes) never
-// share it.
+// share it.  Nor do single answers in neighbouring slots: a launch of one query
+// takes k_scan_mma1, whose operand is 8 MiB, whatever tile was chosen for n = 1
+// (a query tile of BT takes 8 BT MiB, padding included).
 uint8_t* qop_at(kspir_ctx* c, int slot0) { return c->qop + (size_t)slot0 * kN * 2 * 8 * kMmaK; }
 
 template <int BT>
@@ -774,7 +776,7 @@ void enqueue_scan(kspir_ctx* c, int slot0, int nq, int kind, cudaStream_t st, bo
         return;
     }
     int* err = c->errs + (size_t)slot0 * kErrStride;   // the batch's error word
-    if (kind == SCAN_ONE) {
+    if (nq == 1) {
         const Workspace w = ws_host(c, slot0);
         uint8_t* qop = qop_at(c, slot0);
         k_qop_split_rm<1><<<dim3(kN / kSplitZ, 1), kSplitThreads, kSplitSmem, st>>>(
@@ -1042,7 +1044,7 @@ int enqueue_answer(kspir_ctx* c, int slot0, int nq, const int* clients, cudaStre
     if (!io.q) io.q = c->bq64 + (size_t)slot0 * 4 * kN;
     if (!io.resp) io.resp = c->bresp + (size_t)slot0 * 2 * kN;
     int kind = scan_kind_for(c, nq);
-    if (nq == 1 && one_on_tensor_cores(c, beside)) kind = SCAN_ONE;
+    if (nq == 1 && (kind != SCAN_CUDA || one_on_tensor_cores(c, beside))) kind = SCAN_ONE;
     std::fill_n(c->slot_kind.begin() + slot0, nq, (signed char)kind);
     std::fill_n(c->slot_sums.begin() + slot0, nq, (char)ext_wide(c, c->p.r, nq));
     if (c->use_graphs) {

@@ -2,7 +2,8 @@
 do, and their words.  Eight answers are issued on four streams that a sleeping
 kernel holds up, so that how many others each finds in flight is known: none and
 one for the first two (CUDA cores), two or three for the rest (tensor cores from 64
-database rows on).  Word for word against the same queries alone and the oracle,
+database rows on).  A tile chosen for n = 1 means the same scan, on every stream and at
+any number of rows.  Word for word against the same queries alone and the oracle,
 also with every database half at 2^32 - 1 (sums that wrap modulo 2^64)."""
 import numpy as np
 import pytest
@@ -60,3 +61,25 @@ def test_answers_beside_others(r, fill):
             assert np.array_equal(got[i], alone[i]), i
         for i in (2, 3, 7):
             assert np.array_equal(got[i], po.answer(db, r, N1, dict(keys, query=q[i]))), i
+
+
+@pytest.mark.parametrize("r,kind", [(1, kb.SCAN_MMA4), (2, kb.SCAN_MMA8), (4, kb.SCAN_MMA16), (4, kb.SCAN_MMA32)])
+def test_tile_chosen_for_one_query(r, kind):
+    db, keys = database(r, "words"), po.gen_client(720, r, N1)
+    q = serving.random_queries(np.random.default_rng(20 + r), ANSWERS)
+    want = [po.answer(db, r, N1, dict(keys, query=x)) for x in q]
+    with context(r, db, keys) as ctx:
+        ctx.set_scan_kind(1, kind)
+        assert ctx.scan_kind(1) == kind
+        for _ in range(3):
+            got, kinds = issue(ctx, q)
+            assert kinds == [kb.SCAN_ONE] * ANSWERS
+            for i in range(ANSWERS):
+                assert np.array_equal(got[i], want[i]), i
+        assert np.array_equal(ctx.answer(0, q[0]), want[0])   # slot 0 again
+        scan = ctx.fetch_stage(kb.STAGE_SCAN)
+        assert np.array_equal(ctx.answer_batch(np.zeros(1, np.int32), q[:1])[0], want[0])
+        assert np.array_equal(ctx.fetch_stage(kb.STAGE_SCAN), scan)
+        ctx.set_scan_kind(1, kb.SCAN_CUDA)
+        assert np.array_equal(ctx.answer_batch(np.zeros(1, np.int32), q[:1])[0], want[0])
+        assert np.array_equal(ctx.fetch_stage(kb.STAGE_SCAN), scan)
