@@ -248,7 +248,7 @@ int kspir_answer_batch_device(kspir_ctx* ctx, int n, const int32_t* clients, con
  * workspaces.  kspir_set_scan_kind forces a variant (-1 = back to the
  * default), kspir_get_scan_kind reports the one in use.  A single answer with
  * two others or more in flight may run on the tensor cores although
- * kspir_get_scan_kind(1) says 0: kspir_slot_scan_kind reports the variant of
+ * kspir_get_scan_kind(1) says 0, unless that was forced: kspir_slot_scan_kind reports the variant of
  * the last launch in a workspace slot, 5 for the tensor-core scan of one query
  * (KSPIR_ERR_NOT_READY before the first). */
 int kspir_tune_batch(kspir_ctx* ctx, int n, int* kind_out, float* ms_out);

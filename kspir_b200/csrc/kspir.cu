@@ -236,6 +236,7 @@ struct kspir_ctx {
     bool use_graphs = true;
     bool use_pdl = true;              // programmatic dependent launch inside the phases
     std::map<int, int> scan_choice;   // queries per launch -> ScanKind
+    bool one_forced = false;          // the choice for one query was set, not tuned (with nothing else in flight)
     std::vector<signed char> slot_kind;   // scan variant of the slot's last launch (all but SCAN_CUDA read their
                                           // cipherbuf rotation-major), or -1
     std::vector<char> slot_sums;      // the slot's result holds the giant steps' accumulators (giant_sums), not final words
@@ -1000,14 +1001,14 @@ int enqueue_fused(kspir_ctx* c, int client, cudaStream_t st, int ring_slot) {
 
 // Whether the scan of a single answer with `beside` others in flight runs on the
 // tensor cores (k_scan_mma1): from two others and two 32-row tiles on, unless
-// the caller chose a variant for n = 1 or an injected failure waits for a CUDA-core
-// scan.  us per answer, CUDA cores -> tensor cores: 32 answers on eight streams, r =
+// the caller set a variant for n = 1 (a tuned one was timed with nothing beside it and
+// says nothing here) or an injected failure waits for a CUDA-core scan.  us per answer, CUDA cores -> tensor cores: 32 answers on eight streams, r =
 // 16: 225 -> 202, r = 4: 73.6 -> 69.2; 4 answers, r = 16: 261 -> 250, r = 4: 113 -> 112;
 // 8 answers 226 -> 226 (217 with three others), 89 -> 86.  r = 2: 53 to 58 either
 // way, r = 1: 47 -> 50 (half of the tile is padding).
 constexpr int kOneMinBeside = 2, kOneMinRows = 64;
 bool one_on_tensor_cores(const kspir_ctx* c, int beside) {
-    return c->mma && beside >= kOneMinBeside && c->p.r * c->N2 >= kOneMinRows && !c->scan_choice.count(1) && c->scan_skip < 0;
+    return c->mma && beside >= kOneMinBeside && c->p.r * c->N2 >= kOneMinRows && !c->one_forced && c->scan_skip < 0;
 }
 
 // allow_fused: a single answer of slot 0 through the public single-answer
@@ -2437,6 +2438,7 @@ int kspir_tune_batch(kspir_ctx* c, int n, int* kind_out, float* ms_out) {
     rc = finish(c, 0, n);
     if (rc) return rc;
     c->scan_choice[n] = best;
+    if (n == 1) c->one_forced = false;
     if (kind_out) *kind_out = best;
     return KSPIR_OK;
 }
@@ -2445,6 +2447,7 @@ int kspir_set_scan_kind(kspir_ctx* c, int n, int kind) {
     if (!c || n < 1 || kind < -1 || kind >= SCAN_KINDS) return KSPIR_ERR_INVALID_ARG;
     if (kind > SCAN_CUDA && !c->mma) return set_err(c, KSPIR_ERR_INVALID_ARG, "tensor-core scan not enabled");
     std::lock_guard<std::mutex> lk(c->mu);
+    if (n == 1) c->one_forced = kind >= 0;
     if (kind < 0) c->scan_choice.erase(n);
     else c->scan_choice[n] = kind;
     return KSPIR_OK;

@@ -83,3 +83,24 @@ def test_tile_chosen_for_one_query(r, kind):
         ctx.set_scan_kind(1, kb.SCAN_CUDA)
         assert np.array_equal(ctx.answer_batch(np.zeros(1, np.int32), q[:1])[0], want[0])
         assert np.array_equal(ctx.fetch_stage(kb.STAGE_SCAN), scan)
+
+
+def test_tuning_for_one_query_leaves_the_rule_beside_others():
+    r = 4
+    db, keys = database(r, "words"), po.gen_client(730, r, N1)
+    q = serving.random_queries(np.random.default_rng(30), ANSWERS)
+    with context(r, db, keys) as ctx:
+        alone = [ctx.answer(0, q[i]) for i in range(ANSWERS)]
+        tuned, _ = ctx.tune_batch(1)
+        assert ctx.scan_kind(1) == tuned
+        ctx.answer(0, q[0])
+        assert ctx.slot_scan_kind(0) == (kb.SCAN_CUDA if tuned == kb.SCAN_CUDA else kb.SCAN_ONE)
+        for i in range(1, ANSWERS):   # slot 0 comes next again
+            ctx.answer(0, q[i])
+        for choose, beside in ((None, kb.SCAN_ONE), (kb.SCAN_CUDA, kb.SCAN_CUDA), (-1, kb.SCAN_ONE)):
+            if choose is not None:
+                ctx.set_scan_kind(1, choose)
+            got, kinds = issue(ctx, q)
+            assert kinds[2:] == [beside] * (ANSWERS - 2), choose
+            for i in range(ANSWERS):
+                assert np.array_equal(got[i], alone[i]), i
