@@ -346,8 +346,9 @@ int kspir_fetch_stage_slot(kspir_ctx* ctx, int slot, int stage, uint64_t* out, s
  * wait of the database scan on the device is bounded: a wait that runs out
  * records an error word and the kernel returns, and the call that collects
  * the launch reports KSPIR_ERR_TIMEOUT; the context stays usable.  This sets
- * the limit of those waits (wait_limit_ns <= 0: the default of 2 s) and makes
- * the next CUDA-core database scan (the one of a single answer) skip the copy
+ * the limit of those waits (wait_limit_ns <= 0: the default of 2 s; the
+ * tensor-core scan of a batch always keeps that) and makes the next database
+ * scan of one query, on the CUDA cores or the tensor cores, skip the copy
  * of local work item `skip_item` of its first CTA (-1: none), so that the
  * wait for it runs out.  No GPU fault is involved: the kernel only waits for
  * bytes that were never requested. */

@@ -409,10 +409,13 @@ struct Mma1Cfg {
     static_assert((2 * NA + 2 * NB + 2 * NTB + 1) * 8 + 4 <= 256, "barriers");
 };
 
+// limit_ns and skip (a database tile of CTA 0, in its order, or -1): as k_scan takes
+// them.  The waits for copies and MMAs still in flight before the kernel leaves keep
+// kMmaWaitNs, which no copy needs.
 __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t* __restrict__ dbop,
                                                                  const uint8_t* __restrict__ qop1,
                                                                  uint32_t* __restrict__ sout, int G, int rows,
-                                                                 int* __restrict__ err) {
+                                                                 int* __restrict__ err, uint64_t limit_ns, long skip) {
     using C = Mma1Cfg;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -449,12 +452,13 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
     if (warp == 0) {
         if (lane == 0) {
             const uint64_t pol_db = l2_policy_evict_first();
+            const long skip_i = blockIdx.x == 0 ? skip : -1;
             uint32_t ia = 0, ib = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ib++) {
                 const int ch = u & 1, z0 = (u >> 1) * C::ZB;
                 const int sb = (int)(ib % C::NB);
-                if (ib >= C::NB && !mbar_wait_bounded(&b_empty[sb], (uint32_t)((ib / C::NB - 1) & 1), kMmaWaitNs)) {
+                if (ib >= C::NB && !mbar_wait_bounded(&b_empty[sb], (uint32_t)((ib / C::NB - 1) & 1), limit_ns)) {
                     atomicOr(err, 8);
                     break;
                 }
@@ -463,21 +467,22 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
                 for (int g = 0; g < G && ok; g++)
                     for (int zi = 0; zi < C::ZB; zi++) {
                         const int sa = (int)(ia % C::NA);
-                        if (ia >= C::NA && !mbar_wait_bounded(&a_empty[sa], (uint32_t)((ia / C::NA - 1) & 1), kMmaWaitNs)) {
+                        if (ia >= C::NA && !mbar_wait_bounded(&a_empty[sa], (uint32_t)((ia / C::NA - 1) & 1), limit_ns)) {
                             atomicOr(err, 8);
                             ok = false;
                             break;
                         }
+                        if ((long)ia++ == skip_i) continue;   // injected failure: nothing arrives on a_full[sa]
                         mbar_arrive_expect_tx(&a_full[sa], kATile);
                         bulk_g2s_hint(atiles + sa * kATile, dbop + (((size_t)(z0 + zi) * 2 + ch) * G + g) * kATile, kATile,
                                       &a_full[sa], pol_db);
-                        ia++;
                     }
             }
             // never leave with copies in flight into shared memory (ib counts the units
             // whose query operand was asked for, but for one that was given up)
             for (uint32_t j = ia > C::NA ? ia - C::NA : 0; j < ia; j++)
-                if (!mbar_wait_bounded(&a_full[j % C::NA], (uint32_t)((j / C::NA) & 1), kMmaWaitNs)) atomicOr(err, 16);
+                if ((long)j != skip_i && !mbar_wait_bounded(&a_full[j % C::NA], (uint32_t)((j / C::NA) & 1), kMmaWaitNs))
+                    atomicOr(err, 16);
             for (uint32_t j = ib > C::NB ? ib - C::NB : 0; j < ib; j++)
                 if (!mbar_wait_bounded(&b_full[j % C::NB], (uint32_t)((j / C::NB) & 1), kMmaWaitNs)) atomicOr(err, 16);
         }
@@ -489,20 +494,20 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ib++) {
                 const int sb = (int)(ib % C::NB);
-                if (!mbar_wait_bounded(&b_full[sb], (uint32_t)((ib / C::NB) & 1), kMmaWaitNs)) {
+                if (!mbar_wait_bounded(&b_full[sb], (uint32_t)((ib / C::NB) & 1), limit_ns)) {
                     atomicOr(err, 32);
                     break;
                 }
                 for (int g = 0; g < G && ok; g++, tc++) {
                     const int tb = (int)(tc % C::NTB);
-                    if (tc >= C::NTB && !mbar_wait_bounded(&t_empty[tb], (uint32_t)((tc / C::NTB - 1) & 1), kMmaWaitNs)) {
+                    if (tc >= C::NTB && !mbar_wait_bounded(&t_empty[tb], (uint32_t)((tc / C::NTB - 1) & 1), limit_ns)) {
                         atomicOr(err, 32);
                         ok = false;
                         break;
                     }
                     for (int zi = 0; zi < C::ZB; zi++, ia++) {
                         const int sa = (int)(ia % C::NA);
-                        if (!mbar_wait_bounded(&a_full[sa], (uint32_t)((ia / C::NA) & 1), kMmaWaitNs)) {
+                        if (!mbar_wait_bounded(&a_full[sa], (uint32_t)((ia / C::NA) & 1), limit_ns)) {
                             atomicOr(err, 32);
                             ok = false;
                             break;
@@ -538,7 +543,7 @@ __global__ void __launch_bounds__(Mma1Cfg::THREADS, 1) k_scan_mma1(const uint8_t
             for (int g = 0; g < G; g++, tc++) {
                 const int tb = (int)(tc % C::NTB);
                 // warp-uniform outcome: tcgen05.ld below needs the whole warp
-                const bool got = mbar_wait_bounded(&t_full[tb], (uint32_t)((tc / C::NTB) & 1), kMmaWaitNs);
+                const bool got = mbar_wait_bounded(&t_full[tb], (uint32_t)((tc / C::NTB) & 1), limit_ns);
                 if (!__all_sync(0xffffffffu, got)) {
                     if (lane == 0) atomicOr(err, 128);
                     ok = false;

@@ -782,7 +782,9 @@ void enqueue_scan(kspir_ctx* c, int slot0, int nq, int kind, cudaStream_t st, bo
         uint8_t* qop = qop_at(c, slot0);
         k_qop_split_rm<1><<<dim3(kN / kSplitZ, 1), kSplitThreads, kSplitSmem, st>>>(
             reinterpret_cast<const uint32_t*>(c->ws0.cipherbuf), c->ws_bytes, slot0, 1, 1, qop);
-        k_scan_mma1<<<c->scan_ctas, Mma1Cfg::THREADS, Mma1Cfg::SMEM, st>>>(c->dbop, qop, w.sout, c->G, R * c->N2, w.err);
+        k_scan_mma1<<<c->scan_ctas, Mma1Cfg::THREADS, Mma1Cfg::SMEM, st>>>(c->dbop, qop, w.sout, c->G, R * c->N2, w.err,
+                                                                           c->wait_limit_ns, c->scan_skip);
+        c->scan_skip = -1;
         return;
     }
     auto tiles = [&](int kind, int slot, int n) {
@@ -1002,13 +1004,13 @@ int enqueue_fused(kspir_ctx* c, int client, cudaStream_t st, int ring_slot) {
 // Whether the scan of a single answer with `beside` others in flight runs on the
 // tensor cores (k_scan_mma1): from two others and two 32-row tiles on, unless
 // the caller set a variant for n = 1 (a tuned one was timed with nothing beside it and
-// says nothing here) or an injected failure waits for a CUDA-core scan.  us per answer, CUDA cores -> tensor cores: 32 answers on eight streams, r =
-// 16: 225 -> 202, r = 4: 73.6 -> 69.2; 4 answers, r = 16: 261 -> 250, r = 4: 113 -> 112;
-// 8 answers 226 -> 226 (217 with three others), 89 -> 86.  r = 2: 53 to 58 either
-// way, r = 1: 47 -> 50 (half of the tile is padding).
+// says nothing here).  us per answer, CUDA cores -> tensor cores: 32 answers on eight
+// streams, r = 16: 225 -> 202, r = 4: 73.6 -> 69.2; 4 answers, r = 16: 261 -> 250, r = 4:
+// 113 -> 112; 8 answers 226 -> 226 (217 with three others), 89 -> 86.  r = 2: 53 to 58
+// either way, r = 1: 47 -> 50 (half of the tile is padding).
 constexpr int kOneMinBeside = 2, kOneMinRows = 64;
 bool one_on_tensor_cores(const kspir_ctx* c, int beside) {
-    return c->mma && beside >= kOneMinBeside && c->p.r * c->N2 >= kOneMinRows && !c->one_forced && c->scan_skip < 0;
+    return c->mma && beside >= kOneMinBeside && c->p.r * c->N2 >= kOneMinRows && !c->one_forced;
 }
 
 // allow_fused: a single answer of slot 0 through the public single-answer

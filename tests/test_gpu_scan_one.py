@@ -5,6 +5,8 @@ one for the first two (CUDA cores), two or three for the rest (tensor cores from
 database rows on).  A tile chosen for n = 1 means the same scan, on every stream and at
 any number of rows.  Word for word against the same queries alone and the oracle,
 also with every database half at 2^32 - 1 (sums that wrap modulo 2^64)."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -104,3 +106,23 @@ def test_tuning_for_one_query_leaves_the_rule_beside_others():
             assert kinds[2:] == [beside] * (ANSWERS - 2), choose
             for i in range(ANSWERS):
                 assert np.array_equal(got[i], alone[i]), i
+
+
+@pytest.mark.parametrize("skip", [0, 3, 9])   # in the first lap of the ring of four tiles, its end, the third
+def test_wait_runs_out_after_the_callers_limit(skip):
+    r = 4
+    db, keys = database(r, "words"), po.gen_client(740, r, N1)
+    want = po.answer(db, r, N1, keys)
+    with context(r, db, keys) as ctx:
+        ctx.set_scan_kind(1, kb.SCAN_MMA4)
+        assert np.array_equal(ctx.answer(0, keys["query"]), want)
+        ctx.debug_scan_fault(wait_limit_ns=1_000_000, skip_item=skip)
+        t0 = time.perf_counter()
+        with pytest.raises(kb.KspirError) as e:
+            ctx.answer(0, keys["query"])
+        assert e.value.code == kb.native.ERR_TIMEOUT
+        assert time.perf_counter() - t0 < 1.0   # not the default limit of two seconds
+        for _ in range(ANSWERS):
+            assert np.array_equal(ctx.answer(0, keys["query"]), want)
+        ctx.debug_scan_fault()
+        assert np.array_equal(ctx.answer(0, keys["query"]), want)
