@@ -208,12 +208,6 @@ __host__ __device__ __forceinline__ uint32_t mod28(uint64_t x, uint32_t q, uint3
     return min_u32(t, t - q);
 }
 
-// x mod q_ch for the crt primes (ch 0: q1, 1: q2), any 64-bit x.  (mod28 measured
-// no faster than this Barrett reduction inside the key-switch kernels.)
-__device__ __forceinline__ uint32_t mod_crt(uint64_t x, int ch) {
-    return reduce64(x, ch ? kQ2 : kQ1, c_dev.ch[ch].barrett);
-}
-
 __device__ __forceinline__ uint32_t mod_q1(uint64_t v) { return reduce64(v, kQ1, c_dev.ch[CH_Q1].barrett); }
 __device__ __forceinline__ uint32_t mod_q2(uint64_t v) { return reduce64(v, kQ2, c_dev.ch[CH_Q2].barrett); }
 __device__ __forceinline__ uint32_t mod_bs(uint64_t v) { return reduce64(v, kBsMod, c_dev.ch[CH_BS].barrett); }

@@ -38,7 +38,6 @@ __device__ __forceinline__ void query_prep_one(const uint64_t* q, const Workspac
 // The key slots of a launch's queries.
 constexpr int kMaxBatch = 256;     // queries per launch
 struct ClientList {
-    int n;
     int id[kMaxBatch];
 };
 

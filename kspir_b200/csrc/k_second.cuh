@@ -49,10 +49,7 @@ __device__ __forceinline__ void key_mac4(const uint32_t* d, int dstride, const u
 }
 
 // ---------------------------------------------------------------------------
-// giant steps
-
-// ---------------------------------------------------------------------------
-// external product
+// external product, unfused (the allocation-free entry point)
 
 // Signed digits of decompose_rlwe(a, b) (utils.cpp:974-1044) of the
 // coefficient-form first-dimension result: edig[r][row][ch][k], rows 0..ell-1
@@ -105,10 +102,6 @@ __global__ void __launch_bounds__(kNttThreads) k_ext_mac_intt(const uint32_t* __
 #pragma unroll
     for (int k = threadIdx.x; k < kN; k += T) o[k] = s[pidx(k)];
 }
-
-}  // namespace kspir
-
-namespace kspir {
 
 // ---------------------------------------------------------------------------
 // fused giant step: one CTA per (r, c >= 1) (blockIdx.y = query of the batch) runs the whole key switch of
@@ -304,10 +297,6 @@ __device__ __forceinline__ void first_dim_to_smem(uint32_t* s, const uint32_t* f
     for (int k = threadIdx.x % T; k < kN / 4; k += T)
         *reinterpret_cast<uint4*>(s + pidx(4 * k)) = giant_sum4(g, wo, fd, r, cv, 4 * k);
 }
-
-}  // namespace kspir
-
-namespace kspir {
 
 // ---------------------------------------------------------------------------
 // fused packing level: one CTA per (pair j, prime ch) runs convertTwoRLWEs

@@ -644,7 +644,6 @@ bool giant_two_acc(const kspir_ctx* c) { return c->N2 - 1 > kGiantTermsPerAcc; }
 // query words [nq][4][N] at q -> digits and residues; key slots of the queries
 void enqueue_prep(kspir_ctx* c, int slot0, int nq, const int* clients, const uint64_t* q, cudaStream_t st) {
     ClientList cl;
-    cl.n = nq;
     for (int i = 0; i < nq; i++) cl.id[i] = clients[i];
     launch(c, false, k_query_prep, dim3(kN / 256, nq), 256, 0, st, q, cl, c->client_of, c->ws0, c->gad.baby,
            batch_of(c, slot0), c->p.r * 4 * kN, giant_two_acc(c) ? 1 : 0);
@@ -716,7 +715,7 @@ int scan_tail(int kind, int nq) {
     return kind == SCAN_MMA32 && nq > 32 && rem <= 16 ? rem : 0;
 }
 
-long scan_launches(const kspir_ctx*, int kind, int nq) {
+long scan_launches(int kind, int nq) {
     return kind == SCAN_CUDA ? nq : scan_tail(kind, nq) ? 4 : 2;
 }
 
@@ -859,7 +858,7 @@ void enqueue_ext(kspir_ctx* c, int slot0, int nq, int count, bool sums, const ui
 // per CTA, latency) rather than whole merges per CTA pair (throughput): few
 // queries and few merges.  One query, us per level: I = 32 and 16 together 70 split, 45
 // fused; I <= 8: 12 to 16 split, 18 to 20 fused.  c2out only the split kernels write.
-bool pack_split(const kspir_ctx*, int nq, int I, const uint32_t* c2out) {
+bool pack_split(int nq, int I, const uint32_t* c2out) {
     return c2out || (nq <= kPackSplitMaxBatch && nq * I < 16);
 }
 
@@ -875,7 +874,7 @@ void enqueue_packing(kspir_ctx* c, int slot0, int nq, cudaStream_t st, uint32_t*
         const uint32_t ginv = inv_mod_2n((uint32_t)(kN / I + 1));
         uint32_t* out = (cur == w.ext) ? w.ext2 : w.ext;
         const uint32_t* key = c->keys0.packing + (size_t)lv * pe * 4 * kN;
-        if (pack_split(c, nq, I, c2out)) {   // latency: one transform per CTA
+        if (pack_split(nq, I, c2out)) {   // latency: one transform per CTA
             launch(c, true, k_pack_split_fwd<4>, dim3(I * 2 * 5, nq), kNttThreads, kPackSplitSmem, st, cur, w.pkpart, key, I,
                    ginv, c->ntabs, c->gad.pack, bt);
             launch(c, true, k_pack_split_inv<4>, dim3(I * 4, nq), kNttThreads, kPackSplitSmem, st, cur,
@@ -900,8 +899,8 @@ long answer_launches(const kspir_ctx* c, int kind, int nq) {
     // baby 7 (and the transpose of a CUDA-core scan's), scan, giant 1 or 2, external product 1, packing one or
     // two per level + compose
     long packing = 0;
-    for (int lv = 0; lv < c->levels; lv++) packing += pack_split(c, nq, 1 << lv, nullptr) ? 2 : 1;
-    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(c, kind, nq) + (ext_wide(c, c->p.r, nq) ? 1 : 2) + 1 +
+    for (int lv = 0; lv < c->levels; lv++) packing += pack_split(nq, 1 << lv, nullptr) ? 2 : 1;
+    return 7 + (kind == SCAN_CUDA ? 1 : 0) + scan_launches(kind, nq) + (ext_wide(c, c->p.r, nq) ? 1 : 2) + 1 +
            packing + 1;
 }
 
