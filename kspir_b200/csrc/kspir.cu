@@ -395,10 +395,10 @@ uint2 lazy_twiddle(uint64_t w, uint32_t q) {
     return make_uint2((uint32_t)c, (uint32_t)(c < 0 ? -p : p));
 }
 
-// The device table of one channel (layout in ntt.cuh).
-void build_twiddles(uint64_t psi, uint32_t q, uint2* out) {
-    std::vector<uint32_t> pw(2 * kN);   // psi^e
-    pw[0] = 1;
+// The device table of one channel (layout in ntt.cuh).  pw: scratch, [2N]; no
+// allocation here (kspir_external_product_noalloc).
+void build_twiddles(uint64_t psi, uint32_t q, uint2* out, uint32_t* pw) {
+    pw[0] = 1;   // psi^e
     for (int e = 1; e < 2 * kN; e++) pw[e] = (uint32_t)((uint64_t)pw[e - 1] * psi % q);
     const uint64_t ninv = h_invmod(kN, q);
     // entry e of unit i of a pass with `units` units
@@ -464,7 +464,9 @@ int init_constants(kspir_ctx* c) {
     // twiddles: crt channels use root_of_unity_crt (reference crt.h:81) reduced
     // per prime; bsMod and p use HEXL's minimal primitive root
     std::vector<uint2> tw((size_t)CH_COUNT * kTwChannel);
-    for (int ch = 0; ch < CH_COUNT; ch++) build_twiddles(chan_root(ch), kChanQ[ch], tw.data() + (size_t)ch * kTwChannel);
+    std::vector<uint32_t> pw(2 * kN);
+    for (int ch = 0; ch < CH_COUNT; ch++)
+        build_twiddles(chan_root(ch), kChanQ[ch], tw.data() + (size_t)ch * kTwChannel, pw.data());
     KS_CUDA(c, cudaMalloc(&c->tw, tw.size() * sizeof(uint2)));
     KS_COPY(c, c->tw, tw.data(), tw.size() * sizeof(uint2), cudaMemcpyHostToDevice);
     for (int ch = 0; ch < CH_COUNT; ch++) c->ntabs.tw[ch] = c->tw + (size_t)ch * kTwChannel;
@@ -2819,10 +2821,11 @@ int na_setup(int device, cudaStream_t st) {
     const DevConst dc = make_dev_const();   // the same constants a context writes
     if (cudaMemcpyToSymbolAsync(c_dev, &dc, sizeof(dc), 0, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return KSPIR_ERR_CUDA;
-    std::vector<uint2> tw(3 * (size_t)kTwChannel);
-    for (int ch = 0; ch < 3; ch++) build_twiddles(chan_root(ch), kChanQ[ch], tw.data() + (size_t)ch * kTwChannel);
-    if (cudaMemcpyAsync(d.tw, tw.data(), tw.size() * sizeof(uint2), cudaMemcpyHostToDevice, st) != cudaSuccess)
-        return KSPIR_ERR_CUDA;
+    // host memory of the library too (g_na_mutex is held)
+    static uint2 tw[3 * kTwChannel];
+    static uint32_t pw[2 * kN];
+    for (int ch = 0; ch < 3; ch++) build_twiddles(chan_root(ch), kChanQ[ch], tw + (size_t)ch * kTwChannel, pw);
+    if (cudaMemcpyAsync(d.tw, tw, sizeof(tw), cudaMemcpyHostToDevice, st) != cudaSuccess) return KSPIR_ERR_CUDA;
     NaLayout L = na_layout(d.scratch);
     k_na_jobs<<<1, kNoAllocMaxCount * 12, 0, st>>>(L.jobs, L.fd_res, L.ecoef, L.edig);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return KSPIR_ERR_CUDA;
