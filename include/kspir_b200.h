@@ -296,7 +296,7 @@ int kspir_packing_rlwes(kspir_ctx* ctx, int client, uint64_t* rlwes, uint64_t* r
  * stream); the call then waits for that stream (cudaStreamSynchronize) and
  * reads a validation word back, so it returns only after its work is done
  * and blocks the calling thread until then.
- * Scratch: a fixed file-scope device array of about 6.3 MiB (plus 300 KiB of
+ * Scratch: a fixed file-scope device array of about 6.3 MiB (plus 204 KiB of
  * transform tables) that every GPU loading this library holds until the
  * process exits.  All calls on a device share it, so calls that overlap on
  * the GPU (other threads, other streams) race and must be serialised by the
@@ -328,9 +328,7 @@ int kspir_timing_summary(kspir_ctx* ctx, int* answers, long* launches, float* to
  * as reference words (host buffer of exactly the stated size):
  *   KSPIR_STAGE_CIPHERBUF [N][N1][2]  reorientCipher output (twosteps.cpp:1386-1403)
  *   KSPIR_STAGE_SCAN      [r][N2][2][N] fastMultiplyQueryByDatabaseDim1InvCRT outputs
- *                         (recomputed from the slot's reorientCipher output by
- *                         the scan variant of the last launch: the giant steps
- *                         reuse the scan output in place)
+ *                         (the staged calls and kspir_tune_batch overwrite them)
  *   KSPIR_STAGE_RESULT    [r][2][N]   first-dimension results (NTT form)
  *   KSPIR_STAGE_EXT       [r][2][N]   external products (coefficient form) */
 #define KSPIR_STAGE_CIPHERBUF 0

@@ -26,8 +26,9 @@
 // digits of a slot and its b side by side (16 bytes), one gather per slot for
 // the three digits of both components.
 //
-// What bounds it: instruction issue and the multiply pipe (ntt.cuh), with the
-// keys (22 MiB per client) streaming from L2 or HBM beside it.  Batch of 64:
+// What bounds it: load and store wavefronts (65 % busy, the digit gathers above all),
+// issue (51 %) and the multiply pipe (41 %; ntt.cuh) together, with the keys (22 MiB
+// per client) streaming from L2 or HBM beside it.  Batch of 64:
 // 1.20 ms with one component per CTA, conditional-subtraction transforms and
 // 64-bit Barrett reductions, 0.77 ms in this form.
 #pragma once

@@ -43,7 +43,8 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;     // 2 s per bounded wait
 // database (consumer warps x stages of 18 KiB, 148 CTAs): 4 x 8 0.156 ms
 // (6.9 TB/s), 6 x 6 0.176 ms, 6 x 12 0.176 ms, 4 x 4 0.214 ms.  The default
 // (streaming) shape is 4 x 8: 145 KiB of shared memory, which leaves 82 KiB of the
-// SM to key-switch CTAs (19 to 76 KiB each) of a concurrent answer.  The sharing shape
+// SM to key-switch CTAs of a concurrent answer (19 to 76 KiB each; k_pack_fused, which
+// packs levels of 16 merges and more, takes 95 and waits for the scan).  The sharing shape
 // (ScanShare) is 6 x 6: 109 KiB, slower alone but leaving 118, which pays at N1 = 128 when
 // other answers are in flight: us for 16 answers on eight streams at r = 1 619
 // (streaming) -> 598, for 32 at r = 2 1611 -> 1561, two at r = 64 1467 -> 1451.  At N1 =

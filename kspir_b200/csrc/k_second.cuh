@@ -20,9 +20,9 @@ namespace kspir {
 // The key products of a thread's coefficients u + 256 (4 v + w), w = 0..3, on prime
 // ch: ra, rb = sum over the ROWS polynomials d (in shared memory at stride
 // `dstride`, lazy signed words below 6.7 q) times the keys of components a
-// and b, reduced to within +-1 q.  The keys (lane order, centred, times +-2^32:
-// k_keys_from_words) come as one 16-byte vector per row and component, at
-// `krow` vectors between rows and `kcomp` between components.
+// and b, reduced to within +-q (ROWS = 2) or +-1.4 q (ROWS = 4).  The keys (lane
+// order, centred, times +-2^32: k_keys_from_words) come as one 16-byte vector per
+// row and component, at `krow` vectors between rows and `kcomp` between components.
 // |sum| <= ROWS 6.7 q q / 2 < 2^60; / 2^32 it is 0.21 ROWS q at most, and the
 // Montgomery term adds q / 2: within +-q for ROWS = 2, +-1.4 q for ROWS = 4.
 template <int ROWS>
@@ -127,8 +127,8 @@ constexpr int kGiantSmem = kGiantPolys * kPadN * 4;
 // set of twiddle loads for both) and the key products.  X -> X^g keeps
 // coefficients u + 256 t in column u, the column that a thread's last inverse and
 // first forward pass hold, so the digits reach the transform in registers and only
-// the other prime's half crosses shared memory.  Bounded by issue, the multiply pipe
-// and shared-memory wavefronts together (each 55 to 60 % busy at 2 CTAs per SM;
+// the other prime's half crosses shared memory.  Bounded by issue, load and store
+// wavefronts and the multiply pipe together (57, 55 and 46 % busy at 2 CTAs per SM;
 // without the decomposition, the b gather and the accumulation 0.99 ms remain of
 // 1.16).  Batch of 64 at r = 16: 1.56 ms with conditional-subtraction radix-8
 // transforms and 64-bit Barrett reductions, 1.18 ms with the digits written

@@ -2,8 +2,9 @@
 after other calls have reused the scan output that their sums were left in: the
 staged packing (slot 0), the staged external product of fewer ciphertexts (slot 0;
 the others' results stay) and the scan tuning (every slot of the batch, here from
-cipherbufs in the other layout than its last variant reads).  One accumulator (N1 = 128) and two (N1 = 64).  Word for word against the results
-read straight after the batch and against the staged first dimension."""
+cipherbufs in the other layout than its last variant reads).  One accumulator
+(N1 = 128) and two (N1 = 64).  Word for word against the results read straight after
+the batch and against the staged first dimension."""
 import numpy as np
 import pytest
 
